@@ -173,7 +173,7 @@ int vtp_solver::parse_config(const json &c) {
         force_div = force_inc = 0;
         force_seq.clear();
         device_loop = true; use_graphs = true; stage_timers = false; stop_on_crash = true;
-        block = 128; unroll = 4; persistent_tiles = false; cube_powf = false; list_lanes = 0; row_lanes = 1;
+        block = 128; unroll = 4; persistent_tiles = false; cube_powf = false; row_lanes = 1;
         cell_cull = false; staged_solve = false; stage_rows = 2048; tape_budget_mb = 8192; adj_lanes = 1;
         cfl = 0.f;
         cell_order_brick = true;
@@ -219,9 +219,10 @@ int vtp_solver::parse_config(const json &c) {
             stage_rows = b.value("stageRows", 2048);
             if (stage_rows < 256 || stage_rows > (int)vtp::kStageMaxRows)
                 return fail(VTP_ERR_CONFIG, "stageRows must be in [256, 32767]");
-            list_lanes = b.value("listLanes", 0);
+            // One builder serves every row count; the key keeps its values and the lists never depended on it.
+            const int list_lanes = b.value("listLanes", 0);
             if (list_lanes != 0 && list_lanes != 1 && list_lanes != 8)
-                return fail(VTP_ERR_CONFIG, "listLanes must be 0 (by row count), 1 or 8");
+                return fail(VTP_ERR_CONFIG, "listLanes must be 0, 1 or 8");
             const std::string cube = b.value("cubicCube", std::string("rounded"));
             if (cube != "rounded" && cube != "powf")
                 return fail(VTP_ERR_CONFIG, "cubicCube must be \"rounded\" or \"powf\"");
@@ -357,7 +358,7 @@ int vtp_solver::attach(const float *p, uint32_t n, const float *v, const json &o
 
 vtp::PbfArgs vtp_solver::pbf_args() {
     vtp::PbfArgs a{};
-    a.nf = L.nf; a.nb = L.nb; a.ell_stride = L.ell_stride; a.k = kc;
+    a.nf = L.nf; a.nb = L.nb; a.shape = L.shape; a.k = kc;
     a.rho0 = rho_f; a.inv_rho0 = 1.f / rho_f; a.rho_b = rho_b; a.eps = pbf_eps; a.dt = dt; a.xsph_k = xsph_k;
     a.form = pbf_form;
     a.h2 = h * h;
@@ -373,7 +374,7 @@ vtp::PbfArgs vtp_solver::pbf_args() {
 
 vtp::DfsphArgs vtp_solver::dfsph_args(int which) {
     vtp::DfsphArgs a{};
-    a.nf = L.nf; a.nb = L.nb; a.ell_stride = L.ell_stride; a.k = kc;
+    a.nf = L.nf; a.nb = L.nb; a.shape = L.shape; a.k = kc;
     a.dt = dt; a.inv_dt = inv_dt; a.inv_dt2 = inv_dt2;
     a.rho0 = rho_f; a.rho_b = rho_b; a.vol_f = vol0;
     a.mass_f = rho_f * vol0;                               // update_mass_cuda: m = rest_density * V
@@ -394,6 +395,7 @@ vtp::DfsphArgs vtp_solver::dfsph_args(int which) {
     a.pk = pk;
     a.tick = d_tick;
     a.unroll = unroll;
+    a.teams = teams;
     a.staged = staged ? 1 : 0;
     a.stg = stg;
     a.dtp = cfl > 0.f ? d_cfl : nullptr;
@@ -409,6 +411,7 @@ vtp::SolveCtl vtp_solver::solve_ctl(int which, cudaGraphConditionalHandle hnd, i
     c.scene_tiles = staged ? d_scene_groups : d_scene_tiles;
     c.nscenes = nscenes();
     c.nobj_max = nobj_max;
+    c.pieces = teams && !staged ? vtp::solve_pieces(block) : 1u;
     c.threshold = which == 0 ? div_thr : incomp_thr;
     c.force_iters = which == 0 ? force_div : force_inc;
     c.force_seq = d_force_seq;
@@ -455,7 +458,6 @@ int vtp_solver::initialize() {
         if (o.mat == 0) L.nf += o.end - o.start;
     }
     L.nb = n - L.nf;
-    L.ell_stride = maxnbr > 1 ? maxnbr - 1 : 1;
     // Attach ids of fluid vs boundary decide how a cell's two runs interleave
     // (per scene; scenes that disagree fall back to the general merge).
     int mode = -1;
@@ -474,8 +476,10 @@ int vtp_solver::initialize() {
         mode = mode < 0 ? m : (mode == m ? m : 2);
     }
     L.merge_mode = mode < 0 ? 0 : mode;
-    L.list_lanes = list_lanes;
     L.cell_cull = cell_cull;
+    teams = L.nf <= vtp::kTeamMaxRows && !persistent_tiles && type == VTP_SOLVER_DFSPH;
+    L.shape.stride = vtp::list_stride(maxnbr > 1 ? maxnbr - 1 : 1);
+    L.shape.lg = teams ? vtp::kTeamListLg : 0u;
 
     // Grids as UniformGirdNeighborSearcher::setConfig (UniformGridNeighborSearch.cpp:214-218),
     // one per scene, each followed by its own outside bucket.
@@ -548,9 +552,9 @@ int vtp_solver::initialize() {
     if (u.scan_tiles > 1024 * 64) return fail(VTP_ERR_BOUNDS, "grid too large for the cell scan");
     AL(&u.scan_sums, u.scan_tiles);
     const size_t fl_rows = ((size_t)L.nf + 31) / 32 * 32, bl_rows = ((size_t)L.nb + 31) / 32 * 32;
-    AL(&u.nbr, fl_rows * L.ell_stride);
+    AL(&u.nbr, fl_rows * L.shape.stride);
     AL(&u.ncnt, L.nf);
-    AL(&u.bnbr, bl_rows * L.ell_stride);
+    AL(&u.bnbr, bl_rows * L.shape.stride);
     AL(&u.bncnt, L.nb);
     AL(&d_status, 4);
     u.status = d_status;
@@ -684,7 +688,7 @@ int vtp_solver::initialize() {
         // do not interleave; residual partials per cell group (plus one for the rows outside).
         staged = staged_solve && type == VTP_SOLVER_DFSPH && S == 1 && scenes[0].grid.brick &&
                  L.merge_mode != 2 && L.nf > 0;
-        size_t npart = std::max<uint32_t>(ntiles, 1);
+        size_t npart = std::max<size_t>((size_t)ntiles * (teams ? vtp::solve_pieces(block) : 1u), 1);
         if (staged) {
             stg.ngroups = scenes[0].grid.nkey / vtp::kStageBuckets;
             stg.scap = (uint32_t)stage_rows;
@@ -692,7 +696,7 @@ int vtp_solver::initialize() {
             stg.fstart = u.fstart;
             stg.bstart = u.bstart;
             const size_t fl_rows = ((size_t)L.nf + 31) / 32 * 32;
-            AL(&stg.snbr, fl_rows * L.ell_stride);
+            AL(&stg.snbr, fl_rows * L.shape.stride);
             vtp::SceneTiles sg = stl[0];
             sg.tile0 = 0;
             sg.ntiles = stg.ngroups + 1;
@@ -711,12 +715,11 @@ int vtp_solver::initialize() {
     vtp::ugns_sort(st, scn(), nbuckets, 0, L.nf, pos.c(), pos.n(), vel.c(), vel.n(), orig.c(), orig.n(), carry, 0.f,
                    u, u.fstart);
     pos.swap(); vel.swap(); orig.swap();
-    vtp::ugns_build_lists(st, scn(), L, 0, L.nf, pos.c(), orig.c(), u, u.nbr, u.ncnt, d_status, d_overflow, block);
-    vtp::ugns_build_lists(st, scn(), L, L.nf, L.nb, pos.c(), orig.c(), u, u.bnbr, u.bncnt, d_status, d_overflow,
-                          block);
+    vtp::ugns_build_lists(st, scn(), L, 0, L.nf, pos.c(), orig.c(), u, u.nbr, u.ncnt, d_status, d_overflow);
+    vtp::ugns_build_lists(st, scn(), L, L.nf, L.nb, pos.c(), orig.c(), u, u.bnbr, u.bncnt, d_status, d_overflow);
     if (type == VTP_SOLVER_PBF) {
         vtp::PbfArgs a = pbf_args();
-        vtp::pbf_init_boundary(st, a, u.bncnt, u.bnbr, L.ell_stride);
+        vtp::pbf_init_boundary(st, a, u.bncnt, u.bnbr, L.shape);
         // boundary volumes live in vol[]; masses in pos.w of both buffers (kernel writes both)
         CU(cudaMemcpyAsync(pos.n() + L.nf, pos.c() + L.nf, (size_t)L.nb * sizeof(float4), cudaMemcpyDeviceToDevice, st));
     } else {
@@ -833,7 +836,7 @@ int vtp_solver::enqueue_pbf_substep(cudaStream_t s, const PbfTapeSlot *tape) {
     pos.swap(); vel.swap(); orig.swap();
     uint32_t *lnbr = tape ? tape->nbr : u.nbr, *lcnt = tape ? tape->ncnt : u.ncnt;
     PROF(this, "ugns_lists", vtp::ugns_build_lists(s, scn(), L, 0, L.nf, pos.c(), orig.c(), u, lnbr, lcnt,
-                                                   d_status, d_overflow, block));
+                                                   d_status, d_overflow));
     launches_per_tick += 7;  // hash, 3 scan kernels, scatter, rank/reorder, lists
     if (tape && nf) {
         CU(cudaMemcpyAsync(tape->orig, orig.c(), nf * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
@@ -887,7 +890,7 @@ int vtp_solver::enqueue_tick(cudaStream_t s, bool capture) {
                                                               d_overflow));
     } else {
         PROF(this, "ugns_lists", vtp::ugns_build_lists(s, scn(), L, 0, L.nf, pos.c(), orig.c(), u, u.nbr, u.ncnt,
-                                                       d_status, d_overflow, block));
+                                                       d_status, d_overflow));
     }
     PROF(this, "dfsph_ratio_alpha", vtp::dfsph_ratio_alpha(s, dfsph_args(), block));
     launches_per_tick += 8;  // neighbour search (7) + ratio/alpha
@@ -1611,9 +1614,9 @@ int vtp_solver_get_neighbors(vtp_solver *s, uint32_t *counts, uint32_t *nbrs, ui
         if (rc) return rc;
     }
     vtp::ugns_build_lists(s->st, s->scn(), s->L, 0, s->L.nf, s->pos.c(), s->orig.c(), s->u, s->u.nbr, s->u.ncnt,
-                          s->d_status, s->d_overflow, s->block);
+                          s->d_status, s->d_overflow);
     vtp::ugns_build_lists(s->st, s->scn(), s->L, s->L.nf, s->L.nb, s->pos.c(), s->orig.c(), s->u, s->u.bnbr,
-                          s->u.bncnt, s->d_status, s->d_overflow, s->block);
+                          s->u.bncnt, s->d_status, s->d_overflow);
     uint32_t *dc = nullptr, *dn = nullptr;
     CU(cudaMalloc(&dc, (size_t)n * 4));
     cudaError_t e = cudaMalloc(&dn, (size_t)n * max_nbr * 4);

@@ -91,7 +91,7 @@ __device__ __forceinline__ uint32_t cell_key(int3 c, const Grid &g) {
 // global key buckets [key_base, key_base + nkey]; the last one is its
 // "outside" bucket, so a scene's rows stay in one fixed contiguous range of
 // the sorted order.  With S = 1 this is exactly the reference's single grid.
-struct SceneGrid {
+struct alignas(16) SceneGrid {   // 48 bytes, read as three 16-byte loads
     float lbx, lby, lbz;
     int gx, gy, gz;
     uint32_t key_base;
@@ -165,11 +165,24 @@ __device__ __forceinline__ int3 nbr_offset(int t) {
     return make_int3(t / 9 - 1, (t / 3) % 3 - 1, t % 3 - 1);
 }
 
-// Warp-interleaved ELL neighbour list: for row r, slot t lives at
-// base + (r/32)*32*stride + t*32 + r%32, so a warp reading slot t of 32
-// consecutive rows touches one 128-byte line.
-__device__ __forceinline__ size_t ell_index(uint32_t row, uint32_t t, uint32_t stride) {
-    return (size_t)(row >> 5) * 32u * stride + (size_t)t * 32u + (row & 31u);
+// Neighbour list storage.  32 entries fill one 128-byte line: 2^lg consecutive entries each of
+// 32 / 2^lg consecutive rows.  lg 0 for passes with a thread per row (a warp reads entry t of its
+// 32 rows from one line); lg 3 for passes with a team of lanes per row (a team reads consecutive
+// entries of its row, a warp's 8 rows read two lines).  The stride (entries a row has room for) is
+// a multiple of 8.
+struct ListShape {
+    uint32_t stride = 0, lg = 0;
+};
+constexpr uint32_t kTeamListLg = 3;
+inline uint32_t list_stride(uint32_t entries) { return (entries + 7u) / 8u * 8u; }
+// Offset of entry t from the row's first entry.
+__device__ __forceinline__ uint32_t ell_slot(uint32_t t, ListShape s) {
+    return ((t >> s.lg) << 5) | (t & ((1u << s.lg) - 1u));
+}
+__device__ __forceinline__ uint32_t team_slot(uint32_t t) { return ((t >> kTeamListLg) << 5) | (t & 7u); }
+__device__ __forceinline__ size_t ell_index(uint32_t row, uint32_t t, ListShape s) {
+    const uint32_t rows = 32u >> s.lg;
+    return (size_t)(row >> (5u - s.lg)) * (s.stride << (5u - s.lg)) + ((row & (rows - 1u)) << s.lg) + ell_slot(t, s);
 }
 
 // Cubic spline (sph::cubic_value / cubic_gradient, KernelFunctions.cuh:13-57).
@@ -275,44 +288,57 @@ __device__ __forceinline__ F4x2 ldg8(const float4 *p) {
     return r;
 }
 
-// Walks `cnt` list entries (warp-interleaved ELL, slot t at lst[t * 32]) in
-// order, U at a time: the list indices of the next batch are loaded before the
-// current batch's gathers (`load(j)`) are issued, so each thread keeps U
-// gathers and U index loads in flight.  `use(j, data)` runs in list order,
-// which keeps FP32 accumulation order identical for every U.
-template <int U, class Load, class Use>
-__device__ __forceinline__ void nbr_loop(const uint32_t *__restrict__ lst, uint32_t cnt, Load load, Use use) {
-    if constexpr (U <= 1) {
-        for (uint32_t t = 0; t < cnt; ++t) {
-            const uint32_t j = __ldcs(lst + (size_t)t * 32u);
-            use(j, load(j));
-        }
-    } else {
-        using T = decltype(load(0u));
-        uint32_t nxt[U];
+// First entry of a row, and the offset of its entry t, in lists of lg 0.
+__device__ __forceinline__ size_t row_index(uint32_t row, ListShape s) {
+    return (size_t)(row >> 5) * 32u * s.stride + (row & 31u);
+}
+struct RowSlots {
+    __device__ __forceinline__ size_t operator()(uint32_t t) const { return (size_t)t * 32u; }
+};
+// The offset of entry t in lists of either shape.
+struct AnySlots {
+    ListShape s;
+    __device__ __forceinline__ uint32_t operator()(uint32_t t) const { return ell_slot(t, s); }
+};
+
+// Walks the `cnt` list entries of a row in order, U at a time: the list indices
+// of the next batch are loaded before the current batch's gathers (`load(j)`)
+// are issued, so each thread keeps U gathers and U index loads in flight.
+// `use(j, data)` runs in list order, which keeps FP32 accumulation order
+// identical for every U.  (The last partial batch one gather at a time: with
+// its gathers issued together the solve passes are 3-9 % slower at 1M rows.)
+template <int U, class Slots, class Load, class Use>
+__device__ __forceinline__ void nbr_loop_at(const uint32_t *__restrict__ lst, Slots at, uint32_t cnt, Load load,
+                                            Use use) {
+    using T = decltype(load(0u));
+    uint32_t nxt[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) nxt[u] = (uint32_t)u < cnt ? __ldcs(lst + (size_t)u * 32u) : 0u;
-        uint32_t t = 0;
-        for (; t + U <= cnt; t += U) {
-            uint32_t j[U];
+    for (int u = 0; u < U; ++u) nxt[u] = (uint32_t)u < cnt ? __ldcs(lst + at((uint32_t)u)) : 0u;
+    uint32_t t = 0;
+    for (; t + U <= cnt; t += U) {
+        uint32_t j[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) j[u] = nxt[u];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const uint32_t tt = t + U + (uint32_t)u;
-                nxt[u] = tt < cnt ? __ldcs(lst + (size_t)tt * 32u) : 0u;
-            }
-            T d[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) d[u] = load(j[u]);
-#pragma unroll
-            for (int u = 0; u < U; ++u) use(j[u], d[u]);
-        }
+        for (int u = 0; u < U; ++u) j[u] = nxt[u];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            if (t + (uint32_t)u < cnt) use(nxt[u], load(nxt[u]));
+            const uint32_t tt = t + U + (uint32_t)u;
+            nxt[u] = tt < cnt ? __ldcs(lst + at(tt)) : 0u;
         }
+        T d[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) d[u] = load(j[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) use(j[u], d[u]);
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        if (t + (uint32_t)u < cnt) use(nxt[u], load(nxt[u]));
+    }
+}
+// In the passes with a thread per row.
+template <int U, class Load, class Use>
+__device__ __forceinline__ void nbr_loop(const uint32_t *__restrict__ lst, uint32_t cnt, Load load, Use use) {
+    nbr_loop_at<U>(lst, RowSlots{}, cnt, load, use);
 }
 
 // Lane groups for rows walked by L lanes each (L divides 32; the L lanes of a
@@ -336,17 +362,17 @@ __device__ __forceinline__ float lane_sum(float v, unsigned mask) {
 // one row's list and each keeps U gathers in flight.  With L == 1 this is
 // nbr_loop itself (same order, same results).
 template <int U, int L, class Load, class Use>
-__device__ __forceinline__ void nbr_loop_lanes(const uint32_t *__restrict__ lst, uint32_t cnt, int lane, Load load,
-                                               Use use) {
+__device__ __forceinline__ void nbr_loop_lanes(const uint32_t *__restrict__ lst, ListShape shape, uint32_t cnt, int lane,
+                                               Load load, Use use) {
     if constexpr (L == 1) {
-        nbr_loop<U>(lst, cnt, load, use);
+        nbr_loop_at<U>(lst, AnySlots{shape}, cnt, load, use);
     } else {
         using T = decltype(load(0u));
         uint32_t t = (uint32_t)lane;
         for (; t + (uint32_t)((U - 1) * L) < cnt; t += (uint32_t)(U * L)) {
             uint32_t j[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) j[u] = __ldcs(lst + (size_t)(t + (uint32_t)(u * L)) * 32u);
+            for (int u = 0; u < U; ++u) j[u] = __ldcs(lst + ell_slot(t + (uint32_t)(u * L), shape));
             T d[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) d[u] = load(j[u]);
@@ -354,7 +380,7 @@ __device__ __forceinline__ void nbr_loop_lanes(const uint32_t *__restrict__ lst,
             for (int u = 0; u < U; ++u) use(j[u], d[u]);
         }
         for (; t < cnt; t += (uint32_t)L) {
-            const uint32_t j = __ldcs(lst + (size_t)t * 32u);
+            const uint32_t j = __ldcs(lst + ell_slot(t, shape));
             use(j, load(j));
         }
     }

@@ -20,6 +20,7 @@
 //                 add_acc_surface_tension_cuda (:298-353) when gamma != 0
 //   finalize    : apply_pressure_acc + update_pos_cuda (:393-404)
 #include "dfsph.h"
+#include "team.cuh"
 
 #include <algorithm>
 
@@ -82,9 +83,9 @@ __global__ void __launch_bounds__(256) k_rigid_volume(DfsphArgs a, const uint32_
     float4 p = a.pos[i];
     uint32_t n = bncnt[r];
     float delta = n > 0 ? a.k.w0 : 0.f;
-    const uint32_t *lst = bnbr + ell_index(r, 0, a.ell_stride);
+    const uint32_t *lst = bnbr + ell_index(r, 0, a.shape);
     for (uint32_t t = 0; t + 1 < n; ++t) {
-        uint32_t j = lst[(size_t)t * 32u];
+        uint32_t j = lst[ell_slot(t, a.shape)];
         if (j < a.nf) continue;
         float4 q = a.pos[j];
         delta += cubic_w(dist2(p.x - q.x, p.y - q.y, p.z - q.z), a.k);
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(256) k_ratio_alpha(DfsphArgs a) {
     RatioAlpha ra;
     ra.begin(n > 0 ? __fmul_rn(p.w, a.k.w0) : 0.f);   // self term V_i W(0)
     const float inv_mf = __fdiv_rn(1.f, a.mass_f);
-    const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+    const uint32_t *lst = a.nbr + row_index(r, a.shape);
     nbr_loop<U>(lst, n > 0 ? n - 1 : 0, [&](uint32_t j) { return ldg4(a.pos + j); },
                 [&](uint32_t j, const float4 &q) {
                     const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
@@ -149,6 +150,58 @@ __global__ void __launch_bounds__(256) k_ratio_alpha(DfsphArgs a) {
                 });
     a.ratio[r] = ra.ratio;
     a.alpha[r] = ra.alpha(a.mass_f);
+}
+
+// The same with a team per row (team.cuh).
+__global__ void __launch_bounds__(kTeamBlock) k_team_ratio_alpha(DfsphArgs a) {
+    __shared__ TeamTerms<8> S;   // V_j, W, gradW, |gradW|^2 V_j^2 (fluid j)
+    const uint32_t r = blockIdx.x * kTeamRows + team_row(), l = team_lane();
+    const bool live = r < a.nf && !halo_ghost(a, r);
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+    uint32_t n = 0;
+    if (live) {
+        p = a.pos[r];
+        n = a.ncnt[r];
+    }
+    const float inv_mf = __fdiv_rn(1.f, a.mass_f);
+    // lane 0: ratio, lanes 1..3: a1; every lane: a2
+    float acc = l == 0 && n > 0 ? __fmul_rn(p.w, a.k.w0) : 0.f, a2 = 1e-6f;
+    team_walk<8>(
+        S, a.nbr + ell_index(r, 0, a.shape), n > 0 ? n - 1 : 0, [&](uint32_t j) { return ldg4(a.pos + j); },
+        [&](uint32_t j, const float4 &q, float *o) {
+            const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+            float w, g;
+            cubic_wg(dist2(dx, dy, dz), a.k, w, g);
+            const float gx = __fmul_rn(g, dx), gy = __fmul_rn(g, dy), gz = __fmul_rn(g, dz);
+            o[0] = q.w;
+            o[1] = w;
+            o[2] = gx;
+            o[3] = gy;
+            o[4] = gz;
+            o[5] = j < a.nf ? __fmul_rn(__fmul_rn(dist2(gx, gy, gz), q.w), q.w) : 0.f;
+            o[6] = o[7] = 0.f;
+        },
+        [&](const float *e) {
+            acc = __fmaf_rn(e[0], e[1 + l], acc);
+            a2 = __fmaf_rn(e[5], inv_mf, a2);
+        });
+    RatioAlpha ra;
+    ra.ratio = acc;
+    ra.a1x = team_get(acc, 1);
+    ra.a1y = team_get(acc, 2);
+    ra.a1z = team_get(acc, 3);
+    ra.a2 = a2;
+    if (!live || l != 0) return;
+    a.ratio[r] = ra.ratio;
+    a.alpha[r] = ra.alpha(a.mass_f);
+}
+
+// V_j gradW_ij . (v*_i - v*_j) of a pair: e = {x_j, V_j}, v*_j.
+__device__ __forceinline__ float solve_a_term(const float4 &p, const float4 &vi, const F4x2 &e, const Cubic &k) {
+    const float rx = p.x - e.a.x, ry = p.y - e.a.y, rz = p.z - e.a.z;
+    const float g = cubic_g(dist2(rx, ry, rz), k);
+    const float dot = g * (rx * (vi.x - e.b.x) + ry * (vi.y - e.b.y) + rz * (vi.z - e.b.z));
+    return dot * e.a.w;
 }
 
 // Tile kernels run a persistent grid over the scene-offset tiles; a tile of a
@@ -169,15 +222,9 @@ __global__ void __launch_bounds__(256) k_solve_a(DfsphArgs a) {
             const float4 vi = a.vadv[r];
             const uint32_t n = a.ncnt[r];
             float d = a.ratio[r] - 1.f;
-            const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+            const uint32_t *lst = a.nbr + row_index(r, a.shape);
             nbr_loop<U>(lst, n > 0 ? n - 1 : 0, [&](uint32_t j) { return ldg8(a.pva + 2 * (size_t)j); },
-                        [&](uint32_t, const F4x2 &e) {
-                            const float rx = p.x - e.a.x, ry = p.y - e.a.y, rz = p.z - e.a.z;
-                            const float g = cubic_g(dist2(rx, ry, rz), a.k);
-                            const float dot =
-                                g * (rx * (vi.x - e.b.x) + ry * (vi.y - e.b.y) + rz * (vi.z - e.b.z));
-                            d = __fmaf_rn(dot * e.a.w, T.dt, d);
-                        });
+                        [&](uint32_t, const F4x2 &e) { d = __fmaf_rn(solve_a_term(p, vi, e, a.k), T.dt, d); });
             if (d < 0.f) d = 0.f;
             a.delta[r] = d;
             const float kap = d / a.alpha[r] * T.inv_dt2 / p.w;
@@ -200,6 +247,65 @@ __global__ void __launch_bounds__(256) k_solve_a(DfsphArgs a) {
                 double s = block_sum(obj == o ? contrib : 0.0);
                 if (threadIdx.x == 0) a.partials[(size_t)t * a.nobj_max + o] = s;
             }
+        }
+    }
+}
+
+// solve_a with a team per row: a block takes a 32-row piece of a tile (`pieces` per tile) and
+// leaves the sum of its rows' errors; k_solve_end adds a tile's pieces as the block sum above does.
+template <bool MULTI>
+__global__ void __launch_bounds__(kTeamBlock) k_team_solve_a(DfsphArgs a, uint32_t pieces) {
+    __shared__ TeamTerms<1> S;
+    __shared__ float err[kTeamRows];
+    const StepDt T = step_dt(a);
+    const uint32_t t = blockIdx.x / pieces, part = blockIdx.x - t * pieces;
+    const uint4 tile = a.tiles[t];
+    const bool stopped = a.state[tile.z].stopped != 0;
+    if (a.tile_ran && part == 0 && threadIdx.x == 0) a.tile_ran[t] = stopped ? 0u : 1u;
+    if (stopped) return;
+    const uint32_t row = part * kTeamRows + team_row(), r = tile.x + row;
+    const bool live = row < tile.y && !halo_ghost(a, r);
+    float4 p = make_float4(0.f, 0.f, 0.f, 1.f), vi = p;
+    float d = 0.f, al = 1.f;
+    uint32_t n = 0;
+    if (live) {
+        p = a.pos[r];
+        vi = a.vadv[r];
+        n = a.ncnt[r];
+        al = a.alpha[r];
+        d = a.ratio[r] - 1.f;
+    }
+    team_walk<1>(
+        S, a.nbr + ell_index(r, 0, a.shape), n > 0 ? n - 1 : 0,
+        [&](uint32_t j) { return ldg8(a.pva + 2 * (size_t)j); },
+        [&](uint32_t, const F4x2 &e, float *o) { o[0] = solve_a_term(p, vi, e, a.k); },
+        [&](const float *e) { d = __fmaf_rn(e[0], T.dt, d); });
+    if (d < 0.f) d = 0.f;
+    if (live && team_lane() == 0) {
+        a.delta[r] = d;
+        const float kap = d / al * T.inv_dt2 / p.w;
+        a.kappa[r] = kap;
+        const float4 pkr = make_float4(p.x, p.y, p.z, kap);
+        a.pk[r] = pkr;
+        halo_each(a, r, [&](const PeerRows &P, uint32_t q) {
+            P.kappa[q] = kap;
+            P.pk[q] = pkr;
+        });
+    }
+    if (team_lane() == 0) err[team_row()] = live ? d : 0.f;
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    const double contrib = (double)err[threadIdx.x];
+    if (!MULTI) {
+        const double s = warp_sum(contrib);
+        if (threadIdx.x == 0) a.partials[blockIdx.x] = s;
+    } else {
+        const uint32_t er = part * kTeamRows + threadIdx.x;
+        const int obj = er < tile.y ? (int)a.obj_of[a.orig[tile.x + er]] - (int)a.scene_tiles[tile.z].obj0 : 0;
+        const int no = (int)a.scene_tiles[tile.z].nobj;
+        for (int o = 0; o < no; ++o) {
+            const double s = warp_sum(obj == o ? contrib : 0.0);
+            if (threadIdx.x == 0) a.partials[(size_t)blockIdx.x * a.nobj_max + o] = s;
         }
     }
 }
@@ -258,7 +364,7 @@ __global__ void __launch_bounds__(kStageBlock) k_solve_a_staged(DfsphArgs a) {
         };
         const uint32_t cnt = n > 0 ? n - 1 : 0;
         if (staged) {
-            slot_loop<U>(a.stg.snbr + ell_index(r, 0, a.ell_stride), cnt,
+            slot_loop<U>(a.stg.snbr + ell_index(r, 0, a.shape), a.shape, cnt,
                          [&](uint16_t s) {
                              uint32_t q = (uint32_t)(s & 0x7fffu);
 #ifdef VTP_CHECKED
@@ -272,7 +378,7 @@ __global__ void __launch_bounds__(kStageBlock) k_solve_a_staged(DfsphArgs a) {
                          },
                          use);
         } else {
-            nbr_loop<U>(a.nbr + ell_index(r, 0, a.ell_stride), cnt,
+            nbr_loop_at<U>(a.nbr + ell_index(r, 0, a.shape), AnySlots{a.shape}, cnt,
                         [&](uint32_t j) { return ldg8(a.pva + 2 * (size_t)j); }, use);
         }
         if (d < 0.f) d = 0.f;
@@ -349,7 +455,7 @@ __global__ void __launch_bounds__(kStageBlock) k_solve_b_staged(DfsphArgs a) {
         };
         const uint32_t cnt = n > 0 ? n - 1 : 0;
         if (staged) {
-            slot_loop<U>(a.stg.snbr + ell_index(r, 0, a.ell_stride), cnt,
+            slot_loop<U>(a.stg.snbr + ell_index(r, 0, a.shape), a.shape, cnt,
                          [&](uint16_t s) {
                              uint32_t q = (uint32_t)(s & 0x7fffu);
 #ifdef VTP_CHECKED
@@ -362,12 +468,21 @@ __global__ void __launch_bounds__(kStageBlock) k_solve_b_staged(DfsphArgs a) {
                          },
                          [&](uint16_t s, const float4 &e) { step(!(s & kSlotBoundary), e); });
         } else {
-            nbr_loop<U>(a.nbr + ell_index(r, 0, a.ell_stride), cnt, [&](uint32_t j) { return ldg4(a.pk + j); },
+            nbr_loop_at<U>(a.nbr + ell_index(r, 0, a.shape), AnySlots{a.shape}, cnt, [&](uint32_t j) { return ldg4(a.pk + j); },
                         [&](uint32_t j, const float4 &e) { step(j < a.nf, e); });
         }
         a.vadv[r] = v;
         a.pva[2 * (size_t)r + 1] = v;
     }
+}
+
+// dt V_i / m_i V_j (kappa_i + kappa_j) g_ij of a pair.  Boundary kappa is 0 (kappa_div zeroed;
+// kappa_incomp never written for boundary); the packed row's w is kappa_j for fluid rows (volume
+// vol_f) and V_j for boundary rows.
+__device__ __forceinline__ float solve_b_factor(bool fj, float w, float d2, float ci, float ki, const DfsphArgs &a) {
+    const float Vj = fj ? a.vol_f : w, kj = fj ? w : 0.f;
+    const float g = cubic_g(d2, a.k);
+    return ci * Vj * (ki + kj) * g;
 }
 
 template <int U>
@@ -385,16 +500,11 @@ __global__ void __launch_bounds__(256) k_solve_b(DfsphArgs a) {
         const uint32_t n = a.ncnt[r];
         const float mi = a.rest_density ? a.rest_density[r] * p.w : a.mass_f;
         const float ci = T.dt * p.w / mi;   // dt V_i / m_i
-        const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
-        // Boundary kappa is 0 (kappa_div zeroed; kappa_incomp never written for boundary); the
-        // packed row carries kappa_j for fluid rows (volume vol_f) and V_j for boundary rows.
+        const uint32_t *lst = a.nbr + row_index(r, a.shape);
         nbr_loop<U>(lst, n > 0 ? n - 1 : 0, [&](uint32_t j) { return ldg4(a.pk + j); },
                     [&](uint32_t j, const float4 &e) {
-                        const bool fj = j < a.nf;
-                        const float Vj = fj ? a.vol_f : e.w, kj = fj ? e.w : 0.f;
                         const float rx = p.x - e.x, ry = p.y - e.y, rz = p.z - e.z;
-                        const float g = cubic_g(dist2(rx, ry, rz), a.k);
-                        const float s = ci * Vj * (ki + kj) * g;
+                        const float s = solve_b_factor(j < a.nf, e.w, dist2(rx, ry, rz), ci, ki, a);
                         v.x = __fmaf_rn(-s, rx, v.x);
                         v.y = __fmaf_rn(-s, ry, v.y);
                         v.z = __fmaf_rn(-s, rz, v.z);
@@ -405,6 +515,52 @@ __global__ void __launch_bounds__(256) k_solve_b(DfsphArgs a) {
             P.vadv[a.halo_vadv][q] = v;
             P.pva[2 * (size_t)q + 1] = v;
         });
+    }
+}
+
+// solve_b with a team per row: lanes 0..2 carry a velocity component each.
+__global__ void __launch_bounds__(kTeamBlock) k_team_solve_b(DfsphArgs a, uint32_t pieces) {
+    __shared__ TeamTerms<4> S;   // -s, x_i - x_j
+    const StepDt T = step_dt(a);
+    const uint32_t t = blockIdx.x / pieces, part = blockIdx.x - t * pieces, l = team_lane();
+    const uint4 tile = a.tiles[t];
+    if (a.tile_ran ? a.tile_ran[t] == 0u : (a.state && a.state[tile.z].stopped)) return;
+    const uint32_t row = part * kTeamRows + team_row(), r = tile.x + row;
+    const bool live = row < tile.y && !halo_ghost(a, r);
+    float4 p = make_float4(0.f, 0.f, 0.f, 1.f);
+    float ki = 0.f, ci = 0.f, v = 0.f;
+    uint32_t n = 0;
+    if (live) {
+        p = a.pos[r];
+        ki = a.kappa[r];
+        n = a.ncnt[r];
+        v = reinterpret_cast<const float *>(a.vadv + r)[l];
+        const float mi = a.rest_density ? a.rest_density[r] * p.w : a.mass_f;
+        ci = T.dt * p.w / mi;   // dt V_i / m_i
+    }
+    const float w = v;   // lane 3: the fourth word, kept
+    const uint32_t c = l < 3 ? 1 + l : 1;
+    team_walk<4>(
+        S, a.nbr + ell_index(r, 0, a.shape), n > 0 ? n - 1 : 0, [&](uint32_t j) { return ldg4(a.pk + j); },
+        [&](uint32_t j, const float4 &e, float *o) {
+            o[1] = p.x - e.x;
+            o[2] = p.y - e.y;
+            o[3] = p.z - e.z;
+            o[0] = -solve_b_factor(j < a.nf, e.w, dist2(o[1], o[2], o[3]), ci, ki, a);
+        },
+        [&](const float *e) { v = __fmaf_rn(e[0], e[c], v); });
+    if (l == 3) v = w;
+    if (live) {
+        reinterpret_cast<float *>(a.vadv + r)[l] = v;
+        reinterpret_cast<float *>(a.pva + 2 * (size_t)r + 1)[l] = v;
+    }
+    if (a.halo) {
+        const float4 o = make_float4(team_get(v, 0), team_get(v, 1), team_get(v, 2), team_get(v, 3));
+        if (live && l == 0)
+            halo_each(a, r, [&](const PeerRows &P, uint32_t q) {
+                P.vadv[a.halo_vadv][q] = o;
+                P.pva[2 * (size_t)q + 1] = o;
+            });
     }
 }
 
@@ -445,6 +601,19 @@ __global__ void k_solve_begin(SolveState *s, LoopState *loop, int nscenes) {
     }
 }
 
+// A tile's sum from the sums of its 32-row pieces, in the order a block sum over the tile adds its
+// warps (block_sum: halving strides).
+__device__ __forceinline__ double tile_sum(const double *__restrict__ part, uint32_t pieces, int stride) {
+    double v[8];
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q) v[q] = q < pieces ? part[(size_t)q * stride] : 0.0;
+#pragma unroll
+    for (uint32_t o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (uint32_t q = 0; q < o; ++q) v[q] += v[q + o];
+    return v[0];
+}
+
 // One block per scene: FP64 residual of the scene from its tiles' partials,
 // the stop test, and (last block to finish) the loop condition.
 __global__ void __launch_bounds__(1024) k_solve_end(SolveCtl c, const double *__restrict__ partials,
@@ -458,19 +627,25 @@ __global__ void __launch_bounds__(1024) k_solve_end(SolveCtl c, const double *__
     if (!was_stopped) {
         double acc = 0.0;
         for (uint32_t o = 0; o < sct.nobj; ++o) {
-            // Each thread adds the partials b = tid, tid + blockDim, ... in that order; the
-            // loads are issued eight at a time so that their latencies overlap.
+            // Each thread adds the tiles b = tid, tid + blockDim, ... in that order; the loads of
+            // several tiles are issued together so that their latencies overlap.
             double s = 0.0;
-            for (uint32_t b = threadIdx.x; b < sct.ntiles; b += 8u * blockDim.x) {
-                double v[8];
+            const uint32_t np = c.pieces;
+            if (np == 1u) {
+                for (uint32_t b = threadIdx.x; b < sct.ntiles; b += 8u * blockDim.x) {
+                    double v[8];
 #pragma unroll
-                for (uint32_t u = 0; u < 8; ++u) {
-                    const uint32_t bb = b + u * blockDim.x;
-                    v[u] = bb < sct.ntiles ? partials[(size_t)(sct.tile0 + bb) * c.nobj_max + o] : 0.0;
+                    for (uint32_t u = 0; u < 8; ++u) {
+                        const uint32_t bb = b + u * blockDim.x;
+                        v[u] = bb < sct.ntiles ? partials[(size_t)(sct.tile0 + bb) * c.nobj_max + o] : 0.0;
+                    }
+#pragma unroll
+                    for (uint32_t u = 0; u < 8; ++u)
+                        if (b + u * blockDim.x < sct.ntiles) s += v[u];
                 }
-#pragma unroll
-                for (uint32_t u = 0; u < 8; ++u)
-                    if (b + u * blockDim.x < sct.ntiles) s += v[u];
+            } else {   // the passes with a team per row leave a partial per 32 rows of a tile
+                for (uint32_t b = threadIdx.x; b < sct.ntiles; b += blockDim.x)
+                    s += tile_sum(partials + (size_t)(sct.tile0 + b) * np * c.nobj_max + o, np, c.nobj_max);
             }
             s = block_sum(s);
             if (threadIdx.x == 0) acc += s * c.inv_count[sct.obj0 + o];
@@ -518,6 +693,62 @@ __global__ void __launch_bounds__(1024) k_solve_end(SolveCtl c, const double *__
     }
 }
 
+// Gravity and the viscosity sum a* of row r (velocity vi after the pressure step): the new velocity,
+// or (surface tension on) the acceleration and the normal n* for the tension pass.
+template <bool TENSION_SPLIT>
+__device__ __forceinline__ void finish_viscosity(const DfsphArgs &a, const StepDt &T, uint32_t r, const float4 &vi,
+                                                 float ax, float ay, float az, float nx, float ny, float nz) {
+    const SceneGrid &sg = a.sc.sg[a.sc.row_scene[r]];
+    const float accx = sg.grav_x + ax, accy = sg.grav_y + ay, accz = sg.grav_z + az;
+    if (TENSION_SPLIT) {
+        a.acc_tmp[r] = make_float4(accx, accy, accz, 0.f);
+        const float4 nrm = make_float4(nx, ny, nz, 0.f);
+        a.normal[r] = nrm;
+        halo_each(a, r, [&](const PeerRows &P, uint32_t q) { P.normal[q] = nrm; });
+        return;
+    }
+    float4 o = vi;
+    o.x = __fmaf_rn(accx, T.dt, vi.x);
+    o.y = __fmaf_rn(accy, T.dt, vi.y);
+    o.z = __fmaf_rn(accz, T.dt, vi.z);
+    a.vel_alt[r] = o;
+    a.vadv_alt[r] = o;
+    halo_each(a, r, [&](const PeerRows &P, uint32_t q) {
+        P.vel[a.halo_vel ^ 1][q] = o;
+        P.vadv[a.halo_vadv ^ 1][q] = o;
+    });
+}
+
+// The tension acceleration of row r added to what the viscosity pass kept: the new velocity.
+__device__ __forceinline__ void finish_tension(const DfsphArgs &a, const StepDt &T, uint32_t r, float tx, float ty,
+                                               float tz) {
+    const float4 vi = pressure_applied(a.vel[r], a.vadv[r], T.inv_dt, T.dt);
+    const float4 acc = a.acc_tmp[r];
+    float4 o = vi;
+    o.x = __fmaf_rn(acc.x + tx, T.dt, vi.x);
+    o.y = __fmaf_rn(acc.y + ty, T.dt, vi.y);
+    o.z = __fmaf_rn(acc.z + tz, T.dt, vi.z);
+    a.vel_alt[r] = o;
+    a.vadv_alt[r] = o;
+    halo_each(a, r, [&](const PeerRows &P, uint32_t q) {
+        P.vel[a.halo_vel ^ 1][q] = o;
+        P.vadv[a.halo_vadv ^ 1][q] = o;
+    });
+}
+
+// Cohesion and normal difference of a pair of fluid rows.
+__device__ __forceinline__ void tension_term(const DfsphArgs &a, const float4 &p, const float4 &ni, const PN &e, float &x,
+                                             float &y, float &z) {
+    const float c1 = -a.gamma * a.mass_f * a.mass_f;
+    const float c2 = -a.gamma * a.mass_f;
+    const float rx = p.x - e.q.x, ry = p.y - e.q.y, rz = p.z - e.q.z;
+    const float rl = sqrtf(dist2(rx, ry, rz));
+    const float cs = c1 * tension_c(rl, a.k.h, a.csigma, a.h6_64) / rl;
+    x = cs * rx + c2 * (ni.x - e.n.x);
+    y = cs * ry + c2 * (ni.y - e.n.y);
+    z = cs * rz + c2 * (ni.z - e.n.z);
+}
+
 template <bool TENSION_SPLIT, int U>
 __global__ void __launch_bounds__(256) k_viscosity(DfsphArgs a) {
     const StepDt T = step_dt(a);
@@ -529,7 +760,7 @@ __global__ void __launch_bounds__(256) k_viscosity(DfsphArgs a) {
     float ax = 0.f, ay = 0.f, az = 0.f;
     float nx = 0.f, ny = 0.f, nz = 0.f;
     const float ncoef = a.k.h * a.mass_f / a.rho0;   // h m_j / rho_rest_j (fluid)
-    const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+    const uint32_t *lst = a.nbr + row_index(r, a.shape);
     nbr_loop<U>(lst, n > 0 ? n - 1 : 0,
                 [&](uint32_t j) {
                     if (j >= a.nf) return F4x2{};   // same-material neighbours only
@@ -554,25 +785,7 @@ __global__ void __launch_bounds__(256) k_viscosity(DfsphArgs a) {
                         nz = __fmaf_rn(sn, rz, nz);
                     }
                 });
-    const SceneGrid &sg = a.sc.sg[a.sc.row_scene[r]];
-    const float accx = sg.grav_x + ax, accy = sg.grav_y + ay, accz = sg.grav_z + az;
-    if (TENSION_SPLIT) {
-        a.acc_tmp[r] = make_float4(accx, accy, accz, 0.f);
-        const float4 nrm = make_float4(nx, ny, nz, 0.f);
-        a.normal[r] = nrm;
-        halo_each(a, r, [&](const PeerRows &P, uint32_t q) { P.normal[q] = nrm; });
-        return;
-    }
-    float4 o = vi;
-    o.x = __fmaf_rn(accx, T.dt, vi.x);
-    o.y = __fmaf_rn(accy, T.dt, vi.y);
-    o.z = __fmaf_rn(accz, T.dt, vi.z);
-    a.vel_alt[r] = o;
-    a.vadv_alt[r] = o;
-    halo_each(a, r, [&](const PeerRows &P, uint32_t q) {
-        P.vel[a.halo_vel ^ 1][q] = o;
-        P.vadv[a.halo_vadv ^ 1][q] = o;
-    });
+    finish_viscosity<TENSION_SPLIT>(a, T, r, vi, ax, ay, az, nx, ny, nz);
 }
 
 template <int U>
@@ -581,15 +794,12 @@ __global__ void __launch_bounds__(256) k_tension(DfsphArgs a) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= a.nf || halo_ghost(a, r)) return;
     const float4 p = a.pos[r];
-    const float4 vi = pressure_applied(a.vel[r], a.vadv[r], T.inv_dt, T.dt);
     const float4 ni = a.normal[r];
     const uint32_t n = a.ncnt[r];
     // Fluid rest densities are equal, so k = 2 rho_i / (rho_i + rho_j) is evaluated once.
     const float kk = 2.f * a.rho0 / (a.rho0 + a.rho0);
-    const float c1 = -a.gamma * a.mass_f * a.mass_f;
-    const float c2 = -a.gamma * a.mass_f;
     float tx = 0.f, ty = 0.f, tz = 0.f;
-    const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+    const uint32_t *lst = a.nbr + row_index(r, a.shape);
     nbr_loop<U>(lst, n > 0 ? n - 1 : 0,
                 [&](uint32_t j) {
                     if (j >= a.nf) return PN{};
@@ -597,24 +807,93 @@ __global__ void __launch_bounds__(256) k_tension(DfsphArgs a) {
                 },
                 [&](uint32_t j, const PN &e) {
                     if (j >= a.nf) return;
-                    const float rx = p.x - e.q.x, ry = p.y - e.q.y, rz = p.z - e.q.z;
-                    const float rl = sqrtf(dist2(rx, ry, rz));
-                    const float cs = c1 * tension_c(rl, a.k.h, a.csigma, a.h6_64) / rl;
-                    tx += kk * (cs * rx + c2 * (ni.x - e.n.x));
-                    ty += kk * (cs * ry + c2 * (ni.y - e.n.y));
-                    tz += kk * (cs * rz + c2 * (ni.z - e.n.z));
+                    float x, y, z;
+                    tension_term(a, p, ni, e, x, y, z);
+                    tx += kk * x;
+                    ty += kk * y;
+                    tz += kk * z;
                 });
-    const float4 acc = a.acc_tmp[r];
-    float4 o = vi;
-    o.x = __fmaf_rn(acc.x + tx, T.dt, vi.x);
-    o.y = __fmaf_rn(acc.y + ty, T.dt, vi.y);
-    o.z = __fmaf_rn(acc.z + tz, T.dt, vi.z);
-    a.vel_alt[r] = o;
-    a.vadv_alt[r] = o;
-    halo_each(a, r, [&](const PeerRows &P, uint32_t q) {
-        P.vel[a.halo_vel ^ 1][q] = o;
-        P.vadv[a.halo_vadv ^ 1][q] = o;
-    });
+    finish_tension(a, T, r, tx, ty, tz);
+}
+
+// The viscosity and tension passes with a team per row.
+template <bool TENSION_SPLIT>
+__global__ void __launch_bounds__(kTeamBlock) k_team_viscosity(DfsphArgs a) {
+    constexpr int W = TENSION_SPLIT ? 8 : 4;
+    __shared__ TeamTerms<W> S;   // viscosity factor, x_i - x_j, normal factor
+    const StepDt T = step_dt(a);
+    const uint32_t r = blockIdx.x * kTeamRows + team_row(), l = team_lane();
+    const bool live = r < a.nf && !halo_ghost(a, r);
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f), vi = p;
+    uint32_t n = 0;
+    if (live) {
+        p = a.pos[r];
+        vi = pressure_applied(a.vel[r], a.vadv[r], T.inv_dt, T.dt);
+        n = a.ncnt[r];
+    }
+    const float ncoef = a.k.h * a.mass_f / a.rho0;   // h m_j / rho_rest_j (fluid)
+    float acc = 0.f, nrm = 0.f;
+    const uint32_t c = l < 3 ? 1 + l : 1;
+    team_walk<W>(
+        S, a.nbr + ell_index(r, 0, a.shape), n > 0 ? n - 1 : 0,
+        [&](uint32_t j) {
+            if (j >= a.nf) return F4x2{};   // same-material neighbours only
+            return ldg8(a.pva + 2 * (size_t)j);
+        },
+        [&](uint32_t j, const F4x2 &e, float *o) {
+            const float rx = p.x - e.a.x, ry = p.y - e.a.y, rz = p.z - e.a.z;
+            const float d2 = dist2(rx, ry, rz);
+            const float g = cubic_g(d2, a.k);
+            const float4 vj = e.b;
+            const float vx = vi.x - vj.x, vy = vi.y - vj.y, vz = vi.z - vj.z;
+            const float pi = a.vis_coef * (vx * rx + vy * ry + vz * rz) / (d2 + a.h2_001);
+            const bool fluid = j < a.nf;   // a boundary neighbour adds nothing
+            o[0] = fluid ? 10.f * pi * g : 0.f;
+            o[1] = rx;
+            o[2] = ry;
+            o[3] = rz;
+            if constexpr (TENSION_SPLIT) {
+                o[4] = fluid ? ncoef * g : 0.f;
+                o[5] = o[6] = o[7] = 0.f;
+            }
+        },
+        [&](const float *e) {
+            acc = __fmaf_rn(e[0], e[c], acc);
+            if constexpr (TENSION_SPLIT) nrm = __fmaf_rn(e[4], e[c], nrm);
+        });
+    const float ax = team_get(acc, 0), ay = team_get(acc, 1), az = team_get(acc, 2);
+    const float nx = team_get(nrm, 0), ny = team_get(nrm, 1), nz = team_get(nrm, 2);
+    if (!live || l != 0) return;
+    finish_viscosity<TENSION_SPLIT>(a, T, r, vi, ax, ay, az, nx, ny, nz);
+}
+
+__global__ void __launch_bounds__(kTeamBlock) k_team_tension(DfsphArgs a) {
+    __shared__ TeamTerms<4> S;
+    const StepDt T = step_dt(a);
+    const uint32_t r = blockIdx.x * kTeamRows + team_row(), l = team_lane();
+    const bool live = r < a.nf && !halo_ghost(a, r);
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f), ni = p;
+    uint32_t n = 0;
+    if (live) {
+        p = a.pos[r];
+        ni = a.normal[r];
+        n = a.ncnt[r];
+    }
+    const float kk = 2.f * a.rho0 / (a.rho0 + a.rho0);
+    float acc = 0.f;
+    team_walk<4>(
+        S, a.nbr + ell_index(r, 0, a.shape), n > 0 ? n - 1 : 0,
+        [&](uint32_t j) {
+            if (j >= a.nf) return PN{};
+            return PN{ldg4(a.pos + j), ldg4(a.normal + j)};
+        },
+        [&](uint32_t j, const PN &e, float *o) {
+            o[0] = o[1] = o[2] = o[3] = 0.f;
+            if (j < a.nf) tension_term(a, p, ni, e, o[0], o[1], o[2]);
+        },
+        [&](const float *e) { acc += kk * e[l]; });
+    const float tx = team_get(acc, 0), ty = team_get(acc, 1), tz = team_get(acc, 2);
+    if (live && l == 0) finish_tension(a, T, r, tx, ty, tz);
 }
 
 __global__ void __launch_bounds__(256) k_finalize(DfsphArgs a) {
@@ -702,7 +981,9 @@ void dfsph_rigid_volume(cudaStream_t st, const DfsphArgs &a, const uint32_t *bnc
     }
 
 void dfsph_ratio_alpha(cudaStream_t st, const DfsphArgs &a, int block) {
-    if (a.nf) VTP_UNROLL_DISPATCH(a.unroll, k_ratio_alpha<UU><<<nblk(a.nf, block), block, 0, st>>>(a))
+    if (!a.nf) return;
+    if (a.teams) k_team_ratio_alpha<<<nblk(a.nf, kTeamRows), kTeamBlock, 0, st>>>(a);
+    else VTP_UNROLL_DISPATCH(a.unroll, k_ratio_alpha<UU><<<nblk(a.nf, block), block, 0, st>>>(a))
 }
 void dfsph_solve_begin(cudaStream_t st, SolveState *s, LoopState *loop, int nscenes) {
     k_solve_begin<<<1, 256, 0, st>>>(s, loop, nscenes);
@@ -725,6 +1006,13 @@ void dfsph_solve_a(cudaStream_t st, const DfsphArgs &a, int block) {
         else VTP_UNROLL_DISPATCH(a.unroll, launch_staged(k_solve_a_staged<false, UU>, st, a, 32))
         return;
     }
+    if (a.teams) {
+        const uint32_t pieces = solve_pieces(block), n = a.ntiles * pieces;
+        if (!n) return;
+        if (a.nobj_max > 1) k_team_solve_a<true><<<n, kTeamBlock, 0, st>>>(a, pieces);
+        else k_team_solve_a<false><<<n, kTeamBlock, 0, st>>>(a, pieces);
+        return;
+    }
     const unsigned nb = dfsph_tile_grid(a.ntiles, block, a.persistent);
     if (a.nobj_max > 1) VTP_UNROLL_DISPATCH(a.unroll, k_solve_a<true, UU><<<nb, block, 0, st>>>(a))
     else VTP_UNROLL_DISPATCH(a.unroll, k_solve_a<false, UU><<<nb, block, 0, st>>>(a))
@@ -732,6 +1020,11 @@ void dfsph_solve_a(cudaStream_t st, const DfsphArgs &a, int block) {
 void dfsph_solve_b(cudaStream_t st, const DfsphArgs &a, int block) {
     if (a.staged) {
         VTP_UNROLL_DISPATCH(a.unroll, launch_staged(k_solve_b_staged<UU>, st, a, 16))
+        return;
+    }
+    if (a.teams) {
+        const uint32_t pieces = solve_pieces(block), n = a.ntiles * pieces;
+        if (n) k_team_solve_b<<<n, kTeamBlock, 0, st>>>(a, pieces);
         return;
     }
     const unsigned nb = dfsph_tile_grid(a.ntiles, block, a.persistent);
@@ -755,13 +1048,19 @@ void dfsph_pressure_pack(cudaStream_t st, const DfsphArgs &a) {
     if (a.nf) k_pressure_pack<<<nblk(a.nf, 256), 256, 0, st>>>(a);
 }
 void dfsph_viscosity(cudaStream_t st, const DfsphArgs &a, int block) {
-    if (a.nf) VTP_UNROLL_DISPATCH(a.unroll, k_viscosity<false, UU><<<nblk(a.nf, block), block, 0, st>>>(a))
+    if (!a.nf) return;
+    if (a.teams) k_team_viscosity<false><<<nblk(a.nf, kTeamRows), kTeamBlock, 0, st>>>(a);
+    else VTP_UNROLL_DISPATCH(a.unroll, k_viscosity<false, UU><<<nblk(a.nf, block), block, 0, st>>>(a))
 }
 void dfsph_vis_normal(cudaStream_t st, const DfsphArgs &a, int block) {
-    if (a.nf) VTP_UNROLL_DISPATCH(a.unroll, k_viscosity<true, UU><<<nblk(a.nf, block), block, 0, st>>>(a))
+    if (!a.nf) return;
+    if (a.teams) k_team_viscosity<true><<<nblk(a.nf, kTeamRows), kTeamBlock, 0, st>>>(a);
+    else VTP_UNROLL_DISPATCH(a.unroll, k_viscosity<true, UU><<<nblk(a.nf, block), block, 0, st>>>(a))
 }
 void dfsph_tension(cudaStream_t st, const DfsphArgs &a, int block) {
-    if (a.nf) VTP_UNROLL_DISPATCH(a.unroll, k_tension<UU><<<nblk(a.nf, block), block, 0, st>>>(a))
+    if (!a.nf) return;
+    if (a.teams) k_team_tension<<<nblk(a.nf, kTeamRows), kTeamBlock, 0, st>>>(a);
+    else VTP_UNROLL_DISPATCH(a.unroll, k_tension<UU><<<nblk(a.nf, block), block, 0, st>>>(a))
 }
 void dfsph_finalize(cudaStream_t st, const DfsphArgs &a) {
     if (a.nf) k_finalize<<<nblk(a.nf, 256), 256, 0, st>>>(a);

@@ -37,7 +37,7 @@ struct SceneTiles {
 
 struct DfsphArgs {
     uint32_t nf, nb;
-    uint32_t ell_stride;
+    ListShape shape;
     Cubic k;
     float dt, inv_dt, inv_dt2;
     float rho0, rho_b, mass_f, vol_f;
@@ -54,7 +54,7 @@ struct DfsphArgs {
     const uint32_t *orig;       // sorted row -> attach id
     const uint16_t *obj_of;     // attach id -> fluid object slot (multi-object scenes only)
     int nobj_max;               // most fluid objects in one scene (>= 1)
-    double *partials;           // [tiles][nobj_max]
+    double *partials;           // [tiles][nobj_max]; a team per row: [tiles][solve_pieces][nobj_max]
     const uint4 *tiles;         // {row0, rows, scene, 0}
     uint32_t ntiles;
     bool persistent;            // persistent grid over the tiles
@@ -76,6 +76,7 @@ struct DfsphArgs {
     // its neighbours from a shared-memory copy of the group's neighbourhood through the slot
     // lists; the residual partials are then per group (ngroups + 1 entries, the last for the
     // rows outside the grid).
+    bool teams;                 // neighbour passes walk a row with a team of lanes (team.cuh)
     int staged;
     Staging stg;
     const float *dtp;           // adaptive time step (CFL) on the device; null: the fixed dt above
@@ -84,13 +85,17 @@ struct DfsphArgs {
     int halo_vadv, halo_vel;    // current buffer index of vadv / vel (the peers' parity equals ours)
 };
 
+// 32-row pieces of a tile of `block` rows, each with its residual partial, where a team walks each row.
+constexpr uint32_t solve_pieces(int block) { return (uint32_t)block / 32u; }
+
 struct SolveCtl {
     SolveState *state;          // [S]
     LoopState *loop;
     const double *inv_count;    // [fluid objects] 1 / object size
     const SceneTiles *scene_tiles;  // [S]
     int nscenes;
-    int nobj_max;               // partials per tile
+    int nobj_max;               // partials per piece
+    uint32_t pieces;            // pieces per tile: solve_pieces with a team per row, else 1
     float threshold;
     uint32_t force_iters;       // 0 = residual test
     const uint32_t *force_seq;  // optional per-substep [div, incomp] counts (device)

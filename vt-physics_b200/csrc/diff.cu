@@ -135,7 +135,8 @@ struct DN {
 };
 
 struct AdjArgs {
-    uint32_t nf, ell_stride;
+    uint32_t nf;
+    ListShape shape;
     Cubic k;
     float dt, inv_dt, rho0, eps, c;
     const uint32_t *nbr, *ncnt, *orig;
@@ -180,9 +181,9 @@ __global__ void __launch_bounds__(256) k_adj_xsph(AdjArgs a) {
         const float4 p = a.x[r], vi = a.v[r], ai = a.abar[r];
         const float Vi = a.vol[r];
         const uint32_t n = a.ncnt[r];
-        const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+        const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
         float vx = 0.f, vy = 0.f, vz = 0.f, xx = 0.f, xy = 0.f, xz = 0.f, ksum = 0.f;
-        nbr_loop_lanes<adj_unroll<L>(), L>(lst, n > 0 ? n - 1 : 0, lane,
+        nbr_loop_lanes<adj_unroll<L>(), L>(lst, a.shape, n > 0 ? n - 1 : 0, lane,
                              [&](uint32_t j) {
                                  XN e;
                                  e.q = __ldg(a.x + j);
@@ -237,10 +238,10 @@ __global__ void __launch_bounds__(256) k_adj_lambda(AdjArgs a) {
     if (r >= a.nf) return;   // the same for every lane of the row
     const float4 p = a.x[r], di = a.Dcur[r];
     const uint32_t n = a.ncnt[r];
-    const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+    const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
     const float ir = 1.f / a.rho0;
     float lb = 0.f, gx = 0.f, gy = 0.f, gz = 0.f, s2 = 0.f;
-    nbr_loop_lanes<adj_unroll<L>(), L>(lst, n > 0 ? n - 1 : 0, lane,
+    nbr_loop_lanes<adj_unroll<L>(), L>(lst, a.shape, n > 0 ? n - 1 : 0, lane,
                          [&](uint32_t j) {
                              LN e;
                              e.q = __ldg(a.x + j);
@@ -279,10 +280,10 @@ __global__ void __launch_bounds__(256) k_adj_dx(AdjArgs a) {
     const float4 p = a.x[r], di = a.Dcur[r], Ai = a.A2[r];
     const float li = a.lam[r], sbi = a.sbar[r];
     const uint32_t n = a.ncnt[r];
-    const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+    const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
     const float ir = 1.f / a.rho0;
     float ax = 0.f, ay = 0.f, az = 0.f;
-    nbr_loop_lanes<adj_unroll<L>(), L>(lst, n > 0 ? n - 1 : 0, lane,
+    nbr_loop_lanes<adj_unroll<L>(), L>(lst, a.shape, n > 0 ? n - 1 : 0, lane,
                          [&](uint32_t j) {
                              DN e;
                              e.q = __ldg(a.x + j);
@@ -355,7 +356,8 @@ __global__ void k_adj_kreduce(const double *part, uint32_t nb, double *acc) {
 // P_i = 1 / (alpha_i dt^2 V_i) (vf_update_vel_adv_from_kappa_*, compute_kappa_*,
 // DFSPHCudaImpl.cu:142-220); the clamp pattern of each iteration is recorded.
 struct DfAdjArgs {
-    uint32_t nf, ell_stride;
+    uint32_t nf;
+    ListShape shape;
     Cubic k;
     float dt, inv_dt2, mass_f;
     const uint32_t *nbr, *ncnt;
@@ -372,10 +374,10 @@ __global__ void __launch_bounds__(256) k_dadj_kappa(DfAdjArgs a) {
     const float4 p = a.pos[r], vi = a.vb[r];
     const float ci = a.dt * p.w / a.mass_f;
     const uint32_t n = a.ncnt[r];
-    const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+    const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
     float s = 0.f;
     for (uint32_t t = 0; t + 1 < n; ++t) {
-        const uint32_t j = lst[(size_t)t * 32u];
+        const uint32_t j = lst[ell_slot(t, a.shape)];
         const float4 q = a.pos[j];
         const float rx = p.x - q.x, ry = p.y - q.y, rz = p.z - q.z;
         const float g = cubic_g(dist2(rx, ry, rz), a.k);
@@ -395,10 +397,10 @@ __global__ void __launch_bounds__(256) k_dadj_vel(DfAdjArgs a) {
     const float4 p = a.pos[r];
     const float ki = a.kb[r];
     const uint32_t n = a.ncnt[r];
-    const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+    const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
     float ax = 0.f, ay = 0.f, az = 0.f;
     for (uint32_t t = 0; t + 1 < n; ++t) {
-        const uint32_t j = lst[(size_t)t * 32u];
+        const uint32_t j = lst[ell_slot(t, a.shape)];
         const float4 q = a.pos[j];
         const float rx = p.x - q.x, ry = p.y - q.y, rz = p.z - q.z;
         const float g = cubic_g(dist2(rx, ry, rz), a.k);
@@ -481,7 +483,7 @@ int adjoint_segment_l(vtp_solver *s, vtp::DiffState &d, uint32_t k, unsigned G, 
     for (int t = (int)k - 1; t >= 0 && nf; --t) {
         const PbfTapeSlot &T = d.tapes[tp][t];
         vtp::AdjArgs a{};
-        a.nf = nf; a.ell_stride = s->L.ell_stride; a.k = s->kc;
+        a.nf = nf; a.shape = s->L.shape; a.k = s->kc;
         a.dt = s->dt; a.inv_dt = 1.f / s->dt; a.rho0 = s->rho_f; a.eps = 1e-6f; a.c = s->xsph_k;
         a.nbr = T.nbr; a.ncnt = T.ncnt; a.orig = T.orig;
         a.v = T.v; a.vol = s->vol;
@@ -577,7 +579,7 @@ int vtp_solver_diff_forward(vtp_solver *s, uint32_t n_steps, uint32_t checkpoint
     const uint32_t every = std::min(checkpoint_every, n_steps);
     const uint32_t nchk_all = (n_steps + every - 1) / every;
     const int I_it = s->iterations;
-    const size_t lrows_all = ((size_t)s->L.nf + 31) / 32 * 32 * s->L.ell_stride;
+    const size_t lrows_all = ((size_t)s->L.nf + 31) / 32 * 32 * s->L.shape.stride;
     const size_t slot_bytes = 4 * (size_t)s->L.nf * 2 + 4 * lrows_all + 16 * (size_t)s->L.n * (I_it + 2) +
                               8 * (size_t)s->L.nf * I_it;
     const size_t tape_bytes = std::max<size_t>(slot_bytes * every, 1);
@@ -603,7 +605,7 @@ int vtp_solver_diff_forward(vtp_solver *s, uint32_t n_steps, uint32_t checkpoint
     d->n = s->L.n;
     const uint32_t nchk = (n_steps + d->every - 1) / d->every;
     const size_t nf = std::max<uint32_t>(d->nf, 1), n = d->n;
-    const size_t lrows = ((size_t)d->nf + 31) / 32 * 32 * s->L.ell_stride;
+    const size_t lrows = ((size_t)d->nf + 31) / 32 * 32 * s->L.shape.stride;
     d->ck_pos.resize(nchk + 1);
     d->ck_vel.resize(nchk + 1);
     d->ck_orig.resize(nchk + 1);
@@ -875,7 +877,7 @@ int vtp_solver_dfsph_solve_forward(vtp_solver *s, int which, const float *v_in, 
                                      s->d_overflow);
     else
         vtp::ugns_build_lists(s->st, s->scn(), s->L, 0, nf, s->pos.c(), s->orig.c(), s->u, s->u.nbr, s->u.ncnt,
-                              s->d_status, s->d_overflow, s->block);
+                              s->d_status, s->d_overflow);
     vtp::dfsph_ratio_alpha(s->st, s->dfsph_args(which), s->block);
     const size_t n3 = (size_t)n * 3 * sizeof(float);
     if ((rc = s->ensure_stage(n3))) return rc;
@@ -933,7 +935,7 @@ int vtp_solver_dfsph_solve_backward(vtp_solver *s, const float *vbar_out, float 
     CU(cudaMemcpyAsync(s->stage, vbar_out, n3, cudaMemcpyHostToDevice, s->st));
     vtp::gather_orig_to_f4(s->st, nf, s->stage, s->orig.c(), d.df_vb, 0);
     vtp::DfAdjArgs a{};
-    a.nf = nf; a.ell_stride = s->L.ell_stride; a.k = s->kc;
+    a.nf = nf; a.shape = s->L.shape; a.k = s->kc;
     a.dt = s->dt; a.inv_dt2 = s->inv_dt2; a.mass_f = s->rho_f * s->vol0;
     a.nbr = s->u.nbr; a.ncnt = s->u.ncnt; a.pos = s->pos.c(); a.alpha = s->alpha;
     a.vb = d.df_vb; a.kb = d.df_kb;

@@ -132,7 +132,8 @@ __device__ __forceinline__ double block_sum_d(double v) {
 }
 
 struct DfdArgs {
-    uint32_t nf, ell_stride;
+    uint32_t nf;
+    ListShape shape;
     Cubic k;
     float dt, mass_f, vis10;   // vis10 = 10 nu V_f (the viscosity pair factor C)
     float eps;                 // 0.001 h^2
@@ -233,9 +234,9 @@ __global__ void __launch_bounds__(256) k_dfd_iter_a(DfdArgs a) {
         ki = a.rec[r].w;
         const float ci = a.dt * p.w / a.mass_f;
         const uint32_t n = a.ncnt[r];
-        const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+        const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
         for (uint32_t t = lane; t + 1 < n; t += L) {
-            const uint32_t j = lst[(size_t)t * 32u];
+            const uint32_t j = lst[ell_slot(t, a.shape)];
             const float4 q = __ldg(a.x + j);
             const bool fj = j < a.nf;
             const float kj = __ldg(&a.rec[j].w);   // 0 for boundary rows
@@ -286,9 +287,9 @@ __global__ void __launch_bounds__(256) k_dfd_iter_b(DfdArgs a) {
         const float4 p = a.x[r], si = a.rec[r];
         const float di = a.db[r];
         const uint32_t n = a.ncnt[r];
-        const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+        const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
         for (uint32_t t = lane; t + 1 < n; t += L) {
-            const uint32_t j = lst[(size_t)t * 32u];
+            const uint32_t j = lst[ell_slot(t, a.shape)];
             const float4 q = __ldg(a.x + j), sj = __ldg(a.rec + j);
             const float rx = p.x - q.x, ry = p.y - q.y, rz = p.z - q.z;
             const float d2 = dist2(rx, ry, rz);
@@ -334,9 +335,9 @@ __global__ void __launch_bounds__(256) k_dfd_visc(DfdArgs a) {
         const float4 p = a.x[r], ui = a.vp[r];
         wi = a.vb[r];
         const uint32_t n = a.ncnt[r];
-        const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+        const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
         for (uint32_t t = lane; t + 1 < n; t += L) {
-            const uint32_t j = lst[(size_t)t * 32u];
+            const uint32_t j = lst[ell_slot(t, a.shape)];
             if (j >= a.nf) continue;   // same-material neighbours only
             const float4 q = __ldg(a.x + j), uj = __ldg(a.vp + j), wj = __ldg(a.vb + j);
             const float rx = p.x - q.x, ry = p.y - q.y, rz = p.z - q.z;
@@ -396,9 +397,9 @@ __global__ void __launch_bounds__(256) k_dfd_a1(DfdArgs a) {
     if (live) {
         const float4 p = a.x[r];
         const uint32_t n = a.ncnt[r];
-        const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+        const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
         for (uint32_t t = lane; t + 1 < n; t += L) {
-            const uint32_t j = lst[(size_t)t * 32u];
+            const uint32_t j = lst[ell_slot(t, a.shape)];
             const float4 q = __ldg(a.x + j);
             const float rx = p.x - q.x, ry = p.y - q.y, rz = p.z - q.z;
             const float gg = cubic_g(dist2(rx, ry, rz), a.k) * q.w;
@@ -429,10 +430,10 @@ __global__ void __launch_bounds__(256) k_dfd_ratio_x(DfdArgs a) {
         const float4 p = a.x[r], Ai = a.a1b[r];
         const float rbi = a.rbar[r];
         const uint32_t n = a.ncnt[r];
-        const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+        const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
         const float im = 1.f / a.mass_f;
         for (uint32_t t = lane; t + 1 < n; t += L) {
-            const uint32_t j = lst[(size_t)t * 32u];
+            const uint32_t j = lst[ell_slot(t, a.shape)];
             const float4 q = __ldg(a.x + j);
             const bool fj = j < a.nf;
             const float4 Aj = fj ? __ldg(a.a1b + j) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -550,7 +551,8 @@ int df_record_solve(vtp_solver &s, DfDiffState &d, DfTape &tape, DfTapeSlot &slo
     vtp::SolveCtl c = s.solve_ctl(which, cudaGraphConditionalHandle{}, 0);
     c.force_iters = which == 0 ? s.force_div : s.force_inc;
     c.force_seq = nullptr;
-    c.scene_tiles = s.d_scene_tiles;   // the unstaged passes write one residual partial per tile
+    c.scene_tiles = s.d_scene_tiles;   // the unstaged passes write residual partials per tile
+    c.pieces = s.teams ? vtp::solve_pieces(s.block) : 1u;
     vtp::dfsph_solve_begin(s.st, s.solve + (size_t)which * s.scenes.size(), s.loop + which, 1);
     vtp::dfsph_solve_pack(s.st, a);
     slot.first[which] = pool;
@@ -602,7 +604,7 @@ int df_record_substep(vtp_solver &s, DfDiffState &d, DfTape &tape, DfTapeSlot &s
                    s.orig.n(), carry, 0.f, s.u, s.u.fstart);
     s.pos.swap(); s.vel.swap(); s.orig.swap(); s.vadv.swap();
     vtp::ugns_build_lists(st, s.scn(), s.L, 0, nf, s.pos.c(), s.orig.c(), s.u, slot.nbr, slot.ncnt, s.d_status,
-                          s.d_overflow, s.block);
+                          s.d_overflow);
     if (nf) {
         CU(cudaMemcpyAsync(slot.orig, s.orig.c(), nf * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
         CU(cudaMemcpyAsync(slot.x, s.pos.c(), nf * sizeof(float4), cudaMemcpyDeviceToDevice, st));
@@ -688,7 +690,8 @@ int df_capture_solve(vtp_solver &s, DfTape &tape, DfTapeSlot &slot, int which, u
     vtp::SolveCtl c = s.solve_ctl(which, hnd, 1);
     c.force_iters = which == 0 ? s.force_div : s.force_inc;
     c.force_seq = nullptr;
-    c.scene_tiles = s.d_scene_tiles;   // the unstaged passes write one residual partial per tile
+    c.scene_tiles = s.d_scene_tiles;   // the unstaged passes write residual partials per tile
+    c.pieces = s.teams ? vtp::solve_pieces(s.block) : 1u;
     const uint32_t nf = s.L.nf;
     vtp::dfsph_solve_a(s.side, a, s.block);
     if (nf)
@@ -715,7 +718,7 @@ int df_capture_substep(vtp_solver &s, DfTape &tape, DfTapeSlot &slot, uint32_t *
                    s.orig.n(), carry, 0.f, s.u, s.u.fstart);
     s.pos.swap(); s.vel.swap(); s.orig.swap(); s.vadv.swap();
     vtp::ugns_build_lists(st, s.scn(), s.L, 0, nf, s.pos.c(), s.orig.c(), s.u, slot.nbr, slot.ncnt, s.d_status,
-                          s.d_overflow, s.block);
+                          s.d_overflow);
     if (nf) {
         CU(cudaMemcpyAsync(slot.orig, s.orig.c(), nf * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
         CU(cudaMemcpyAsync(slot.x, s.pos.c(), nf * sizeof(float4), cudaMemcpyDeviceToDevice, st));
@@ -841,7 +844,7 @@ int df_adjoint_segment_l(vtp_solver &s, DfDiffState &d, uint32_t k, int tp) {
     const DfTape &tape = d.tapes[tp];
     const unsigned G = vtp::nblk(nf, 256), GL = vtp::nblk(nf * (uint32_t)L, 256);
     vtp::DfdArgs a{};
-    a.nf = nf; a.ell_stride = s.L.ell_stride; a.k = s.kc;
+    a.nf = nf; a.shape = s.L.shape; a.k = s.kc;
     a.dt = s.dt; a.mass_f = s.rho_f * s.vol0;
     a.vis10 = 10.f * ((s.viscosity + s.viscosity) / 2 * a.mass_f / s.rho_f);
     a.eps = 0.001f * (s.h * s.h);
@@ -935,7 +938,7 @@ int dfsph_diff_forward(vtp_solver *s, uint32_t n_steps, uint32_t checkpoint_ever
     const uint32_t every = std::min(checkpoint_every, n_steps);
     const uint32_t nchk = (n_steps + every - 1) / every;
     const size_t nf = std::max<uint32_t>(s->L.nf, 1), n = std::max<uint32_t>(s->L.n, 1);
-    const size_t lrows = ((size_t)s->L.nf + 31) / 32 * 32 * s->L.ell_stride;
+    const size_t lrows = ((size_t)s->L.nf + 31) / 32 * 32 * s->L.shape.stride;
     // Tapes kept resident: as many segments' as the budget and half the free memory allow
     // (all of them with keep_lists), estimated at 8 iteration records per substep.
     const size_t slot_bytes = 4 * nf * 2 + 4 * std::max<size_t>(lrows, 1) + 16 * n + 16 * nf + 4 * nf + 16 * n * 8;

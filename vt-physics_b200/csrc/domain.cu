@@ -589,7 +589,7 @@ int vtp_domain_prepare(vtp_domain *d) {
     d->slot.swap(); d->objf.swap();
     const vtp::Layout L = d->layout();
     vtp::ugns_build_lists(d->st, s->scn(), L, 0, d->n_act, s->pos.c(), s->orig.c(), s->u, s->u.nbr, s->u.ncnt,
-                          s->d_status, s->d_overflow, s->block);
+                          s->d_status, s->d_overflow);
     if (d->n_act) {
         k_dd_row_of_slot<<<nblk(d->n_act, 256), 256, 0, d->st>>>(d->n_act, d->slot.c(), d->row_of_slot, d->status);
         if (d->halo_on) {
@@ -601,7 +601,7 @@ int vtp_domain_prepare(vtp_domain *d) {
                                                                              (uint32_t)s->block);
     }
     d->which = 0;
-    if (!pbf) vtp::dfsph_ratio_alpha(d->st, d->args(), s->block);
+    if (!pbf) vtp::dfsph_ratio_alpha(d->st, d->args(), d->s->block);
     CU(cudaGetLastError());
     d->prepared = true;
     return VTP_OK;
@@ -682,10 +682,10 @@ int vtp_domain_forces(vtp_domain *d) {
     const vtp::DfsphArgs a = d->args();
     vtp::dfsph_pressure_pack(d->st, a);
     if (s->gamma == 0.f) {
-        vtp::dfsph_viscosity(d->st, a, s->block);
+        vtp::dfsph_viscosity(d->st, a, d->s->block);
         s->vel.swap(); s->vadv.swap();
     } else {
-        vtp::dfsph_vis_normal(d->st, a, s->block);
+        vtp::dfsph_vis_normal(d->st, a, d->s->block);
     }
     CU(cudaGetLastError());
     return VTP_OK;
@@ -696,7 +696,7 @@ int vtp_domain_tension(vtp_domain *d) {
     if ((rc = need_type(d, VTP_SOLVER_DFSPH))) return rc;
     vtp_solver *s = d->s;
     if (s->gamma == 0.f) return fail(VTP_ERR_STATE, "surface tension pass with surfaceTensionCoefficient 0");
-    vtp::dfsph_tension(d->st, d->args(), s->block);
+    vtp::dfsph_tension(d->st, d->args(), d->s->block);
     s->vel.swap(); s->vadv.swap();
     CU(cudaGetLastError());
     return VTP_OK;

@@ -60,7 +60,7 @@ struct ImmParams {
 
 struct ImmArgs {
     uint32_t nf;
-    uint32_t ell_stride;
+    ListShape shape;
     Cubic k;
     ImmParams p;
     float dt, inv_dt, h, gamma, csigma, h6_64;
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(256) k_precompute(ImmArgs a) {
     const float mi = a.rd[r] * p.w;
     float ratio = n > 0 ? p.w * a.k.w0 : 0.f;
     float a1x = 0.f, a1y = 0.f, a1z = 0.f, a2 = 1e-6f, blocking = 0.f;
-    const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+    const uint32_t *lst = a.nbr + row_index(r, a.shape);
     nbr_loop<U>(lst, n > 0 ? n - 1 : 0,
                 [&](uint32_t j) {
                     const bool f = j < a.nf;
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(256) k_vis(ImmArgs a) {
     }
     float nx = 0.f, ny = 0.f, nz = 0.f;
     const uint32_t n = a.ncnt[r];
-    const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+    const uint32_t *lst = a.nbr + row_index(r, a.shape);
     nbr_loop<U>(lst, n > 0 ? n - 1 : 0,
                 [&](uint32_t j) {
                     if (j >= a.nf) return VisG{};
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(256) k_tension(ImmArgs a) {
     const float mi = rdi * p.w;
     float tx = 0.f, ty = 0.f, tz = 0.f;
     const uint32_t n = a.ncnt[r];
-    const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+    const uint32_t *lst = a.nbr + row_index(r, a.shape);
     nbr_loop<U>(lst, n > 0 ? n - 1 : 0,
                 [&](uint32_t j) {
                     if (j >= a.nf) return TG{};
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(256) k_ct(ImmArgs a) {
 #pragma unroll
     for (int c = 0; c < 9; ++c) G[c] = 0.f;
     const uint32_t n = a.ncnt[r];
-    const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+    const uint32_t *lst = a.nbr + row_index(r, a.shape);
     nbr_loop<U>(lst, n > 0 ? n - 1 : 0,
                 [&](uint32_t j) {
                     if (j >= a.nf) return CG{};
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(256) k_pct(ImmArgs a) {
     for (int k = 0; k < kSym; ++k) ti[k] = a.tau[k][r] / inv_i;
     float ax = 0.f, ay = 0.f, az = 0.f;
     const uint32_t n = a.ncnt[r];
-    const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+    const uint32_t *lst = a.nbr + row_index(r, a.shape);
     nbr_loop<(U > 2 ? 2 : U)>(lst, n > 0 ? n - 1 : 0,
                 [&](uint32_t j) {
                     PG e{};
@@ -553,20 +553,20 @@ __global__ void __launch_bounds__(256) k_drift_mark(ImmArgs a) {
         if (fr == 0) {
             const uint32_t n = a.ncnt[r];
             const uint32_t cnt = n > 0 ? n - 1 : 0;
-            const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+            const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
             // four entries, then their four flags, per round trip (gen >= 1, so rows without a
             // flag word (boundary rows) read as 0)
             uint32_t t = 0;
             for (; t + 4 <= cnt && !redo; t += 4) {
                 uint32_t j[4], f[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) j[u] = lst[(size_t)(t + u) * 32u];
+                for (int u = 0; u < 4; ++u) j[u] = lst[ell_slot(t + u, a.shape)];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) f[u] = j[u] < a.nf ? __ldg(a.flag + j[u]) : 0u;
                 redo = f[0] == gen || f[1] == gen || f[2] == gen || f[3] == gen;
             }
             for (; t < cnt && !redo; ++t) {
-                const uint32_t j = lst[(size_t)t * 32u];
+                const uint32_t j = lst[ell_slot(t, a.shape)];
                 redo = j < a.nf && __ldg(a.flag + j) == gen;
             }
         }
@@ -614,7 +614,7 @@ __global__ void __launch_bounds__(256) k_drift_diffuse(ImmArgs a, int retry) {
             ui[k] = make_float4(vk.x - vi.x, vk.y - vi.y, vk.z - vi.z, 0.f);
         }
         const uint32_t n = a.ncnt[r];
-        const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+        const uint32_t *lst = a.nbr + row_index(r, a.shape);
         const float ndt = -a.dt;
         // drift
         nbr_loop<U>(lst, n > 0 ? n - 1 : 0,
@@ -877,7 +877,7 @@ static ImmArgs imm_args(vtp_solver &s) {
     ImmState &m = *s.imm;
     ImmArgs a{};
     a.nf = s.L.nf;
-    a.ell_stride = s.L.ell_stride;
+    a.shape = s.L.shape;
     a.k = s.kc;
     a.p = m.p;
     a.retry_all = s.phase_retry_all ? 1 : 0;
@@ -1052,7 +1052,7 @@ int immct_enqueue_tick(vtp_solver &s, cudaStream_t st, bool capture) {
     };
     P_("ugns_lists", [&] {
         vtp::ugns_build_lists(st, s.scn(), s.L, 0, nf, s.pos.c(), s.orig.c(), s.u, s.u.nbr, s.u.ncnt, s.d_status,
-                              s.d_overflow, B);
+                              s.d_overflow);
     });
     s.launches_per_tick += 6;   // hash, 3 scan kernels, scatter, rank/reorder
     if (nf == 0) return VTP_OK;

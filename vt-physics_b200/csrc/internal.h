@@ -23,16 +23,24 @@ struct NvtxRange {
     NvtxRange &operator=(const NvtxRange &) = delete;
 };
 
+// Solvers of up to this many fluid rows walk a row with a team of four lanes (team.cuh), larger
+// ones with a thread per row; the bits are the same.  Event-timed launches (B200, about 5 us of
+// which is the events), thread per row -> team, us: DFSPH solve_a / solve_b / ratio + alpha /
+// viscosity at 2,000 rows 13.3 / 11.6 / 16.4 / 13.4 -> 9.9 / 8.5 / 9.4 / 10.4, at 32,000 rows
+// 14.5 / 12.6 / 18.7 / 14.8 -> 13.2 / 10.6 / 13.1 / 12.4, at 64,000 rows 16.4 / 14.4 / 18.8 / 16.6
+// -> 18.3 / 15.1 / 20.8 / 19.0.  A team executes 1.6 times the instructions of the thread, so past
+// the row count that fills the GPU the thread wins (1,000,000 rows: solve_a 113 -> 168).
+constexpr uint32_t kTeamMaxRows = 49152;
+
 constexpr int kConsPhases = 8;   // phases the conservation sums report (vtp_conservation.phase_mass)
 
 // Particles are kept sorted: fluid rows [0, nf) re-sorted by (cell, attach id)
 // every substep, boundary rows [nf, n) sorted once at initialize.
 struct Layout {
     uint32_t n = 0, nf = 0, nb = 0;
-    uint32_t ell_stride = 0;   // slots per row in the ELL neighbour list (maxnbr - 1 others)
+    ListShape shape;           // neighbour-list storage (maxnbr - 1 entries per row)
     int merge_mode = 0;        // 0: fluid ids < boundary ids, 1: boundary ids < fluid ids, 2: general
-    int list_lanes = 0;        // list builder lanes per row: 0 = by row count, 1 or 8 = forced
-    bool cell_cull = false;    // list builder skips neighbour cells beyond h of the row (same lists)
+    bool cell_cull = false;    // the walking list builders skip neighbour cells beyond h of the row (same lists)
 };
 
 // Neighbour-search working set (one per solver).
@@ -98,7 +106,7 @@ void ugns_sort(cudaStream_t st, const Scenes &sc, uint32_t nbuckets, uint32_t ro
 // 27 offsets, then ascending attach id inside a cell).
 void ugns_build_lists(cudaStream_t st, const Scenes &sc, const Layout &L, uint32_t row0, uint32_t cnt,
                       const float4 *pos, const uint32_t *orig, const UgnsBuffers &u,
-                      uint32_t *nbr, uint32_t *ncnt, uint32_t *status, uint32_t *overflow, int block);
+                      uint32_t *nbr, uint32_t *ncnt, uint32_t *status, uint32_t *overflow);
 
 // sigma of the cubic spline computed on the device (0 on success).
 int cubic_sigma_device(cudaStream_t st, float h, float *out_host);

@@ -33,7 +33,7 @@ __device__ __forceinline__ float pbf_w0(const PbfArgs &a) { return a.form ? a.c6
 
 __global__ void __launch_bounds__(256) k_pbf_init_boundary(PbfArgs a, const uint32_t *__restrict__ bncnt,
                                                            const uint32_t *__restrict__ bnbr,
-                                                           uint32_t ell_stride) {
+                                                           ListShape shape) {
     // compute_rigid_particle_volume_cuda (PBFCudaImpl.cu:47-68): V_b = 1 / sum_{boundary j} W_ij
     // (self included), m_b = rho_b V_b.  Only boundary neighbours count.
     uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -42,9 +42,9 @@ __global__ void __launch_bounds__(256) k_pbf_init_boundary(PbfArgs a, const uint
     float4 p = a.pos[i];
     uint32_t n = bncnt[r];
     float delta = n > 0 ? pbf_w0(a) : 0.f;
-    const uint32_t *lst = bnbr + ell_index(r, 0, ell_stride);
+    const uint32_t *lst = bnbr + ell_index(r, 0, shape);
     for (uint32_t t = 0; t + 1 < n; ++t) {
-        uint32_t j = lst[(size_t)t * 32u];
+        uint32_t j = lst[ell_slot(t, shape)];
         if (j < a.nf) continue;
         float4 q = a.pos[j];
         delta += pbf_w(dist2(p.x - q.x, p.y - q.y, p.z - q.z), a);
@@ -66,6 +66,14 @@ struct PV2 {
     float vol;
 };
 
+// One thread per row reads lists of shape lg 0; lanes per row ("rowLanes") read either shape.
+template <int U, int L, class Load, class Use>
+__device__ __forceinline__ void row_loop(const PbfArgs &a, const uint32_t *lst, uint32_t cnt, int lane, Load load,
+                                         Use use) {
+    if constexpr (L == 1) nbr_loop<U>(lst, cnt, load, use);
+    else nbr_loop_lanes<U, L>(lst, a.shape, cnt, lane, load, use);
+}
+
 // Neighbour passes, U list entries in flight per thread and L lanes per row
 // (L = 1: one thread walks the row's list in order; L > 1: the row's lanes
 // take entries lane, lane + L, ... and their partial sums are added by a
@@ -83,8 +91,8 @@ __global__ void __launch_bounds__(256) k_pbf_lambda(PbfArgs a) {
     // Self is the first entry of every list: density gets m_i W(0), gradients 0.
     float rho = (n > 0 && lane == 0) ? p.w * pbf_w0(a) : 0.f;
     float gx = 0.f, gy = 0.f, gz = 0.f, s2 = 0.f;
-    const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
-    nbr_loop_lanes<U, L>(lst, n > 0 ? n - 1 : 0, lane, [&](uint32_t j) { return ldg4(a.pos + j); },
+    const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
+    row_loop<U, L>(a, lst, n > 0 ? n - 1 : 0, lane, [&](uint32_t j) { return ldg4(a.pos + j); },
                          [&](uint32_t, const float4 &q) {
                              const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
                              float w, g;
@@ -131,9 +139,9 @@ __global__ void __launch_bounds__(256) k_pbf_dx(PbfArgs a) {
     const float li = a.lambda[r];
     const uint32_t n = a.ncnt[r];
     float dx = 0.f, dy = 0.f, dz = 0.f;
-    const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
+    const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
     // Boundary lambda is never written by the reference; it is taken as 0.
-    nbr_loop_lanes<U, L>(lst, n > 0 ? n - 1 : 0, lane,
+    row_loop<U, L>(a, lst, n > 0 ? n - 1 : 0, lane,
                          [&](uint32_t j) { return PL{ldg4(a.pos + j), j < a.nf ? __ldg(a.lambda + j) : 0.f}; },
                          [&](uint32_t, const PL &e) {
                              const float rx = p.x - e.q.x, ry = p.y - e.q.y, rz = p.z - e.q.z;
@@ -178,8 +186,8 @@ __global__ void __launch_bounds__(256) k_pbf_xsph(PbfArgs a) {
     const float4 vi = a.vel[r];
     const uint32_t n = a.ncnt[r];
     float ax = 0.f, ay = 0.f, az = 0.f;
-    const uint32_t *lst = a.nbr + ell_index(r, 0, a.ell_stride);
-    nbr_loop_lanes<U, L>(lst, n > 0 ? n - 1 : 0, lane,
+    const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
+    row_loop<U, L>(a, lst, n > 0 ? n - 1 : 0, lane,
                          [&](uint32_t j) { return PV2{ldg4(a.pos + j), ldg4(a.vel + j), __ldg(a.vol + j)}; },
                          [&](uint32_t, const PV2 &e) {
                              const float w = pbf_w(dist2(p.x - e.q.x, p.y - e.q.y, p.z - e.q.z), a);
@@ -209,8 +217,8 @@ inline unsigned nblk(uint32_t n, int b) { return (unsigned)((n + b - 1) / b); }
 }  // namespace
 
 void pbf_init_boundary(cudaStream_t st, const PbfArgs &a, const uint32_t *bncnt, const uint32_t *bnbr,
-                       uint32_t ell_stride) {
-    if (a.nb) k_pbf_init_boundary<<<nblk(a.nb, 256), 256, 0, st>>>(a, bncnt, bnbr, ell_stride);
+                       ListShape shape) {
+    if (a.nb) k_pbf_init_boundary<<<nblk(a.nb, 256), 256, 0, st>>>(a, bncnt, bnbr, shape);
 }
 #define VTP_UNROLL_DISPATCH(U, ...)          \
     switch (U) {                                 \

@@ -8,7 +8,7 @@ namespace vtp {
 
 struct PbfArgs {
     uint32_t nf, nb;
-    uint32_t ell_stride;
+    ListShape shape;
     Cubic k;
     float rho0, inv_rho0, rho_b, eps, dt, xsph_k;
     int form;              // 0: the reference's formulation; 1: standard PBF (poly6 / spiky, mass-weighted)
@@ -29,7 +29,7 @@ struct PbfArgs {
 };
 
 void pbf_init_boundary(cudaStream_t st, const PbfArgs &a, const uint32_t *bncnt, const uint32_t *bnbr,
-                       uint32_t ell_stride);
+                       ListShape shape);
 void pbf_lambda(cudaStream_t st, const PbfArgs &a, int block);
 void pbf_dx(cudaStream_t st, const PbfArgs &a, int block);
 void pbf_xsph(cudaStream_t st, const PbfArgs &a, int block);

@@ -119,13 +119,13 @@ __device__ __forceinline__ uint32_t slot_row(const GroupPlan &P, int u, uint32_t
 
 // nbr_loop over a slot list (2-byte entries, ELL layout): U entries' loads in flight.
 template <int U, class Load, class Use>
-__device__ __forceinline__ void slot_loop(const uint16_t *__restrict__ lst, uint32_t cnt, Load load, Use use) {
+__device__ __forceinline__ void slot_loop(const uint16_t *__restrict__ lst, ListShape shape, uint32_t cnt, Load load, Use use) {
     using T = decltype(load((uint16_t)0));
     uint32_t t = 0;
     for (; t + U <= cnt; t += U) {
         uint16_t j[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) j[u] = __ldcs(lst + (size_t)(t + u) * 32u);
+        for (int u = 0; u < U; ++u) j[u] = __ldcs(lst + ell_slot(t + u, shape));
         T d[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) d[u] = load(j[u]);
@@ -133,7 +133,7 @@ __device__ __forceinline__ void slot_loop(const uint16_t *__restrict__ lst, uint
         for (int u = 0; u < U; ++u) use(j[u], d[u]);
     }
     for (; t < cnt; ++t) {
-        const uint16_t j = __ldcs(lst + (size_t)t * 32u);
+        const uint16_t j = __ldcs(lst + ell_slot(t, shape));
         use(j, load(j));
     }
 }

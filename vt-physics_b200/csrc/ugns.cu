@@ -16,17 +16,20 @@
 #include "internal.h"
 #include "staged.h"
 
+#include <climits>
 #include <type_traits>
+
 
 namespace vtp {
 
 namespace {
 
+// More rows than this take the builder with a thread per row.
+constexpr uint32_t kWalkRows = 300000;
+constexpr int kWalkBlock = 128;
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
-// Up to this many rows the list builder runs eight lanes per row.
-constexpr uint32_t kSplitRows = 131072;
 
 __device__ __forceinline__ float4 apply_force(float4 p, float4 &v, float dt, float3 g) {
     // apply_ext_force_cuda (PBFCudaImpl.cu:146-157): v += g dt; x += v dt.
@@ -259,12 +262,14 @@ struct FaceGaps {
 };
 
 // One candidate of the neighbour walk (UGNSCudaImpl.cu:189-199).
+template <class Slots>
 struct Walker {
     float px, py, pz;
     uint32_t self;
     uint32_t cnt;        // entries written incl. self
     uint32_t maxnbr;
-    uint32_t *out;       // ELL base for this row (slot t at out[t*32])
+    uint32_t *out;       // the row's first list entry
+    Slots at;            // offsets of the others
     bool overflow;
 
     // The row itself (d2 == 0) fails `d2 > 0` like every coincident particle,
@@ -273,7 +278,7 @@ struct Walker {
         float d2 = dist2(px - q.x, py - q.y, pz - q.z);
         if (d2 > 0.f && d2 <= d2max) {
             if (cnt < maxnbr) {
-                out[(size_t)(cnt - 1) * 32u] = j;
+                out[at(cnt - 1)] = j;
                 ++cnt;
             } else {
                 overflow = true;
@@ -286,7 +291,7 @@ struct Walker {
     __device__ __forceinline__ void accept_room(uint32_t j, const float4 &q, float d2max) {
         const float d2 = dist2(px - q.x, py - q.y, pz - q.z);
         const bool acc = d2 > 0.f && d2 <= d2max;
-        if (acc) out[(size_t)(cnt - 1) * 32u] = j;
+        if (acc) out[at(cnt - 1)] = j;
         cnt += acc ? 1u : 0u;
     }
 
@@ -341,8 +346,13 @@ struct Walker {
     }
 };
 
+// One thread per row walks its 27 cells and appends to its list: the faster builder from some
+// hundred thousand rows on (kWalkRows; 500,000 rows 138 us against 154 for k_build_lists,
+// 1,000,000 rows 240 against 258), where every SM has rows enough and the cells' shared memory
+// phases of k_build_lists cost more than the lookups they share.  Issue-bound at 80 % of the issue
+// slots (29 warp instructions per warp-level candidate test).
 template <int MODE, bool CULL>
-__global__ void k_build_lists(Scenes sc, uint32_t row0, uint32_t cnt, uint32_t ell_stride,
+__global__ void k_walk_lists(Scenes sc, uint32_t row0, uint32_t cnt, ListShape shape,
                               const float4 *__restrict__ pos, const uint32_t *__restrict__ orig,
                               const uint32_t *__restrict__ fstart, const uint32_t *__restrict__ bstart,
                               uint32_t *__restrict__ nbr, uint32_t *__restrict__ ncnt,
@@ -358,12 +368,12 @@ __global__ void k_build_lists(Scenes sc, uint32_t row0, uint32_t cnt, uint32_t e
         ncnt[r] = 0;
         return;
     }
-    Walker w;
+    Walker<RowSlots> w;
     w.px = p.x; w.py = p.y; w.pz = p.z;
     w.self = i;
     w.cnt = 1;
     w.maxnbr = sc.maxnbr;
-    w.out = nbr + ell_index(r, 0, ell_stride);
+    w.out = nbr + row_index(r, shape);
     w.overflow = false;
     const float d2max = sc.d2max;
     FaceGaps fg;
@@ -389,147 +399,302 @@ __global__ void k_build_lists(Scenes sc, uint32_t row0, uint32_t cnt, uint32_t e
     }
 }
 
-// Lane-split walk for small row counts, where one thread per row leaves most
-// of the GPU idle and the kernel time is one thread's serial walk: L lanes per
-// row, lane l walking the contiguous group [27 l / L, 27 (l+1) / L) of the 27
-// offsets.  Pass 1 counts the lane's accepted candidates, a shuffle scan over
-// the row's lanes gives each lane its first slot, pass 2 walks again and
-// writes.  The concatenation is the one-thread walk's list, truncation at
-// maxNbr included, so both builders write identical lists.
-// Passes of the lane-split walk: kCount tests every candidate, counts the
-// accepted ones and keeps the first kSplitKeep of them in the block's shared
-// buffer; kWrite tests again and writes every accepted candidate into its
-// slot (only for a lane that accepted more than kSplitKeep).
-enum SplitPass { kCount = 0, kWrite = 1 };
-constexpr int kSplitBlock = 256;   // threads per block of the lane-split builder
-constexpr uint32_t kSplitKeep = 16; // accepted candidates a lane keeps for the copy-out
+// Two FP32 lanes of one 64-bit register pair (sm_100 packed arithmetic; each lane rounds as the
+// scalar instruction does).
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 f2_unpack(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
 
-template <int PASS>
-struct SplitSink {
-    float px, py, pz;
-    uint32_t n;       // candidates accepted by this lane so far
-    uint32_t base;    // kWrite: this lane's first slot
-    uint32_t cap;     // list slots per row (maxNbr - 1)
-    uint32_t *out;    // kCount: this thread's column of the shared buffer (stride kSplitBlock); kWrite: ELL row
+// The general interleaving of a cell's fluid and boundary runs: merged by attach id.
+__device__ __forceinline__ uint32_t merge_next(uint32_t &f, uint32_t f1, uint32_t &b, uint32_t b1,
+                                               const uint32_t *__restrict__ orig) {
+    if (b >= b1) return f++;
+    if (f >= f1) return b++;
+    return __ldg(orig + f) < __ldg(orig + b) ? f++ : b++;
+}
 
-    __device__ __forceinline__ void take(uint32_t j, const float4 &q, float d2max) {
-        const float d2 = dist2(px - q.x, py - q.y, pz - q.z);
-        if (d2 > 0.f && d2 <= d2max) {
-            if (PASS == kCount) {
-                if (n < kSplitKeep) out[n * kSplitBlock] = j;
-            } else {
-                const uint32_t slot = base + n;
-                if (slot < cap) out[(size_t)slot * 32u] = j;
-            }
-            ++n;
-        }
-    }
+// List builder: one warp per occupied cell.  The rows of a cell share their 27 neighbour cells,
+// so the warp lays the candidates of those cells out once in shared memory, in list order (27
+// offsets in the reference's order, each cell's two runs in MODE's order), and every row of the
+// cell walks that layout: R rows at a time, 32 / R lanes per row, each lane a contiguous share of
+// the candidates.  A lane tests two candidates per packed FP32 instruction (the roundings of
+// dist2) and keeps the accepted ones as bits; the lanes' bit counts, scanned over the row, give
+// each lane its first slot, and the lists are composed in shared memory and written segment by
+// segment.  Against a walk per row, the cell lookups, the candidate loads and the loop control
+// are paid once per cell instead of once per row.
+// It is bound by issue.  Event-timed launches (B200, us), the former builders (eight lanes per row
+// up to 131,072 rows, above that one thread per row) -> this: 16,000 rows 19 -> 12.5, 31,000 rows
+// 39 -> 23 (DFSPH blocks), 64,000 rows 68 -> 24, 128,000 rows 119 -> 41, 250,000 rows 93 -> 72.
+constexpr uint32_t kCellScan = 8;        // rows a warp scans for cells that start there: about one cell
+constexpr int kCellWarps = 4;            // warps per block
+constexpr uint32_t kCellWindow = 320;    // candidates laid out at a time (4 lanes x 80, 8 lanes x 40)
+constexpr uint32_t kCellKept = 84;       // bytes of a lane's accepted candidates (80 used; 21 words apart: few conflicts)
 
-    __device__ __forceinline__ void visit(uint32_t j, const float4 *__restrict__ pos, float d2max) {
-        take(j, __ldg(pos + j), d2max);
-    }
-
-    __device__ __forceinline__ void run(uint32_t j0, uint32_t j1, const float4 *__restrict__ pos, float d2max) {
-        uint32_t j = j0;
-        for (; j + 4 <= j1; j += 4) {
-            const float4 q0 = __ldg(pos + j), q1 = __ldg(pos + j + 1), q2 = __ldg(pos + j + 2),
-                         q3 = __ldg(pos + j + 3);
-            take(j, q0, d2max);
-            take(j + 1, q1, d2max);
-            take(j + 2, q2, d2max);
-            take(j + 3, q3, d2max);
-        }
-        for (; j < j1; ++j) take(j, __ldg(pos + j), d2max);
-    }
+struct CellScratch {
+    float x[3][kCellWindow];             // candidate positions of the window, in list order
+    uint32_t cand[kCellWindow];          // their rows
+    uint8_t kept[32][kCellKept];         // each lane's accepted candidates, as offsets into its share
 };
 
-template <int MODE, bool CULL, int PASS>
-__device__ __forceinline__ void split_walk(SplitSink<PASS> &k, int3 c, const SceneGrid &g, int t0, int t1,
-                                           const float4 *__restrict__ pos, const uint32_t *__restrict__ orig,
-                                           const uint32_t *__restrict__ fstart, const uint32_t *__restrict__ bstart,
-                                           float d2max, const FaceGaps &fg) {
-    for (int t = t0; t < t1; ++t) {
-        int3 cc = c;
-        const int3 o = nbr_offset(t);
-        cc.x += o.x; cc.y += o.y; cc.z += o.z;
-        if (!cell_available(cc, g)) continue;
-        if (CULL && !fg.reachable(o, d2max)) continue;
-        const uint32_t key = g.key_base + cell_key(cc, g);
-        uint32_t f0 = __ldg(fstart + key), f1 = __ldg(fstart + key + 1);
-        uint32_t b0 = __ldg(bstart + key), b1 = __ldg(bstart + key + 1);
-        if (MODE == 0) {
-            k.run(f0, f1, pos, d2max);
-            k.run(b0, b1, pos, d2max);
-        } else if (MODE == 1) {
-            k.run(b0, b1, pos, d2max);
-            k.run(f0, f1, pos, d2max);
-        } else {
-            while (f0 < f1 || b0 < b1) {
-                uint32_t j;
-                if (b0 >= b1) j = f0++;
-                else if (f0 >= f1) j = b0++;
-                else j = (__ldg(orig + f0) < __ldg(orig + b0)) ? f0++ : b0++;
-                k.visit(j, pos, d2max);
+// The runs of one neighbour cell, held by lane t < 27 for the t-th offset, and where its
+// candidates start in list order.
+struct CellRuns {
+    uint32_t f0, f1, b0, b1, excl;
+};
+
+// Lays candidates [wb, wb + wl) out: rows and positions, infinity from wl up to `padded`.
+template <int MODE>
+__device__ __forceinline__ void stage_candidates(CellScratch &S, const CellRuns &R, uint32_t wb, uint32_t wl,
+                                                 uint32_t padded, const float4 *__restrict__ pos,
+                                                 const uint32_t *__restrict__ orig) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t nf = R.f1 - R.f0, nb = R.b1 - R.b0, len = nf + nb;
+    __syncwarp();
+    if (MODE == 2) {
+        uint32_t fi = R.f0, bi = R.b0;
+        for (uint32_t o = 0; o < len; ++o) {
+            const uint32_t j = merge_next(fi, R.f1, bi, R.b1, orig);
+            if (R.excl + o - wb < wl) S.cand[R.excl + o - wb] = j;
+        }
+    } else {
+        // the part of this lane's runs that lies in the window
+        const uint32_t na = MODE == 0 ? nf : nb, a0 = MODE == 0 ? R.f0 : R.b0, c0 = (MODE == 0 ? R.b0 : R.f0) - na;
+        const uint32_t o0 = wb > R.excl ? min(wb - R.excl, len) : 0u;
+        const uint32_t o1 = wb + wl > R.excl ? min(wb + wl - R.excl, len) : 0u;
+        for (uint32_t o = o0; o < o1; ++o) S.cand[R.excl + o - wb] = (o < na ? a0 : c0) + o;
+    }
+    __syncwarp();
+    for (uint32_t q = lane; q < padded; q += 32u) {
+        const float far = __int_as_float(0x7f800000);
+        float4 v = make_float4(far, far, far, 0.f);
+        if (q < wl) v = __ldg(pos + S.cand[q]);
+        S.x[0][q] = v.x;
+        S.x[1][q] = v.y;
+        S.x[2][q] = v.z;
+    }
+    __syncwarp();
+}
+
+// Appends `off` to the lane's accepted candidates at shared address `to` if 0 < d2 <= d2max
+// (`0 < |x_i - x_j|` also drops the row itself): predicated, no branch.  The asm names no memory
+// clobber, so that the next candidates' loads are not held up by it: what it stores is read only
+// after a warp barrier.
+__device__ __forceinline__ void keep_candidate(uint32_t &to, uint32_t off, float d2, float d2max) {
+    asm(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.gt.f32 p, %2, 0f00000000;\n\t"
+        "setp.le.and.f32 p, %2, %3, p;\n\t"
+        "@p st.shared.u8 [%0], %1;\n\t"
+        "@p add.u32 %0, %0, 1;\n\t}"
+        : "+r"(to)
+        : "r"(off), "f"(d2), "f"(d2max));
+}
+
+// Tests the 4 candidates at index `at` (offset `off` of the lane's share) against -p = (px, py, pz).
+__device__ __forceinline__ void test4(const CellScratch &S, uint32_t at, uint32_t off, uint32_t &to, uint64_t px,
+                                      uint64_t py, uint64_t pz, float d2max) {
+    const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(&S.x[0][at]);
+    const ulonglong2 y = *reinterpret_cast<const ulonglong2 *>(&S.x[1][at]);
+    const ulonglong2 z = *reinterpret_cast<const ulonglong2 *>(&S.x[2][at]);
+    const uint64_t ax = f2_add(px, x.x), ay = f2_add(py, y.x), az = f2_add(pz, z.x);
+    const uint64_t bx = f2_add(px, x.y), by = f2_add(py, y.y), bz = f2_add(pz, z.y);
+    const float2 a = f2_unpack(f2_fma(az, az, f2_fma(ay, ay, f2_mul(ax, ax))));
+    const float2 b = f2_unpack(f2_fma(bz, bz, f2_fma(by, by, f2_mul(bx, bx))));
+    keep_candidate(to, off, a.x, d2max);
+    keep_candidate(to, off + 1u, a.y, d2max);
+    keep_candidate(to, off + 2u, b.x, d2max);
+    keep_candidate(to, off + 3u, b.y, d2max);
+}
+
+// Lists of up to R rows of one cell.  Lane l works for row l % R: `row` (absolute, the same for
+// the row's lanes), `live` for rows that exist.
+template <int MODE, uint32_t R>
+__device__ __forceinline__ void cell_lists(CellScratch &S, const CellRuns &runs, uint32_t total, bool live,
+                                           uint32_t row, uint32_t row0, float4 p, float d2max, uint32_t cap,
+                                           ListShape shape, const float4 *__restrict__ pos,
+                                           const uint32_t *__restrict__ orig, uint32_t *__restrict__ nbr,
+                                           uint32_t *__restrict__ ncnt, uint32_t *__restrict__ status,
+                                           uint32_t *__restrict__ overflow_count) {
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr uint32_t H = 32u / R;   // lanes per row
+    const uint32_t lane = threadIdx.x & 31u, k = lane % R, h = lane / R;
+    const uint64_t px = f2_pack(-p.x, -p.x), py = f2_pack(-p.y, -p.y), pz = f2_pack(-p.z, -p.z);
+    const uint32_t to0 = (uint32_t)__cvta_generic_to_shared(&S.kept[lane][0]);
+    uint32_t found = 0;   // entries of the row in earlier windows
+    for (uint32_t wb = 0; wb < total; wb += kCellWindow) {
+        const uint32_t wl = min(kCellWindow, total - wb);
+        const uint32_t share = ((wl + H - 1u) / H + 7u) & ~7u;   // candidates per lane, in eights
+        stage_candidates<MODE>(S, runs, wb, wl, H * share, pos, orig);
+        uint32_t to = to0;
+        for (uint32_t off = 0; off < share; off += 8u) {
+            test4(S, h * share + off, off, to, px, py, pz, d2max);
+            test4(S, h * share + off + 4u, off + 4u, to, px, py, pz, d2max);
+        }
+        const uint32_t mine = live ? to - to0 : 0u;
+        uint32_t x = mine;
+#pragma unroll
+        for (uint32_t o = R; o < 32u; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kAll, x, o);
+            if (lane >= o) x += y;
+        }
+        __syncwarp();
+        // The lists leave as they are stored: 8 entries of 4 rows, or H entries of R rows, at a
+        // time.  Entry e of a row is in the share of the last lane whose entries start at or
+        // before e.
+        auto flush = [&](uint32_t kk, uint32_t e0, uint32_t step) {
+            uint32_t lo[H];
+#pragma unroll
+            for (uint32_t t = 0; t < H; ++t) lo[t] = __shfl_sync(kAll, x - mine, (int)(kk + R * t));
+            const uint32_t n = __shfl_sync(kAll, x, (int)(kk + 32u - R));
+            const uint32_t before = __shfl_sync(kAll, found, (int)kk);
+            const uint32_t i = __shfl_sync(kAll, row, (int)kk) - row0;
+            uint32_t *dst = nbr + ell_index(i, 0, shape);
+            for (uint32_t e = e0; e < n; e += step) {
+                uint32_t at = kk * kCellKept + e, share_of = 0;
+#pragma unroll
+                for (uint32_t t = 1; t < H; ++t)
+                    if (e >= lo[t]) at = (kk + R * t) * kCellKept + (e - lo[t]), share_of = t * share;
+                const uint32_t slot = before + e;
+                if (slot < cap) dst[ell_slot(slot, shape)] = S.cand[share_of + (&S.kept[0][0])[at]];
             }
+        };
+        if (shape.lg) {
+#pragma unroll
+            for (uint32_t r = 0; r < R; r += 4) flush(r + (lane >> 3), lane & 7u, 8u);
+        } else {
+            flush(k, h, H);
+        }
+        found += __shfl_sync(kAll, x, (int)(k + 32u - R));
+    }
+    if (live && h == 0) {
+        ncnt[row - row0] = min(found, cap) + 1u;
+        if (found > cap) {
+            atomicAdd(overflow_count, 1u);
+            atomicOr(status, ST_BOUNDS);
         }
     }
 }
 
-template <int MODE, bool CULL, int L>
-__global__ void __launch_bounds__(kSplitBlock) k_build_lists_split(
-    Scenes sc, uint32_t row0, uint32_t cnt, uint32_t ell_stride, const float4 *__restrict__ pos,
-    const uint32_t *__restrict__ orig, const uint32_t *__restrict__ fstart, const uint32_t *__restrict__ bstart,
-    uint32_t *__restrict__ nbr, uint32_t *__restrict__ ncnt, uint32_t *__restrict__ status,
-    uint32_t *__restrict__ overflow_count) {
+// Each warp builds the cells that start among its kCellScan rows.
+template <int MODE>
+__global__ void __launch_bounds__(kCellWarps * 32, 7) k_build_lists(
+    Scenes sc, uint32_t row0, uint32_t cnt, ListShape shape, const float4 *__restrict__ pos,
+    const uint32_t *__restrict__ orig, const uint32_t *__restrict__ start, const uint32_t *__restrict__ fstart,
+    const uint32_t *__restrict__ bstart, uint32_t *__restrict__ nbr, uint32_t *__restrict__ ncnt,
+    uint32_t *__restrict__ status, uint32_t *__restrict__ overflow_count) {
     pdl_enter();
-    static_assert(L >= 2 && L <= 16 && (L & (L - 1)) == 0, "L divides the warp");
-    // Accepted candidates of each thread, [kSplitKeep][kSplitBlock] (a thread's column is strided, so
-    // a warp's stores and loads of entry k fall in 32 consecutive words).
-    __shared__ uint32_t keep[kSplitKeep * kSplitBlock];
-    const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t r = gt / L;
-    const int lane = (int)(gt % L);
-    // The L lanes of a row are one aligned group of a warp and leave together.
-    if (r >= cnt) return;
-    const unsigned gmask = ((1u << L) - 1u) << ((threadIdx.x & 31u) & ~(unsigned)(L - 1));
-    const uint32_t i = row0 + r;
-    const SceneGrid g = load_scene(sc, i);
-    const float4 p = pos[i];
-    const int3 c = cell_of(p.x, p.y, p.z, g, sc.cell);
-    if (!cell_available(c, g)) {  // outside the grid: no neighbours, not even self
-        if (lane == 0) ncnt[r] = 0;
-        return;
-    }
-    const int t0 = 27 * lane / L, t1 = 27 * (lane + 1) / L;
+    __shared__ __align__(16) CellScratch scratch[kCellWarps];
+    constexpr unsigned kAll = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t first = (blockIdx.x * kCellWarps + (threadIdx.x >> 5)) * kCellScan;
+    if (first >= cnt) return;
+    CellScratch &S = scratch[threadIdx.x >> 5];
     const float d2max = sc.d2max;
-    FaceGaps fg;
-    if (CULL) fg.init(p, c, g, sc.cell);
-    SplitSink<kCount> cnt1{p.x, p.y, p.z, 0u, 0u, 0u, keep + threadIdx.x};
-    split_walk<MODE, CULL>(cnt1, c, g, t0, t1, pos, orig, fstart, bstart, d2max, fg);
-    uint32_t x = cnt1.n;
-#pragma unroll
-    for (int o = 1; o < L; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(gmask, x, o, L);
-        if (lane >= o) x += y;
-    }
-    const uint32_t total = __shfl_sync(gmask, x, L - 1, L);
     const uint32_t cap = sc.maxnbr - 1u;
-    uint32_t *const out = nbr + ell_index(r, 0, ell_stride);
-    const uint32_t base = x - cnt1.n;
-    if (base < cap && cnt1.n > 0) {
-        if (cnt1.n <= kSplitKeep) {   // the lane's accepted candidates are in shared memory
-            const uint32_t m = min(cnt1.n, cap - base);
-            for (uint32_t k = 0; k < m; ++k) out[(size_t)(base + k) * 32u] = keep[k * kSplitBlock + threadIdx.x];
+    const int3 o = nbr_offset((int)min(lane, 26u));
+
+    // Rows of this warp's window that start a cell; the warp builds the lists of those whole cells.
+    uint32_t cell_end = 0;
+    int3 own = make_int3(0, 0, 0);
+    bool leads = false;
+    if (lane < kCellScan && first + lane < cnt) {
+        const uint32_t i = row0 + first + lane;
+        const SceneGrid g = load_scene(sc, i);
+        const float4 p = pos[i];
+        own = cell_of(p.x, p.y, p.z, g, sc.cell);
+        if (cell_available(own, g)) {
+            const uint32_t k = g.key_base + cell_key(own, g);
+            leads = __ldg(start + k) == i;
+            cell_end = __ldg(start + k + 1);
         } else {
-            SplitSink<kWrite> wr{p.x, p.y, p.z, 0u, base, cap, out};
-            split_walk<MODE, CULL>(wr, c, g, t0, t1, pos, orig, fstart, bstart, d2max, fg);
+            ncnt[first + lane] = 0;   // outside the grid: no neighbours, not even self
         }
     }
-    if (lane == 0) {
-        ncnt[r] = total < cap ? total + 1u : sc.maxnbr;
-        if (total > cap) {
-            atomicAdd(overflow_count, 1u);
-            atomicOr(status, ST_BOUNDS);
+    for (unsigned todo = __ballot_sync(kAll, leads); todo; todo &= todo - 1u) {
+        const int leader = __ffs((int)todo) - 1;
+        const uint32_t beg = row0 + first + (uint32_t)leader;
+        const uint32_t end = __shfl_sync(kAll, cell_end, leader);
+        int3 c0 = make_int3(__shfl_sync(kAll, own.x, leader), __shfl_sync(kAll, own.y, leader),
+                            __shfl_sync(kAll, own.z, leader));
+        const SceneGrid g = load_scene(sc, beg);
+        int3 at = make_int3(INT_MIN, 0, 0);   // the cell whose runs are held
+        CellRuns runs{};
+        uint32_t total = 0;
+        for (uint32_t rg = beg; rg < end; rg += 8u) {
+            const uint32_t n = min(8u, end - rg);
+            const uint32_t row = rg + min(lane & 7u, n - 1u);
+            const float4 p = pos[row];
+            // A bucket of the bricked order is one cell.  In the linear order a cell on the grid's
+            // inclusive upper face shares its bucket with another cell: one round per cell then.
+            for (unsigned left = (1u << n) - 1u; left;) {
+                bool mine = (lane & 7u) < n;
+                if (g.brick) {
+                    left = 0;
+                } else {
+                    const int3 c = cell_of(p.x, p.y, p.z, g, sc.cell);
+                    const int f = __ffs((int)left) - 1;
+                    c0 = make_int3(__shfl_sync(kAll, c.x, f), __shfl_sync(kAll, c.y, f), __shfl_sync(kAll, c.z, f));
+                    mine = ((left >> (lane & 7u)) & 1u) && c.x == c0.x && c.y == c0.y && c.z == c0.z;
+                    left &= ~__ballot_sync(kAll, mine);
+                }
+                if (c0.x != at.x || c0.y != at.y || c0.z != at.z) {
+                    at = c0;
+                    runs = CellRuns{};
+                    if (lane < 27u) {
+                        const int3 cc = make_int3(c0.x + o.x, c0.y + o.y, c0.z + o.z);
+                        if (cell_available(cc, g)) {
+                            const uint32_t k = g.key_base + cell_key(cc, g);
+                            runs.f0 = __ldg(fstart + k); runs.f1 = __ldg(fstart + k + 1);
+                            runs.b0 = __ldg(bstart + k); runs.b1 = __ldg(bstart + k + 1);
+                        }
+                    }
+                    const uint32_t len = (runs.f1 - runs.f0) + (runs.b1 - runs.b0);
+                    uint32_t incl = len;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t y = __shfl_up_sync(kAll, incl, o);
+                        if ((int)lane >= o) incl += y;
+                    }
+                    runs.excl = incl - len;
+                    total = __shfl_sync(kAll, incl, 31);
+                }
+                // Up to four rows of a last, short group take 8 lanes each, else 4 lanes each.
+                if (n <= 4u) {
+                    const uint32_t row4 = __shfl_sync(kAll, row, (int)(lane & 3u));
+                    const float4 p4 = make_float4(__shfl_sync(kAll, p.x, (int)(lane & 3u)),
+                                                  __shfl_sync(kAll, p.y, (int)(lane & 3u)),
+                                                  __shfl_sync(kAll, p.z, (int)(lane & 3u)), 0.f);
+                    const bool live = __shfl_sync(kAll, (int)mine, (int)(lane & 3u)) != 0;
+                    cell_lists<MODE, 4>(S, runs, total, live, row4, row0, p4, d2max, cap, shape, pos, orig,
+                                        nbr, ncnt, status, overflow_count);
+                } else {
+                    cell_lists<MODE, 8>(S, runs, total, mine, row, row0, p, d2max, cap, shape, pos, orig,
+                                        nbr, ncnt, status, overflow_count);
+                }
+                __syncwarp();
+            }
         }
     }
 }
@@ -539,7 +704,7 @@ __global__ void __launch_bounds__(kSplitBlock) k_build_lists_split(
 // after each build - count <= maxNbr, entries inside the solver's rows, no
 // row listed as its own neighbour - with the first offence recorded in
 // `status` (ST_BOUNDS); the passes consume only validated lists.
-__global__ void k_check_lists(uint32_t row0, uint32_t cnt, uint32_t nrows, uint32_t ell_stride, uint32_t maxnbr,
+__global__ void k_check_lists(uint32_t row0, uint32_t cnt, uint32_t nrows, ListShape shape, uint32_t maxnbr,
                               const uint32_t *__restrict__ nbr, const uint32_t *__restrict__ ncnt,
                               uint32_t *__restrict__ status) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -547,7 +712,7 @@ __global__ void k_check_lists(uint32_t row0, uint32_t cnt, uint32_t nrows, uint3
     const uint32_t n = ncnt[r];
     bool bad = n > maxnbr;
     for (uint32_t t = 0; !bad && t + 1 < n; ++t) {
-        const uint32_t j = nbr[ell_index(r, t, ell_stride)];
+        const uint32_t j = nbr[ell_index(r, t, shape)];
         bad = j >= nrows || j == row0 + r;
     }
     if (bad) atomicOr(status, ST_BOUNDS);
@@ -565,7 +730,7 @@ __global__ void k_check_lists(uint32_t row0, uint32_t cnt, uint32_t nrows, uint3
 // block `ngroups` gives the rows outside the grid empty lists.
 template <int MODE, bool CULL>
 __global__ void __launch_bounds__(kStageBlock) k_build_lists_staged(
-    Scenes sc, Staging stg, uint32_t ell_stride, const float4 *__restrict__ pos, uint32_t *__restrict__ nbr,
+    Scenes sc, Staging stg, ListShape shape, const float4 *__restrict__ pos, uint32_t *__restrict__ nbr,
     uint32_t *__restrict__ ncnt, uint32_t *__restrict__ status, uint32_t *__restrict__ overflow_count) {
     pdl_enter();
     extern __shared__ float4 stage[];
@@ -600,12 +765,13 @@ __global__ void __launch_bounds__(kStageBlock) k_build_lists_staged(
         FaceGaps fg;
         if (CULL) fg.init(p, c, g, sc.cell);
         if (!staged) {
-            Walker w;
+            Walker<AnySlots> w;
             w.px = p.x; w.py = p.y; w.pz = p.z;
             w.self = r;
             w.cnt = 1;
             w.maxnbr = maxnbr;
-            w.out = nbr + ell_index(r, 0, ell_stride);
+            w.out = nbr + ell_index(r, 0, shape);
+            w.at = AnySlots{shape};
             w.overflow = false;
             for (int t = 0; t < 27; ++t) {
                 const int3 o = nbr_offset(t);
@@ -627,8 +793,8 @@ __global__ void __launch_bounds__(kStageBlock) k_build_lists_staged(
             }
             continue;
         }
-        uint32_t *const out = nbr + ell_index(r, 0, ell_stride);
-        uint16_t *const sout = stg.snbr + ell_index(r, 0, ell_stride);
+        uint32_t *const out = nbr + ell_index(r, 0, shape);
+        uint16_t *const sout = stg.snbr + ell_index(r, 0, shape);
         uint32_t cnt = 1;
         bool over = false;
         for (int t = 0; t < 27; ++t) {
@@ -653,8 +819,8 @@ __global__ void __launch_bounds__(kStageBlock) k_build_lists_staged(
                 if (d2 > 0.f && d2 <= d2max) {
                     if (room || cnt < maxnbr) {
                         const bool bnd = MODE == 0 ? sl >= sb : sl < sb;
-                        out[(size_t)(cnt - 1) * 32u] = __float_as_uint(q.w);
-                        sout[(size_t)(cnt - 1) * 32u] = (uint16_t)(sl | (bnd ? kSlotBoundary : 0u));
+                        out[ell_slot(cnt - 1, shape)] = __float_as_uint(q.w);
+                        sout[ell_slot(cnt - 1, shape)] = (uint16_t)(sl | (bnd ? kSlotBoundary : 0u));
                         ++cnt;
                     } else {
                         over = true;
@@ -833,7 +999,7 @@ __global__ void k_iota(uint32_t n, uint32_t *dst, uint32_t base) {
     if (i < n) dst[i] = base + i;
 }
 
-__global__ void k_export_neighbors(uint32_t row0, uint32_t cnt, uint32_t ell_stride,
+__global__ void k_export_neighbors(uint32_t row0, uint32_t cnt, ListShape shape,
                                    const uint32_t *__restrict__ nbr, const uint32_t *__restrict__ ncnt,
                                    const uint32_t *__restrict__ orig, uint32_t maxnbr,
                                    uint32_t *__restrict__ out_cnt, uint32_t *__restrict__ out_nbr) {
@@ -847,7 +1013,7 @@ __global__ void k_export_neighbors(uint32_t row0, uint32_t cnt, uint32_t ell_str
     for (uint32_t t = 0; t < maxnbr; ++t) dst[t] = 0xffffffffu;
     if (c == 0) return;
     dst[0] = o;
-    for (uint32_t t = 1; t < c; ++t) dst[t] = orig[nbr[ell_index(r, t - 1, ell_stride)]];
+    for (uint32_t t = 1; t < c; ++t) dst[t] = orig[nbr[ell_index(r, t - 1, shape)]];
 }
 
 __global__ void k_export_sorted(Scenes sc, uint32_t n, const float4 *__restrict__ pos,
@@ -946,43 +1112,43 @@ void ugns_sort(cudaStream_t st, const Scenes &sc, uint32_t nbuckets, uint32_t ro
     E("ugns_rank_reorder");
 }
 
-template <int MODE, bool CULL>
-static void build_lists_as(cudaStream_t st, bool split, const Scenes &sc, const Layout &L, uint32_t row0,
-                           uint32_t cnt, const float4 *pos, const uint32_t *orig, const UgnsBuffers &u, uint32_t *nbr,
-                           uint32_t *ncnt, uint32_t *status, uint32_t *overflow, int block) {
-    if (split) {
-        constexpr int S = 8;
-        launch(k_build_lists_split<MODE, CULL, S>, nblk(cnt * S, kSplitBlock), kSplitBlock, 0, st, sc, row0, cnt,
-               L.ell_stride, pos, orig, u.fstart, u.bstart, nbr, ncnt, status, overflow);
-    } else {
-        launch(k_build_lists<MODE, CULL>, nblk(cnt, block), block, 0, st, sc, row0, cnt, L.ell_stride, pos, orig,
-               u.fstart, u.bstart, nbr, ncnt, status, overflow);
-    }
-}
-
 void ugns_build_lists(cudaStream_t st, const Scenes &sc, const Layout &L, uint32_t row0, uint32_t cnt,
                       const float4 *pos, const uint32_t *orig, const UgnsBuffers &u, uint32_t *nbr, uint32_t *ncnt,
-                      uint32_t *status, uint32_t *overflow, int block) {
+                      uint32_t *status, uint32_t *overflow) {
     if (cnt == 0) return;
-    // Few rows: eight lanes per row (same lists, a quarter to an eighth of the
-    // serial walk per thread).
-    const bool split = L.list_lanes == 8 || (L.list_lanes == 0 && cnt <= kSplitRows);
-    auto go = [&](auto mode, auto cull) {
-        build_lists_as<decltype(mode)::value, decltype(cull)::value>(st, split, sc, L, row0, cnt, pos, orig, u, nbr,
-                                                                     ncnt, status, overflow, block);
-    };
-    using T = std::true_type;
-    using F = std::false_type;
+    const uint32_t *start = row0 == L.nf ? u.bstart : u.fstart;   // the table of the rows themselves
     using M0 = std::integral_constant<int, 0>;
     using M1 = std::integral_constant<int, 1>;
     using M2 = std::integral_constant<int, 2>;
-    switch (L.merge_mode) {
-        case 0: L.cell_cull ? go(M0{}, T{}) : go(M0{}, F{}); break;
-        case 1: L.cell_cull ? go(M1{}, T{}) : go(M1{}, F{}); break;
-        default: L.cell_cull ? go(M2{}, T{}) : go(M2{}, F{}); break;
+    // Lists of either builder are the same; a thread per row writes shape lg 0 well (its stores of
+    // one entry index share a line), so it takes the large solvers, whose lists have that shape.
+    if (cnt > kWalkRows && L.shape.lg == 0) {
+        auto walk = [&](auto mode, auto cull) {
+            constexpr int M = decltype(mode)::value;
+            constexpr bool C = decltype(cull)::value;
+            launch(k_walk_lists<M, C>, nblk(cnt, kWalkBlock), kWalkBlock, 0, st, sc, row0, cnt, L.shape, pos, orig,
+                   u.fstart, u.bstart, nbr, ncnt, status, overflow);
+        };
+        const std::true_type T;
+        const std::false_type F;
+        switch (L.merge_mode) {
+            case 0: L.cell_cull ? walk(M0{}, T) : walk(M0{}, F); break;
+            case 1: L.cell_cull ? walk(M1{}, T) : walk(M1{}, F); break;
+            default: L.cell_cull ? walk(M2{}, T) : walk(M2{}, F); break;
+        }
+    } else {
+        auto cells = [&](auto mode) {
+            launch(k_build_lists<decltype(mode)::value>, nblk(cnt, kCellWarps * kCellScan), kCellWarps * 32, 0, st, sc,
+                   row0, cnt, L.shape, pos, orig, start, u.fstart, u.bstart, nbr, ncnt, status, overflow);
+        };
+        switch (L.merge_mode) {
+            case 0: cells(M0{}); break;
+            case 1: cells(M1{}); break;
+            default: cells(M2{}); break;
+        }
     }
 #ifdef VTP_CHECKED
-    k_check_lists<<<nblk(cnt, 256), 256, 0, st>>>(row0, cnt, L.n, L.ell_stride, sc.maxnbr, nbr, ncnt, status);
+    k_check_lists<<<nblk(cnt, 256), 256, 0, st>>>(row0, cnt, L.n, L.shape, sc.maxnbr, nbr, ncnt, status);
 #endif
 }
 
@@ -995,23 +1161,23 @@ void ugns_build_lists_staged(cudaStream_t st, const Scenes &sc, const Layout &L,
     auto room = [&](auto kern) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); };
     if (stg.mode == 0 && L.cell_cull) {
         room(k_build_lists_staged<0, true>);
-        launch(k_build_lists_staged<0, true>, grid, kStageBlock, smem, st, sc, stg, L.ell_stride, pos, nbr, ncnt,
+        launch(k_build_lists_staged<0, true>, grid, kStageBlock, smem, st, sc, stg, L.shape, pos, nbr, ncnt,
                status, overflow);
     } else if (stg.mode == 0) {
         room(k_build_lists_staged<0, false>);
-        launch(k_build_lists_staged<0, false>, grid, kStageBlock, smem, st, sc, stg, L.ell_stride, pos, nbr, ncnt,
+        launch(k_build_lists_staged<0, false>, grid, kStageBlock, smem, st, sc, stg, L.shape, pos, nbr, ncnt,
                status, overflow);
     } else if (L.cell_cull) {
         room(k_build_lists_staged<1, true>);
-        launch(k_build_lists_staged<1, true>, grid, kStageBlock, smem, st, sc, stg, L.ell_stride, pos, nbr, ncnt,
+        launch(k_build_lists_staged<1, true>, grid, kStageBlock, smem, st, sc, stg, L.shape, pos, nbr, ncnt,
                status, overflow);
     } else {
         room(k_build_lists_staged<1, false>);
-        launch(k_build_lists_staged<1, false>, grid, kStageBlock, smem, st, sc, stg, L.ell_stride, pos, nbr, ncnt,
+        launch(k_build_lists_staged<1, false>, grid, kStageBlock, smem, st, sc, stg, L.shape, pos, nbr, ncnt,
                status, overflow);
     }
 #ifdef VTP_CHECKED
-    k_check_lists<<<nblk(L.nf, 256), 256, 0, st>>>(0, L.nf, L.n, L.ell_stride, sc.maxnbr, nbr, ncnt, status);
+    k_check_lists<<<nblk(L.nf, 256), 256, 0, st>>>(0, L.nf, L.n, L.shape, sc.maxnbr, nbr, ncnt, status);
 #endif
 }
 
@@ -1059,7 +1225,7 @@ void export_neighbors(cudaStream_t st, const Layout &L, uint32_t row0, uint32_t 
                       const uint32_t *ncnt, const uint32_t *orig, uint32_t maxnbr, uint32_t *out_cnt,
                       uint32_t *out_nbr) {
     if (cnt)
-        k_export_neighbors<<<nblk(cnt, 256), 256, 0, st>>>(row0, cnt, L.ell_stride, nbr, ncnt, orig, maxnbr, out_cnt,
+        k_export_neighbors<<<nblk(cnt, 256), 256, 0, st>>>(row0, cnt, L.shape, nbr, ncnt, orig, maxnbr, out_cnt,
                                                            out_nbr);
 }
 void export_sorted(cudaStream_t st, const Scenes &sc, uint32_t n, const float4 *pos, const uint32_t *orig,
