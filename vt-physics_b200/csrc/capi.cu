@@ -369,6 +369,7 @@ vtp::PbfArgs vtp_solver::pbf_args() {
     a.vol = vol; a.density = density; a.lambda = lambda;
     a.unroll = unroll;
     a.lanes = row_lanes;
+    a.teams = teams;
     return a;
 }
 
@@ -477,7 +478,8 @@ int vtp_solver::initialize() {
     }
     L.merge_mode = mode < 0 ? 0 : mode;
     L.cell_cull = cell_cull;
-    teams = L.nf <= vtp::kTeamMaxRows && !persistent_tiles && type == VTP_SOLVER_DFSPH;
+    teams = L.nf <= vtp::kTeamMaxRows && !persistent_tiles &&
+            (type == VTP_SOLVER_DFSPH || type == VTP_SOLVER_PBF);
     L.shape.stride = vtp::list_stride(maxnbr > 1 ? maxnbr - 1 : 1);
     L.shape.lg = teams ? vtp::kTeamListLg : 0u;
 

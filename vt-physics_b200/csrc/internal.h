@@ -28,7 +28,9 @@ struct NvtxRange {
 // which is the events), thread per row -> team, us: DFSPH solve_a / solve_b / ratio + alpha /
 // viscosity at 2,000 rows 13.3 / 11.6 / 16.4 / 13.4 -> 9.9 / 8.5 / 9.4 / 10.4, at 32,000 rows
 // 14.5 / 12.6 / 18.7 / 14.8 -> 13.2 / 10.6 / 13.1 / 12.4, at 64,000 rows 16.4 / 14.4 / 18.8 / 16.6
-// -> 18.3 / 15.1 / 20.8 / 19.0.  A team executes 1.6 times the instructions of the thread, so past
+// -> 18.3 / 15.1 / 20.8 / 19.0; PBF lambda / dx / XSPH at 2,000 rows 16.9 / 12.4 / 14.6 -> 10.5 /
+// 10.3 / 10.6, at 32,000 rows 18.7 / 12.6 / 16.7 -> 14.7 / 12.6 / 12.6, at 64,000 rows 20.8 / 14.7
+// / 18.8 -> 20.7 / 16.7 / 18.8.  A team executes 1.6 times the instructions of the thread, so past
 // the row count that fills the GPU the thread wins (1,000,000 rows: solve_a 113 -> 168).
 constexpr uint32_t kTeamMaxRows = 49152;
 
