@@ -111,6 +111,7 @@ struct ImmState {
     uint32_t bodies_seen = 0;        // counter[5] at the last launch count
     float4 *tpk = nullptr;
     float4 *pk2 = nullptr;           // [2 nf] packed gather rows (viscosity -> tension / conformation)
+    float *bfrac_dev = nullptr;      // the same on the device (allocated by the first read of the fractions)
     std::vector<float> bfrac;        // boundary rows' phase fractions in attach order (host)
     cudaGraphConditionalHandle cond{};
 };
@@ -745,6 +746,14 @@ __global__ void k_phase_finish(ImmArgs a) {
     if (r == 0 && a.tick) *a.tick += 1;
 }
 
+// Fractions of the fluid rows into [attach id][phase].
+__global__ void k_fractions(ImmArgs a, const uint32_t *__restrict__ orig, float *__restrict__ out) {
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= a.nf) return;
+    float *o = out + (size_t)orig[r] * a.p.P;
+    for (int k = 0; k < a.p.P; ++k) o[k] = a.frac[k][r];
+}
+
 }  // namespace
 
 }  // namespace vtp
@@ -1133,10 +1142,28 @@ int immct_enqueue_tick(vtp_solver &s, cudaStream_t st, bool capture) {
     return VTP_OK;
 }
 
+// Phase fractions of every particle in attach order: the boundary's are the attached ones, kept on
+// the device from the first read on, and the fluid rows are scattered over them.
+static int imm_fractions(vtp_solver &s, float *dev_out) {
+    ImmState &m = *s.imm;
+    const size_t bytes = m.bfrac.size() * sizeof(float);
+    if (!m.bfrac_dev) {
+        int rc = s.alloc(&m.bfrac_dev, m.bfrac.size());
+        if (rc) return rc;
+        CUI(cudaMemcpyAsync(m.bfrac_dev, m.bfrac.data(), bytes, cudaMemcpyHostToDevice, s.st));
+    }
+    CUI(cudaMemcpyAsync(dev_out, m.bfrac_dev, bytes, cudaMemcpyDeviceToDevice, s.st));
+    if (s.L.nf) vtp::k_fractions<<<vtp::nblk(s.L.nf, 256), 256, 0, s.st>>>(imm_args(s), s.orig.c(), dev_out);
+    CUI(cudaGetLastError());
+    CUI(cudaStreamSynchronize(s.st));
+    return VTP_OK;
+}
+
 int immct_get_field(vtp_solver &s, int field, float *dev_out, size_t elems) {
     ImmState &m = *s.imm;
     const int P = m.p.P;
     const uint32_t n = s.L.n, nf = s.L.nf;
+    if (field == VTP_FIELD_VOL_FRAC) return imm_fractions(s, dev_out);
     std::vector<uint32_t> ids(n);
     CUI(cudaMemcpy(ids.data(), s.orig.c(), n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
     std::vector<float> out(n * elems, 0.f);
@@ -1147,14 +1174,7 @@ int immct_get_field(vtp_solver &s, int field, float *dev_out, size_t elems) {
     };
     std::vector<float> tmp;
     int rc;
-    if (field == VTP_FIELD_VOL_FRAC) {
-        for (uint32_t i = 0; i < n; ++i)
-            for (int k = 0; k < P; ++k) out[(size_t)i * P + k] = m.bfrac[(size_t)i * P + k];
-        for (int k = 0; k < P; ++k) {
-            if ((rc = fetch(m.frac[k].c(), tmp))) return rc;
-            for (uint32_t r = 0; r < nf; ++r) out[(size_t)ids[r] * P + k] = tmp[r];
-        }
-    } else if (field == VTP_FIELD_PHASE_VEL) {
+    if (field == VTP_FIELD_PHASE_VEL) {
         std::vector<float4> v4(nf);
         std::vector<float4> bv(n - nf);
         if (n > nf) CUI(cudaMemcpy(bv.data(), s.vel.c() + nf, (n - nf) * sizeof(float4), cudaMemcpyDeviceToHost));
