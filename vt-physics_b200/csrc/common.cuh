@@ -358,9 +358,10 @@ __device__ __forceinline__ float lane_sum(float v, unsigned mask) {
     return v;
 }
 
-// nbr_loop over a row's entries lane, lane + L, lane + 2L, ...: L lanes share
-// one row's list and each keeps U gathers in flight.  With L == 1 this is
-// nbr_loop itself (same order, same results).
+// nbr_loop over a row's entries lane, lane + L, lane + 2L, ...: L lanes share one row's list.  Each
+// takes U entries at a time - their U indices, then their U gathers in flight, the last partial
+// batch included - and loads the next batch's indices before it uses this one's data.  With L == 1
+// this is nbr_loop itself (same order, same results).
 template <int U, int L, class Load, class Use>
 __device__ __forceinline__ void nbr_loop_lanes(const uint32_t *__restrict__ lst, ListShape shape, uint32_t cnt, int lane,
                                                Load load, Use use) {
@@ -368,20 +369,28 @@ __device__ __forceinline__ void nbr_loop_lanes(const uint32_t *__restrict__ lst,
         nbr_loop_at<U>(lst, AnySlots{shape}, cnt, load, use);
     } else {
         using T = decltype(load(0u));
-        uint32_t t = (uint32_t)lane;
-        for (; t + (uint32_t)((U - 1) * L) < cnt; t += (uint32_t)(U * L)) {
-            uint32_t j[U];
+        uint32_t nxt[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) j[u] = __ldcs(lst + ell_slot(t + (uint32_t)(u * L), shape));
+        for (int u = 0; u < U; ++u) {
+            const uint32_t t = (uint32_t)(lane + u * L);
+            if (t < cnt) nxt[u] = __ldcs(lst + ell_slot(t, shape));
+        }
+        for (uint32_t t0 = (uint32_t)lane; t0 < cnt; t0 += (uint32_t)(U * L)) {
+            uint32_t j[U];
             T d[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) d[u] = load(j[u]);
+            for (int u = 0; u < U; ++u) j[u] = nxt[u];
 #pragma unroll
-            for (int u = 0; u < U; ++u) use(j[u], d[u]);
-        }
-        for (; t < cnt; t += (uint32_t)L) {
-            const uint32_t j = __ldcs(lst + ell_slot(t, shape));
-            use(j, load(j));
+            for (int u = 0; u < U; ++u)
+                if (t0 + (uint32_t)(u * L) < cnt) d[u] = load(j[u]);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const uint32_t t = t0 + (uint32_t)((U + u) * L);
+                if (t < cnt) nxt[u] = __ldcs(lst + ell_slot(t, shape));
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (t0 + (uint32_t)(u * L) < cnt) use(j[u], d[u]);
         }
     }
 }

@@ -166,8 +166,12 @@ __global__ void k_adj_gather(AdjArgs a) {
 // nbr_loop_lanes / lane_sum of common.cuh): with L = 1 one thread walks the row with four
 // neighbours' gathers in flight; with L > 1 the row's lanes take entries lane, lane + L, ...
 // (AU gathers in flight each, fewer registers) and a butterfly adds their partials.
+// The gathers in flight per lane are measured per pass: the correction's adjoint keeps 18 words a
+// neighbour and is best with one, the other two with two.
 template <int L>
-constexpr int adj_unroll() { return L == 1 ? 4 : (L == 2 ? 2 : 1); }
+constexpr int adj_unroll() { return L == 1 ? 4 : 2; }
+template <int L>
+constexpr int adj_unroll_dx() { return L == 1 ? 4 : 1; }
 
 // XSPH adjoint; epilogue: Delta-bar of the last constraint iteration.
 template <int L>
@@ -283,7 +287,7 @@ __global__ void __launch_bounds__(256) k_adj_dx(AdjArgs a) {
     const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
     const float ir = 1.f / a.rho0;
     float ax = 0.f, ay = 0.f, az = 0.f;
-    nbr_loop_lanes<adj_unroll<L>(), L>(lst, a.shape, n > 0 ? n - 1 : 0, lane,
+    nbr_loop_lanes<adj_unroll_dx<L>(), L>(lst, a.shape, n > 0 ? n - 1 : 0, lane,
                          [&](uint32_t j) {
                              DN e;
                              e.q = __ldg(a.x + j);
@@ -511,7 +515,12 @@ int adjoint_segment_l(vtp_solver *s, vtp::DiffState &d, uint32_t k, unsigned G, 
 }
 
 int adjoint_segment(vtp_solver *s, vtp::DiffState &d, uint32_t k, unsigned G, int tp) {
-    switch (s->adj_lanes) {
+    // Lanes per row unless configured: the fewer the rows, the more of the GPU a lane each leaves
+    // idle.  Backward of 6 recorded substeps with 1 / 2 / 4 / 8 lanes (B200, us): 5,832 rows 1101 / 876
+    // / 663 / 569, 13,824 rows 1169 / 948 / 760 / 684, 32,768 rows 1345 / 1183 / 1093 / 1098, 64,000
+    // rows 1815 / 1714 / 1769 / 1828, 216,000 rows 4432 / 4121 / 4199 / 4849.
+    const uint32_t rows = s->L.nf;
+    switch (s->adj_lanes ? s->adj_lanes : rows <= 24576 ? 8 : rows <= 49152 ? 4 : 2) {
         case 2: return adjoint_segment_l<2>(s, d, k, G, tp);
         case 4: return adjoint_segment_l<4>(s, d, k, G, tp);
         case 8: return adjoint_segment_l<8>(s, d, k, G, tp);

@@ -217,6 +217,26 @@ __device__ __forceinline__ float lanes_sum(float v) {
     return v;
 }
 
+// Gathered neighbour data: position, a vector, a scalar; the viscosity pass two vectors.
+struct IterA {
+    float4 q, v;
+    float k;
+};
+struct ViscA {
+    float4 q, u, w;
+};
+
+// The entries of a lane, the next entry's index loaded ahead of this entry's gathers
+// (nbr_loop_lanes).  One entry at a time: with two or four entries' gathers in flight the passes
+// need 60-109 registers and lose more to occupancy.  ncu launch times at 27,000 rows, without the
+// index ahead -> with it (4 entries in flight): iter_a 16.7 -> 14.4 (20.1) us, iter_b 16.0 -> 13.1
+// (13.8), ratio_x 14.1 -> 11.9 (17.6), visc 16.6 -> 15.9 (19.0), a1 9.3 -> 7.4 (8.9).
+template <int L, class Load, class Use>
+__device__ __forceinline__ void lanes_loop(const uint32_t *lst, ListShape shape, uint32_t n, uint32_t lane, Load load,
+                                           Use use) {
+    nbr_loop_lanes<1, L>(lst, shape, n > 0 ? n - 1 : 0, (int)lane, load, use);
+}
+
 // Pressure-solve iteration adjoint, pass A: kappa-bar_i = sum_j gradW_ij.w_ij with
 // w_ij = c_j V_i vb_j - c_i V_j vb_i (c = dt V / m; the j term only for fluid j), then
 // delta-bar (clamp of the forward), ratio-bar and alpha-bar, and the position adjoint of
@@ -235,17 +255,22 @@ __global__ void __launch_bounds__(256) k_dfd_iter_a(DfdArgs a) {
         const float ci = a.dt * p.w / a.mass_f;
         const uint32_t n = a.ncnt[r];
         const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
-        for (uint32_t t = lane; t + 1 < n; t += L) {
-            const uint32_t j = lst[ell_slot(t, a.shape)];
-            const float4 q = __ldg(a.x + j);
+        lanes_loop<L>(lst, a.shape, n, lane, [&](uint32_t j) {
+            IterA e;
+            e.q = __ldg(a.x + j);
+            e.k = __ldg(&a.rec[j].w);   // 0 for boundary rows
+            if (j < a.nf) e.v = __ldg(a.vb + j);
+            return e;
+        }, [&](uint32_t j, const IterA &e) {
+            const float4 q = e.q;
             const bool fj = j < a.nf;
-            const float kj = __ldg(&a.rec[j].w);   // 0 for boundary rows
+            const float kj = e.k;
             const float rx = p.x - q.x, ry = p.y - q.y, rz = p.z - q.z;
             const float d2 = dist2(rx, ry, rz);
             const float gg = cubic_g(d2, a.k), hh = cubic_hh(d2, a.k);
             float wx = -ci * q.w * vi.x, wy = -ci * q.w * vi.y, wz = -ci * q.w * vi.z;
             if (fj) {
-                const float4 vj = __ldg(a.vb + j);
+                const float4 vj = e.v;
                 const float cj = a.dt * q.w / a.mass_f * p.w;
                 wx += cj * vj.x;
                 wy += cj * vj.y;
@@ -257,7 +282,7 @@ __global__ void __launch_bounds__(256) k_dfd_iter_a(DfdArgs a) {
             xx += kk * (gg * wx + hh * rx * rw);
             xy += kk * (gg * wy + hh * ry * rw);
             xz += kk * (gg * wz + hh * rz * rw);
-        }
+        });
     }
     kb = lanes_sum<L>(kb);
     xx = lanes_sum<L>(xx);
@@ -288,13 +313,18 @@ __global__ void __launch_bounds__(256) k_dfd_iter_b(DfdArgs a) {
         const float di = a.db[r];
         const uint32_t n = a.ncnt[r];
         const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
-        for (uint32_t t = lane; t + 1 < n; t += L) {
-            const uint32_t j = lst[ell_slot(t, a.shape)];
-            const float4 q = __ldg(a.x + j), sj = __ldg(a.rec + j);
+        lanes_loop<L>(lst, a.shape, n, lane, [&](uint32_t j) {
+            IterA e;
+            e.q = __ldg(a.x + j);
+            e.v = __ldg(a.rec + j);
+            if (j < a.nf) e.k = __ldg(a.db + j);
+            return e;
+        }, [&](uint32_t j, const IterA &e) {
+            const float4 q = e.q, sj = e.v;
             const float rx = p.x - q.x, ry = p.y - q.y, rz = p.z - q.z;
             const float d2 = dist2(rx, ry, rz);
             const float gg = cubic_g(d2, a.k), hh = cubic_hh(d2, a.k);
-            const float c = a.dt * (q.w * di + (j < a.nf ? p.w * __ldg(a.db + j) : 0.f));
+            const float c = a.dt * (q.w * di + (j < a.nf ? p.w * e.k : 0.f));
             const float ux = si.x - sj.x, uy = si.y - sj.y, uz = si.z - sj.z;
             const float ru = rx * ux + ry * uy + rz * uz;
             vx += c * gg * rx;
@@ -303,7 +333,7 @@ __global__ void __launch_bounds__(256) k_dfd_iter_b(DfdArgs a) {
             xx += c * (gg * ux + hh * rx * ru);
             xy += c * (gg * uy + hh * ry * ru);
             xz += c * (gg * uz + hh * rz * ru);
-        }
+        });
     }
     vx = lanes_sum<L>(vx);
     vy = lanes_sum<L>(vy);
@@ -336,10 +366,17 @@ __global__ void __launch_bounds__(256) k_dfd_visc(DfdArgs a) {
         wi = a.vb[r];
         const uint32_t n = a.ncnt[r];
         const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
-        for (uint32_t t = lane; t + 1 < n; t += L) {
-            const uint32_t j = lst[ell_slot(t, a.shape)];
-            if (j >= a.nf) continue;   // same-material neighbours only
-            const float4 q = __ldg(a.x + j), uj = __ldg(a.vp + j), wj = __ldg(a.vb + j);
+        lanes_loop<L>(lst, a.shape, n, lane, [&](uint32_t j) {
+            ViscA e;
+            if (j < a.nf) {
+                e.q = __ldg(a.x + j);
+                e.u = __ldg(a.vp + j);
+                e.w = __ldg(a.vb + j);
+            }
+            return e;
+        }, [&](uint32_t j, const ViscA &e) {
+            if (j >= a.nf) return;   // same-material neighbours only
+            const float4 q = e.q, uj = e.u, wj = e.w;
             const float rx = p.x - q.x, ry = p.y - q.y, rz = p.z - q.z;
             const float d2 = dist2(rx, ry, rz);
             const float gg = cubic_g(d2, a.k), hh = cubic_hh(d2, a.k);
@@ -358,7 +395,7 @@ __global__ void __launch_bounds__(256) k_dfd_visc(DfdArgs a) {
             xy += cx * (phi * uy * rw + ru * (phi * wy + psi * ry * rw));
             xz += cx * (phi * uz * rw + ru * (phi * wz + psi * rz * rw));
             ps += ru * phi * (rx * wi.x + ry * wi.y + rz * wi.z);
-        }
+        });
     }
     vx = lanes_sum<L>(vx);
     vy = lanes_sum<L>(vy);
@@ -398,15 +435,13 @@ __global__ void __launch_bounds__(256) k_dfd_a1(DfdArgs a) {
         const float4 p = a.x[r];
         const uint32_t n = a.ncnt[r];
         const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
-        for (uint32_t t = lane; t + 1 < n; t += L) {
-            const uint32_t j = lst[ell_slot(t, a.shape)];
-            const float4 q = __ldg(a.x + j);
+        lanes_loop<L>(lst, a.shape, n, lane, [&](uint32_t j) { return __ldg(a.x + j); }, [&](uint32_t, const float4 &q) {
             const float rx = p.x - q.x, ry = p.y - q.y, rz = p.z - q.z;
             const float gg = cubic_g(dist2(rx, ry, rz), a.k) * q.w;
             ax += gg * rx;
             ay += gg * ry;
             az += gg * rz;
-        }
+        });
     }
     ax = lanes_sum<L>(ax);
     ay = lanes_sum<L>(ay);
@@ -432,12 +467,19 @@ __global__ void __launch_bounds__(256) k_dfd_ratio_x(DfdArgs a) {
         const uint32_t n = a.ncnt[r];
         const uint32_t *lst = a.nbr + ell_index(r, 0, a.shape);
         const float im = 1.f / a.mass_f;
-        for (uint32_t t = lane; t + 1 < n; t += L) {
-            const uint32_t j = lst[ell_slot(t, a.shape)];
-            const float4 q = __ldg(a.x + j);
+        lanes_loop<L>(lst, a.shape, n, lane, [&](uint32_t j) {
+            IterA e;
+            e.q = __ldg(a.x + j);
+            if (j < a.nf) {
+                e.v = __ldg(a.a1b + j);
+                e.k = __ldg(a.rbar + j);
+            }
+            return e;
+        }, [&](uint32_t j, const IterA &e) {
+            const float4 q = e.q;
             const bool fj = j < a.nf;
-            const float4 Aj = fj ? __ldg(a.a1b + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float rbj = fj ? __ldg(a.rbar + j) : 0.f;
+            const float4 Aj = fj ? e.v : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float rbj = fj ? e.k : 0.f;
             const float rx = p.x - q.x, ry = p.y - q.y, rz = p.z - q.z;
             const float d2 = dist2(rx, ry, rz);
             const float gg = cubic_g(d2, a.k), hh = cubic_hh(d2, a.k);
@@ -449,7 +491,7 @@ __global__ void __launch_bounds__(256) k_dfd_ratio_x(DfdArgs a) {
             xx += s * rx + gg * wx + hh * rx * rw;
             xy += s * ry + gg * wy + hh * ry * rw;
             xz += s * rz + gg * wz + hh * rz * rw;
-        }
+        });
     }
     xx = lanes_sum<L>(xx);
     xy = lanes_sum<L>(xy);
