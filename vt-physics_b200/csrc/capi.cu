@@ -553,6 +553,7 @@ int vtp_solver::initialize() {
     u.scan_tiles = ((size_t)nbuckets + 2047) / 2048;
     if (u.scan_tiles > 1024 * 64) return fail(VTP_ERR_BOUNDS, "grid too large for the cell scan");
     AL(&u.scan_sums, u.scan_tiles);
+    CU(cudaMemsetAsync(u.scan_sums, 0, u.scan_tiles * sizeof(uint32_t), st));
     const size_t fl_rows = ((size_t)L.nf + 31) / 32 * 32, bl_rows = ((size_t)L.nb + 31) / 32 * 32;
     AL(&u.nbr, fl_rows * L.shape.stride);
     AL(&u.ncnt, L.nf);
@@ -839,7 +840,7 @@ int vtp_solver::enqueue_pbf_substep(cudaStream_t s, const PbfTapeSlot *tape) {
     uint32_t *lnbr = tape ? tape->nbr : u.nbr, *lcnt = tape ? tape->ncnt : u.ncnt;
     PROF(this, "ugns_lists", vtp::ugns_build_lists(s, scn(), L, 0, L.nf, pos.c(), orig.c(), u, lnbr, lcnt,
                                                    d_status, d_overflow));
-    launches_per_tick += 7;  // hash, 3 scan kernels, scatter, rank/reorder, lists
+    launches_per_tick += vtp::ugns_sort_launches(nbuckets) + 1;  // sort, lists
     if (tape && nf) {
         CU(cudaMemcpyAsync(tape->orig, orig.c(), nf * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
         CU(cudaMemcpyAsync(tape->x[0], pos.c(), nf * sizeof(float4), cudaMemcpyDeviceToDevice, s));

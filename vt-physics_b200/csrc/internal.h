@@ -55,7 +55,7 @@ struct UgnsBuffers {
     uint32_t *tmp_src = nullptr;   // [max(nf, nb)] scattered: old slot
     uint32_t *tmp_orig = nullptr;  // [max(nf, nb)] scattered: attach id
     uint32_t *tmp_key = nullptr;   // [max(nf, nb)] scattered: key
-    uint32_t *scan_sums = nullptr; // [tiles]
+    uint32_t *scan_sums = nullptr; // [tiles] zero between sorts where the hash counts into it
     uint32_t *nbr = nullptr;       // ELL list for fluid rows
     uint32_t *ncnt = nullptr;      // [nf] neighbour count incl. self (0 = outside the grid)
     uint32_t *bnbr = nullptr;      // ELL list for boundary rows (init / diagnostics)
@@ -103,6 +103,9 @@ void ugns_sort(cudaStream_t st, const Scenes &sc, uint32_t nbuckets, uint32_t ro
                const float4 *pos_in, float4 *pos_out, const float4 *vel_in, float4 *vel_out,
                const uint32_t *orig_in, uint32_t *orig_out, const Carry &carry,
                float force_dt, UgnsBuffers &u, uint32_t *start, Profiler *prof = nullptr);
+
+// Kernels a sort over `nbuckets` buckets launches.
+uint32_t ugns_sort_launches(uint32_t nbuckets);
 
 // Build the neighbour lists of rows [row0, row0 + cnt) (reference order:
 // 27 offsets, then ascending attach id inside a cell).

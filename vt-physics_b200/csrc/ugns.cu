@@ -43,12 +43,11 @@ __device__ __forceinline__ float4 apply_force(float4 p, float4 &v, float dt, flo
     return p;
 }
 
-__global__ void k_hash(Scenes sc, uint32_t row0, uint32_t cnt, const float4 *__restrict__ pos,
-                       const float4 *__restrict__ vel, float force_dt, uint32_t *__restrict__ key,
-                       uint32_t *__restrict__ rank, uint32_t *__restrict__ count) {
-    pdl_enter();
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cnt) return;
+// Bucket and arrival rank of one row, its bucket's counter advanced.
+__device__ __forceinline__ uint32_t hash_row(const Scenes &sc, uint32_t row0, uint32_t i,
+                                             const float4 *__restrict__ pos, const float4 *__restrict__ vel,
+                                             float force_dt, uint32_t *__restrict__ rank,
+                                             uint32_t *__restrict__ count) {
     const SceneGrid g = load_scene(sc, row0 + i);
     float4 p = pos[row0 + i];
     if (force_dt > 0.f) {
@@ -58,7 +57,6 @@ __global__ void k_hash(Scenes sc, uint32_t row0, uint32_t cnt, const float4 *__r
     int3 c = cell_of(p.x, p.y, p.z, g, sc.cell);
     const bool outside = !cell_available(c, g);
     uint32_t k = g.key_base + (outside ? g.nkey : cell_key(c, g));
-    key[i] = k;
     const unsigned om = __ballot_sync(__activemask(), outside);
     if (outside) {
         // Every row outside its scene's grid counts into the scene's one outside bucket (whole
@@ -75,6 +73,31 @@ __global__ void k_hash(Scenes sc, uint32_t row0, uint32_t cnt, const float4 *__r
     } else {
         rank[i] = atomicAdd(&count[k], 1u);
     }
+    return k;
+}
+
+// `sums` (or null): the scan's tile sums are counted as well.
+__global__ void k_hash(Scenes sc, uint32_t row0, uint32_t cnt, const float4 *__restrict__ pos,
+                       const float4 *__restrict__ vel, float force_dt, uint32_t *__restrict__ key,
+                       uint32_t *__restrict__ rank, uint32_t *__restrict__ count, uint32_t *__restrict__ sums) {
+    pdl_enter();
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t k = 0;
+    if (i < cnt) {
+        k = hash_row(sc, row0, i, pos, vel, force_dt, rank, count);
+        key[i] = k;
+    }
+    if (!sums) return;
+    // The rows are nearly sorted already: a block's rows mostly fall in its first row's tile, and
+    // go in with one atomic (one per warp cost 10 us at 1,000,000 rows).
+    __shared__ uint32_t first;
+    const uint32_t t = k / kScanTile;
+    if (threadIdx.x == 0) first = t;
+    __syncthreads();
+    const bool other = i < cnt && t != first;
+    const int n = __syncthreads_count(i < cnt && !other);
+    if (threadIdx.x == 0) atomicAdd(&sums[first], (uint32_t)n);
+    if (other) atomicAdd(&sums[t], 1u);
 }
 
 // Block-wide exclusive scan of one value per thread; returns the block total.
@@ -142,11 +165,21 @@ __global__ void __launch_bounds__(1024) k_scan_sums(uint32_t *sums, size_t tiles
 
 // Exclusive scan of the counters into `out` (plus `base_add`), out[n] = grand
 // total.  The counters are zeroed after they are read, so the next hash starts
-// from zero without a separate clear.
+// from zero without a separate clear.  PREFIX: `sums` holds the tiles' own sums
+// (counted by k_hash) and each block adds up those before it; else their scan.
+template <bool PREFIX>
 __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(uint32_t *__restrict__ in, size_t n,
                                                              const uint32_t *__restrict__ sums, uint32_t base_add,
                                                              uint32_t *__restrict__ out) {
     pdl_enter();
+    uint32_t before = 0;
+    if (PREFIX) {
+        uint32_t v = 0;
+        for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kScanThreads) v += sums[t];
+        block_excl_scan(v, before);
+    } else {
+        before = sums[blockIdx.x];
+    }
     // Each thread scans kScanItems consecutive counters.
     __shared__ uint32_t tile[kScanTile];
     size_t t0 = (size_t)blockIdx.x * kScanTile;
@@ -164,7 +197,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(uint32_t *__restric
         s += vals[k];
     }
     uint32_t total;
-    uint32_t off = block_excl_scan(s, total) + sums[blockIdx.x] + base_add;
+    uint32_t off = block_excl_scan(s, total) + before + base_add;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         const size_t idx = t0 + (size_t)threadIdx.x * kScanItems + k;
@@ -182,9 +215,12 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(uint32_t *__restric
 __global__ void k_scatter(uint32_t row0, uint32_t cnt, const uint32_t *__restrict__ key,
                           const uint32_t *__restrict__ rank, const uint32_t *__restrict__ start,
                           const uint32_t *__restrict__ orig, uint32_t *__restrict__ tmp_src,
-                          uint32_t *__restrict__ tmp_orig, uint32_t *__restrict__ tmp_key, uint32_t *status) {
+                          uint32_t *__restrict__ tmp_orig, uint32_t *__restrict__ tmp_key, uint32_t *status,
+                          uint32_t *__restrict__ sums, uint32_t tiles) {
     pdl_enter();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (sums)   // the scan has read them: zero for the next hash
+        for (uint32_t t = i; t < tiles; t += gridDim.x * blockDim.x) sums[t] = 0u;
     if (i >= cnt) return;
     uint32_t k = key[i];
     uint32_t d = start[k] - row0 + rank[i];
@@ -1001,12 +1037,27 @@ int cubic_sigma_device(cudaStream_t st, float h, float *out_host) {
     return e == cudaSuccess ? 0 : 1;
 }
 
+// Up to this many scan tiles (2,048 cells each) the hash counts the tiles' sums as well and each
+// block of the scan adds up the sums before its own (at most 4 a thread): one launch in place of
+// three, which for a small grid is most of the scan's time.  B200, event-timed, about 5 us of it
+// the events: 2,000 rows 12.3 -> 8.4 us, 250,000 rows 12.6 -> 8.6, 1,000,000 rows 16.7 -> 8.7; the
+// hash keeps its time (14.5 -> 15.3 at 1,000,000 rows).
+constexpr size_t kPrefixTiles = 1024;
+
 static void scan_counts(cudaStream_t st, uint32_t *count, size_t n, uint32_t base_add, uint32_t *out,
                         UgnsBuffers &u) {
     size_t tiles = (n + kScanTile - 1) / kScanTile;
+    if (tiles <= kPrefixTiles) {
+        launch(k_scan_tiles<true>, (unsigned)tiles, kScanThreads, 0, st, count, n, u.scan_sums, base_add, out);
+        return;
+    }
     launch(k_scan_tile_sums, (unsigned)tiles, kScanThreads, 0, st, count, n, u.scan_sums);
     launch(k_scan_sums, 1, 1024, 0, st, u.scan_sums, tiles);
-    launch(k_scan_tiles, (unsigned)tiles, kScanThreads, 0, st, count, n, u.scan_sums, base_add, out);
+    launch(k_scan_tiles<false>, (unsigned)tiles, kScanThreads, 0, st, count, n, u.scan_sums, base_add, out);
+}
+
+uint32_t ugns_sort_launches(uint32_t nbuckets) {   // hash, scan, scatter, rank / reorder
+    return ((size_t)nbuckets + kScanTile - 1) / kScanTile <= kPrefixTiles ? 4u : 6u;
 }
 
 void ugns_sort(cudaStream_t st, const Scenes &sc, uint32_t nbuckets, uint32_t row0, uint32_t cnt,
@@ -1017,9 +1068,13 @@ void ugns_sort(cudaStream_t st, const Scenes &sc, uint32_t nbuckets, uint32_t ro
     auto B = [&] { if (prof) prof->begin(); };
     auto E = [&](const char *nm) { if (prof) prof->end_(nm); };
     B();
-    // u.count is all zero here: zeroed once at allocation and by every scan after reading it.
+    // u.count is all zero here: zeroed once at allocation and by every scan after reading it; the
+    // same holds for u.scan_sums (by the scatter) where the hash counts into it.
+    const size_t tiles = (nb + kScanTile - 1) / kScanTile;
+    uint32_t *const sums = tiles <= kPrefixTiles ? u.scan_sums : nullptr;
     if (cnt > 0) {
-        launch(k_hash, nblk(cnt, 256), 256, 0, st, sc, row0, cnt, pos_in, vel_in, force_dt, u.key, u.rank, u.count);
+        launch(k_hash, nblk(cnt, 256), 256, 0, st, sc, row0, cnt, pos_in, vel_in, force_dt, u.key, u.rank, u.count,
+               sums);
     }
     E("ugns_clear_hash");
     B();
@@ -1028,7 +1083,7 @@ void ugns_sort(cudaStream_t st, const Scenes &sc, uint32_t nbuckets, uint32_t ro
     if (cnt == 0) return;
     B();
     launch(k_scatter, nblk(cnt, 256), 256, 0, st, row0, cnt, u.key, u.rank, start, orig_in, u.tmp_src, u.tmp_orig,
-           u.tmp_key, u.status);
+           u.tmp_key, u.status, sums, (uint32_t)tiles);
     E("ugns_scatter");
     B();
     launch(k_rank_reorder, nblk(cnt, 256), 256, 0, st, sc, row0, cnt, start, u.tmp_src, u.tmp_orig, u.tmp_key, pos_in,
