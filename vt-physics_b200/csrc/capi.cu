@@ -392,7 +392,7 @@ vtp::DfsphArgs vtp_solver::dfsph_args(int which) {
     a.tiles = d_tiles; a.ntiles = ntiles; a.scene_tiles = d_scene_tiles; a.persistent = persistent_tiles;
     a.state = solve ? solve + (size_t)which * scenes.size() : nullptr;
     a.sc = scn();
-    a.pva = pva;
+    a.pva = which == 0 ? pva : pva2;
     a.pk = pk;
     a.tick = d_tick;
     a.unroll = unroll;
@@ -619,6 +619,8 @@ int vtp_solver::initialize() {
     } else {
         for (int k = 0; k < 2; ++k) AL(&vadv.b[k], n);
         AL(&pva, 2 * (size_t)n);
+        pva2 = pva;
+        if (type == VTP_SOLVER_DFSPH) { AL(&pva2, 2 * (size_t)n); }
         AL(&pk, n);
         AL(&ratio, L.nf);
         AL(&alpha, L.nf);
@@ -732,6 +734,7 @@ int vtp_solver::initialize() {
         vtp::DfsphArgs a = dfsph_args();
         vtp::dfsph_rigid_volume(st, a, u.bncnt, u.bnbr, rest_b);
         CU(cudaMemcpyAsync(pos.n() + L.nf, pos.c() + L.nf, (size_t)L.nb * sizeof(float4), cudaMemcpyDeviceToDevice, st));
+        vtp::dfsph_pack_boundary(st, dfsph_args(), pva2);
         if (type != VTP_SOLVER_DFSPH) {
             if ((rc = immct_init(*this))) return rc;
         }
@@ -752,12 +755,15 @@ int vtp_solver::initialize() {
 
 // ---------------------------------------------------------------- tick
 
-int vtp_solver::enqueue_solve(cudaStream_t s, int which, bool capture) {
+// packed: an earlier pass of the substep has reset the solve's states and packed its rows.
+int vtp_solver::enqueue_solve(cudaStream_t s, int which, bool capture, bool packed) {
     const vtp::NvtxRange nvtx_range(which == 0 ? "vtp divergence solve" : "vtp density solve");
     vtp::DfsphArgs a = dfsph_args(which);
-    vtp::dfsph_solve_begin(s, solve + (size_t)which * scenes.size(), loop + which, nscenes());
-    PROF(this, "dfsph_solve_pack", vtp::dfsph_solve_pack(s, a));
-    launches_per_tick += 2;
+    if (!packed) {
+        PROF(this, "dfsph_solve_pack", vtp::dfsph_solve_pack(s, a, solve + (size_t)which * scenes.size(), loop + which,
+                                                             nscenes()));
+        launches_per_tick += 1;
+    }
     if (capture && device_loop) {
         cudaStreamCaptureStatus cs;
         cudaGraph_t g;
@@ -895,10 +901,19 @@ int vtp_solver::enqueue_tick(cudaStream_t s, bool capture) {
         PROF(this, "ugns_lists", vtp::ugns_build_lists(s, scn(), L, 0, L.nf, pos.c(), orig.c(), u, u.nbr, u.ncnt,
                                                        d_status, d_overflow));
     }
-    PROF(this, "dfsph_ratio_alpha", vtp::dfsph_ratio_alpha(s, dfsph_args(), block));
-    launches_per_tick += 8;  // neighbour search (7) + ratio/alpha
-    if ((rc = enqueue_solve(s, 0, capture))) return rc;
+    // The ratio / alpha pass packs the divergence solve's rows and starts both solves, the forces
+    // pass packs the density solve's.
+    const bool packed = L.nf > 0;
+    vtp::DfsphArgs ra = dfsph_args();
+    ra.pack = pva;
+    ra.reset = solve;
+    ra.reset_loop = loop;
+    ra.nreset = nscenes();
+    PROF(this, "dfsph_ratio_alpha", vtp::dfsph_ratio_alpha(s, ra, block));
+    launches_per_tick += vtp::ugns_sort_launches(nbuckets) + 2;  // sort, lists, ratio / alpha
+    if ((rc = enqueue_solve(s, 0, capture, packed))) return rc;
     vtp::DfsphArgs a = dfsph_args();
+    a.pack = pva2;
     PROF(this, "dfsph_pressure_pack", vtp::dfsph_pressure_pack(s, a));
     launches_per_tick += 1;
     if (gamma == 0.f) {
@@ -911,7 +926,7 @@ int vtp_solver::enqueue_tick(cudaStream_t s, bool capture) {
         launches_per_tick += 2;
     }
     vel.swap(); vadv.swap();
-    if ((rc = enqueue_solve(s, 1, capture))) return rc;
+    if ((rc = enqueue_solve(s, 1, capture, packed))) return rc;
     PROF(this, "dfsph_finalize", vtp::dfsph_finalize(s, dfsph_args()));
     launches_per_tick += 1;
     return VTP_OK;

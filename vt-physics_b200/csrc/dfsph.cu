@@ -96,6 +96,21 @@ __global__ void __launch_bounds__(256) k_rigid_volume(DfsphArgs a, const uint32_
     rest_density_b[r] = vb * a.rho_b;
 }
 
+__device__ __forceinline__ void reset_solve(SolveState *s, LoopState *loop, int nscenes);
+
+// What the ratio / alpha pass prepares beside its own results for the solver's substep: both
+// solves' states (first block), and row r's {pos, v*} for the first one.
+__device__ __forceinline__ void start_solves(const DfsphArgs &a) {
+    if (!a.reset || blockIdx.x != 0) return;
+    reset_solve(a.reset, a.reset_loop, a.nreset);
+    reset_solve(a.reset + a.nreset, a.reset_loop + 1, a.nreset);
+}
+__device__ __forceinline__ void pack_row(const DfsphArgs &a, uint32_t r, const float4 &p, const float4 &v) {
+    if (!a.pack) return;
+    a.pack[2 * (size_t)r] = p;
+    a.pack[2 * (size_t)r + 1] = v;
+}
+
 // DFSPH compression ratio and alpha of one row (compute_compression_ratio_cuda +
 // compute_df_beta_cuda, DFSPHCudaImpl.cu:85-140), accumulated entry by entry in list
 // order, every rounding explicit.
@@ -135,6 +150,7 @@ struct PN {
 
 template <int U>
 __global__ void __launch_bounds__(256) k_ratio_alpha(DfsphArgs a) {
+    start_solves(a);
     uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= a.nf || halo_ghost(a, r)) return;
     const float4 p = a.pos[r];
@@ -148,6 +164,7 @@ __global__ void __launch_bounds__(256) k_ratio_alpha(DfsphArgs a) {
                     const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
                     ra.add(dist2(dx, dy, dz), dx, dy, dz, q.w, j < a.nf, a.k, inv_mf);
                 });
+    if (a.pack) pack_row(a, r, p, a.vadv[r]);
     a.ratio[r] = ra.ratio;
     a.alpha[r] = ra.alpha(a.mass_f);
 }
@@ -155,6 +172,7 @@ __global__ void __launch_bounds__(256) k_ratio_alpha(DfsphArgs a) {
 // The same with a team per row (team.cuh).
 __global__ void __launch_bounds__(kTeamBlock) k_team_ratio_alpha(DfsphArgs a) {
     __shared__ TeamTerms<8> S;   // V_j, W, gradW, |gradW|^2 V_j^2 (fluid j)
+    start_solves(a);
     const uint32_t r = blockIdx.x * kTeamRows + team_row(), l = team_lane();
     const bool live = r < a.nf && !halo_ghost(a, r);
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -192,6 +210,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_ratio_alpha(DfsphArgs a) {
     ra.a1z = team_get(acc, 3);
     ra.a2 = a2;
     if (!live || l != 0) return;
+    if (a.pack) pack_row(a, r, p, a.vadv[r]);
     a.ratio[r] = ra.ratio;
     a.alpha[r] = ra.alpha(a.mass_f);
 }
@@ -576,19 +595,8 @@ __global__ void k_pressure_pack(DfsphArgs a) {
     a.pva[2 * (size_t)r + 1] = pressure_applied(a.vel[r], a.vadv[r], T.inv_dt, T.dt);
 }
 
-__global__ void k_solve_pack(DfsphArgs a, uint32_t n) {
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n) return;
-    const float4 p = a.pos[r];
-    a.pva[2 * (size_t)r] = p;
-    a.pva[2 * (size_t)r + 1] = a.vadv[r];
-    // With peer-store halos a ghost's {x, kappa} row is written only by its owner's solve_a
-    // (which may already be storing it: no fence separates this pack from the peers' solve_a).
-    if (r < a.nf && halo_ghost(a, r)) return;
-    a.pk[r] = r < a.nf ? make_float4(p.x, p.y, p.z, 0.f) : p;
-}
-
-__global__ void k_solve_begin(SolveState *s, LoopState *loop, int nscenes) {
+// Starts `nscenes` solve states and a loop state (called by one block).
+__device__ __forceinline__ void reset_solve(SolveState *s, LoopState *loop, int nscenes) {
     for (int i = threadIdx.x; i < nscenes; i += blockDim.x) {
         s[i].iter = 0;
         s[i].stopped = 0;
@@ -600,6 +608,30 @@ __global__ void k_solve_begin(SolveState *s, LoopState *loop, int nscenes) {
         loop->iters = 0;
     }
 }
+
+__global__ void k_solve_pack(DfsphArgs a, SolveState *state, LoopState *loop, int nscenes) {
+    if (state && blockIdx.x == 0) reset_solve(state, loop, nscenes);
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= a.nf) return;
+    const float4 p = a.pos[r];
+    a.pva[2 * (size_t)r] = p;
+    a.pva[2 * (size_t)r + 1] = a.vadv[r];
+    // With peer-store halos a ghost's {x, kappa} row is written only by its owner's solve_a
+    // (which may already be storing it: no fence separates this pack from the peers' solve_a).
+    if (halo_ghost(a, r)) return;
+    a.pk[r] = make_float4(p.x, p.y, p.z, 0.f);
+}
+
+__global__ void k_pack_boundary(DfsphArgs a, float4 *pva2) {
+    const uint32_t r = a.nf + blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= a.nf + a.nb) return;
+    const float4 p = a.pos[r], v = a.vadv[r];
+    a.pva[2 * (size_t)r] = pva2[2 * (size_t)r] = p;
+    a.pva[2 * (size_t)r + 1] = pva2[2 * (size_t)r + 1] = v;
+    a.pk[r] = p;
+}
+
+__global__ void k_solve_begin(SolveState *s, LoopState *loop, int nscenes) { reset_solve(s, loop, nscenes); }
 
 // A tile's sum from the sums of its 32-row pieces, in the order a block sum over the tile adds its
 // warps (block_sum: halving strides).
@@ -713,6 +745,7 @@ __device__ __forceinline__ void finish_viscosity(const DfsphArgs &a, const StepD
     o.z = __fmaf_rn(accz, T.dt, vi.z);
     a.vel_alt[r] = o;
     a.vadv_alt[r] = o;
+    if (a.pack) pack_row(a, r, a.pos[r], o);
     halo_each(a, r, [&](const PeerRows &P, uint32_t q) {
         P.vel[a.halo_vel ^ 1][q] = o;
         P.vadv[a.halo_vadv ^ 1][q] = o;
@@ -730,6 +763,7 @@ __device__ __forceinline__ void finish_tension(const DfsphArgs &a, const StepDt 
     o.z = __fmaf_rn(acc.z + tz, T.dt, vi.z);
     a.vel_alt[r] = o;
     a.vadv_alt[r] = o;
+    if (a.pack) pack_row(a, r, a.pos[r], o);
     halo_each(a, r, [&](const PeerRows &P, uint32_t q) {
         P.vel[a.halo_vel ^ 1][q] = o;
         P.vadv[a.halo_vadv ^ 1][q] = o;
@@ -988,9 +1022,11 @@ void dfsph_ratio_alpha(cudaStream_t st, const DfsphArgs &a, int block) {
 void dfsph_solve_begin(cudaStream_t st, SolveState *s, LoopState *loop, int nscenes) {
     k_solve_begin<<<1, 256, 0, st>>>(s, loop, nscenes);
 }
-void dfsph_solve_pack(cudaStream_t st, const DfsphArgs &a) {
-    const uint32_t n = a.nf + a.nb;
-    if (n) k_solve_pack<<<nblk(n, 256), 256, 0, st>>>(a, n);
+void dfsph_solve_pack(cudaStream_t st, const DfsphArgs &a, SolveState *state, LoopState *loop, int nscenes) {
+    if (a.nf || state) k_solve_pack<<<nblk(std::max(a.nf, 1u), 256), 256, 0, st>>>(a, state, loop, nscenes);
+}
+void dfsph_pack_boundary(cudaStream_t st, const DfsphArgs &a, float4 *pva2) {
+    if (a.nb) k_pack_boundary<<<nblk(a.nb, 256), 256, 0, st>>>(a, pva2);
 }
 template <class K>
 static void launch_staged(K kern, cudaStream_t st, const DfsphArgs &a, size_t row_bytes) {

@@ -71,6 +71,11 @@ struct DfsphArgs {
     const float *rest_density;  // IMM / IMM-CT: per-row rest density (mass = rest_density * volume)
     // Packed gather rows of the pressure solve (filled by dfsph_solve_pack):
     float4 *pva;                // [2n] row j = {pos_j, v*_j} (32 B): one 256-bit load per pair in solve_a
+    float4 *pack;               // ratio / alpha and the forces pass: also leave the next solve's {pos, v*} rows here
+                                // (null: dfsph_solve_pack does it)
+    SolveState *reset;          // ratio / alpha: also start the substep's solves (2 x nreset states, 2 loops); null: not
+    LoopState *reset_loop;
+    int nreset;
     float4 *pk;                 // [n] {x, y, z, kappa_j} for fluid rows, {x, y, z, V_j} for boundary rows
     // Staged pressure solve (single scene, bricked order): one block per cell group gathers
     // its neighbours from a shared-memory copy of the group's neighbourhood through the slot
@@ -111,8 +116,12 @@ void dfsph_rigid_volume(cudaStream_t st, const DfsphArgs &a, const uint32_t *bnc
                         float *rest_density_b);
 void dfsph_ratio_alpha(cudaStream_t st, const DfsphArgs &a, int block);
 void dfsph_solve_begin(cudaStream_t st, SolveState *s, LoopState *loop, int nscenes);
-// Packs pva / pk for a pressure solve (after v* and positions are final for it).
-void dfsph_solve_pack(cudaStream_t st, const DfsphArgs &a);
+// Packs the fluid rows of pva / pk for a pressure solve (after v* and positions are final for it);
+// with `state`, dfsph_solve_begin is part of the same launch.
+void dfsph_solve_pack(cudaStream_t st, const DfsphArgs &a, SolveState *state = nullptr, LoopState *loop = nullptr,
+                      int nscenes = 0);
+// The boundary rows of pva / pk and of a second pva; they never change.
+void dfsph_pack_boundary(cudaStream_t st, const DfsphArgs &a, float4 *pva2);
 void dfsph_solve_a(cudaStream_t st, const DfsphArgs &a, int block);
 void dfsph_solve_b(cudaStream_t st, const DfsphArgs &a, int block);
 void dfsph_solve_end(cudaStream_t st, const SolveCtl &c, const double *partials, uint32_t *status);

@@ -482,6 +482,7 @@ int vtp_domain_create(const char *config_json, const float *fluid_pos, uint32_t 
         if ((rc = vtp_solver_initialize(d->s))) return rc;
         vtp_solver *s = d->s;
         if (s->L.nf != capacity || s->L.nb != nb) return fail(VTP_ERR_STATE, "domain worker layout");
+        s->pva2 = s->pva;   // one set of packed rows: the peers store into it, and each solve packs it anew
         d->st = s->st;
         CU(cudaMallocHost((void **)&d->h_status, 2 * sizeof(uint32_t)));
         if ((rc = d->alloc(&d->status, 1))) return rc;
@@ -513,8 +514,6 @@ int vtp_domain_create(const char *config_json, const float *fluid_pos, uint32_t 
                                                             d->status);
             CU(cudaGetLastError());
         }
-        // DFSPH: the boundary rows' packed gather rows ({x, V_b}, {x, v*}) never change: pack them once.
-        if (!pbf) vtp::dfsph_solve_pack(d->st, s->dfsph_args());
         CU(cudaGetLastError());
         CU(cudaStreamSynchronize(d->st));
         *out = d.release();
@@ -640,9 +639,7 @@ int vtp_domain_solve_begin(vtp_domain *d, int which) {
     d->which = which;
     vtp_solver *s = d->s;
     vtp::dfsph_solve_begin(d->st, s->solve + which, s->loop + which, 1);
-    vtp::DfsphArgs a = d->args();
-    a.nb = 0;   // the boundary rows were packed at create
-    vtp::dfsph_solve_pack(d->st, a);
+    vtp::dfsph_solve_pack(d->st, d->args());
     CU(cudaGetLastError());
     return VTP_OK;
 }

@@ -143,7 +143,8 @@ struct vtp_solver {
     float *vol = nullptr, *density = nullptr, *lambda = nullptr;
     float *ratio = nullptr, *alpha = nullptr, *kappa = nullptr, *delta = nullptr, *rest_b = nullptr;
     float4 *acc_tmp = nullptr, *normal = nullptr;
-    float4 *pva = nullptr, *pk = nullptr;   // packed gather rows of the pressure solve
+    float4 *pva = nullptr, *pk = nullptr;   // packed gather rows of the pressure solves
+    float4 *pva2 = nullptr;                 // DFSPH: the density solve's own pva (the forces pass fills it); else pva
     double *partials = nullptr, *inv_count = nullptr;
     uint16_t *obj_of = nullptr;
     vtp::SolveState *solve = nullptr;   // [2][S]: divergence, density per scene
@@ -245,7 +246,7 @@ struct vtp_solver {
     int tick_n(uint32_t n, const std::function<int()> &tail = nullptr);
     int enqueue_tick(cudaStream_t s, bool capture);
     int enqueue_pbf_substep(cudaStream_t s, const PbfTapeSlot *tape);
-    int enqueue_solve(cudaStream_t s, int which, bool capture);
+    int enqueue_solve(cudaStream_t s, int which, bool capture, bool packed = false);
     int build_graphs();
     int sort_boundary_and_lists();
     int get_field(int f, void *host, size_t bytes);
