@@ -5,7 +5,7 @@
 // shared memory; then the team's lanes add the terms up entry by entry in list order, each lane
 // its own accumulator.  The sums are the bits one thread walking the row gets, whatever L is; the
 // gathers and the pair arithmetic - the latency and most of the instructions - run L rows' worth
-// wide.  Used where a thread per row leaves most of the GPU idle and a pass takes one thread's
+// wide (the next batch's indices load while a batch is evaluated).  Used where a thread per row leaves most of the GPU idle and a pass takes one thread's
 // serial walk (kTeamMaxRows, internal.h, says where that ends).
 #pragma once
 
@@ -45,17 +45,24 @@ __device__ __forceinline__ void team_walk(TeamTerms<W> &S, const uint32_t *__res
     using T = decltype(load(0u));
     const uint32_t l = team_lane();
     float *const mine = S.t[threadIdx.x >> 5] + ((threadIdx.x & 31u) / kTeamLanes) * (kTeamPitch * W);
+    uint32_t nxt[kTeamDepth];
+#pragma unroll
+    for (uint32_t u = 0; u < kTeamDepth; ++u)
+        if (u * kTeamLanes + l < cnt) nxt[u] = __ldcs(lst + team_slot(u * kTeamLanes + l));
     for (uint32_t c0 = 0; __any_sync(0xffffffffu, c0 < cnt); c0 += kTeamBatch) {
         uint32_t j[kTeamDepth];
         T d[kTeamDepth];
 #pragma unroll
-        for (uint32_t u = 0; u < kTeamDepth; ++u) {
-            const uint32_t t = c0 + u * kTeamLanes + l;
-            if (t < cnt) j[u] = __ldcs(lst + team_slot(t));
-        }
+        for (uint32_t u = 0; u < kTeamDepth; ++u) j[u] = nxt[u];
 #pragma unroll
         for (uint32_t u = 0; u < kTeamDepth; ++u)
             if (c0 + u * kTeamLanes + l < cnt) d[u] = load(j[u]);
+        // the next batch's indices load while this batch is evaluated
+#pragma unroll
+        for (uint32_t u = 0; u < kTeamDepth; ++u) {
+            const uint32_t t = c0 + kTeamBatch + u * kTeamLanes + l;
+            if (t < cnt) nxt[u] = __ldcs(lst + team_slot(t));
+        }
 #pragma unroll
         for (uint32_t u = 0; u < kTeamDepth; ++u) {
             const uint32_t e = u * kTeamLanes + l;
