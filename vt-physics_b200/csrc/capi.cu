@@ -478,8 +478,10 @@ int vtp_solver::initialize() {
     }
     L.merge_mode = mode < 0 ? 0 : mode;
     L.cell_cull = cell_cull;
-    teams = L.nf <= vtp::kTeamMaxRows && !persistent_tiles &&
-            (type == VTP_SOLVER_DFSPH || type == VTP_SOLVER_PBF);
+    teams = persistent_tiles || (type != VTP_SOLVER_DFSPH && type != VTP_SOLVER_PBF) ? 0
+            : L.nf <= vtp::kTeam8MaxRows                                             ? 8
+            : L.nf <= vtp::kTeamMaxRows                                              ? 4
+                                                                                     : 0;
     L.shape.stride = vtp::list_stride(maxnbr > 1 ? maxnbr - 1 : 1);
     L.shape.lg = teams ? vtp::kTeamListLg : 0u;
 

@@ -170,10 +170,11 @@ __global__ void __launch_bounds__(256) k_ratio_alpha(DfsphArgs a) {
 }
 
 // The same with a team per row (team.cuh).
-__global__ void __launch_bounds__(kTeamBlock) k_team_ratio_alpha(DfsphArgs a) {
-    __shared__ TeamTerms<8> S;   // V_j, W, gradW, |gradW|^2 V_j^2 (fluid j)
+template <int L>
+__global__ void __launch_bounds__(kTeamRows * L) k_team_ratio_alpha(DfsphArgs a) {
+    __shared__ TeamTerms<8, L> S;   // V_j, W, gradW, |gradW|^2 V_j^2 (fluid j)
     start_solves(a);
-    const uint32_t r = blockIdx.x * kTeamRows + team_row(), l = team_lane();
+    const uint32_t r = blockIdx.x * kTeamRows + team_row<L>(), l = team_lane<L>();
     const bool live = r < a.nf && !halo_ghost(a, r);
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
     uint32_t n = 0;
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_ratio_alpha(DfsphArgs a) {
     const float inv_mf = __fdiv_rn(1.f, a.mass_f);
     // lane 0: ratio, lanes 1..3: a1; every lane: a2
     float acc = l == 0 && n > 0 ? __fmul_rn(p.w, a.k.w0) : 0.f, a2 = 1e-6f;
-    team_walk<8>(
+    team_walk<L, 8>(
         S, a.nbr + ell_index(r, 0, a.shape), n > 0 ? n - 1 : 0, [&](uint32_t j) { return ldg4(a.pos + j); },
         [&](uint32_t j, const float4 &q, float *o) {
             const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
@@ -200,14 +201,14 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_ratio_alpha(DfsphArgs a) {
             o[6] = o[7] = 0.f;
         },
         [&](const float *e) {
-            acc = __fmaf_rn(e[0], e[1 + l], acc);
+            acc = __fmaf_rn(e[0], e[1 + (l & 3)], acc);
             a2 = __fmaf_rn(e[5], inv_mf, a2);
         });
     RatioAlpha ra;
     ra.ratio = acc;
-    ra.a1x = team_get(acc, 1);
-    ra.a1y = team_get(acc, 2);
-    ra.a1z = team_get(acc, 3);
+    ra.a1x = team_get<L>(acc, 1);
+    ra.a1y = team_get<L>(acc, 2);
+    ra.a1z = team_get<L>(acc, 3);
     ra.a2 = a2;
     if (!live || l != 0) return;
     if (a.pack) pack_row(a, r, p, a.vadv[r]);
@@ -272,9 +273,9 @@ __global__ void __launch_bounds__(256) k_solve_a(DfsphArgs a) {
 
 // solve_a with a team per row: a block takes a 32-row piece of a tile (`pieces` per tile) and
 // leaves the sum of its rows' errors; k_solve_end adds a tile's pieces as the block sum above does.
-template <bool MULTI>
-__global__ void __launch_bounds__(kTeamBlock) k_team_solve_a(DfsphArgs a, uint32_t pieces) {
-    __shared__ TeamTerms<1> S;
+template <bool MULTI, int L>
+__global__ void __launch_bounds__(kTeamRows * L) k_team_solve_a(DfsphArgs a, uint32_t pieces) {
+    __shared__ TeamTerms<1, L> S;
     __shared__ float err[kTeamRows];
     const StepDt T = step_dt(a);
     const uint32_t t = blockIdx.x / pieces, part = blockIdx.x - t * pieces;
@@ -282,7 +283,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_solve_a(DfsphArgs a, uint32
     const bool stopped = a.state[tile.z].stopped != 0;
     if (a.tile_ran && part == 0 && threadIdx.x == 0) a.tile_ran[t] = stopped ? 0u : 1u;
     if (stopped) return;
-    const uint32_t row = part * kTeamRows + team_row(), r = tile.x + row;
+    const uint32_t row = part * kTeamRows + team_row<L>(), r = tile.x + row;
     const bool live = row < tile.y && !halo_ghost(a, r);
     float4 p = make_float4(0.f, 0.f, 0.f, 1.f), vi = p;
     float d = 0.f, al = 1.f;
@@ -294,13 +295,13 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_solve_a(DfsphArgs a, uint32
         al = a.alpha[r];
         d = a.ratio[r] - 1.f;
     }
-    team_walk<1>(
+    team_walk<L, 1>(
         S, a.nbr + ell_index(r, 0, a.shape), n > 0 ? n - 1 : 0,
         [&](uint32_t j) { return ldg8(a.pva + 2 * (size_t)j); },
         [&](uint32_t, const F4x2 &e, float *o) { o[0] = solve_a_term(p, vi, e, a.k); },
         [&](const float *e) { d = __fmaf_rn(e[0], T.dt, d); });
     if (d < 0.f) d = 0.f;
-    if (live && team_lane() == 0) {
+    if (live && team_lane<L>() == 0) {
         a.delta[r] = d;
         const float kap = d / al * T.inv_dt2 / p.w;
         a.kappa[r] = kap;
@@ -311,7 +312,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_solve_a(DfsphArgs a, uint32
             P.pk[q] = pkr;
         });
     }
-    if (team_lane() == 0) err[team_row()] = live ? d : 0.f;
+    if (team_lane<L>() == 0) err[team_row<L>()] = live ? d : 0.f;
     __syncthreads();
     if (threadIdx.x >= 32) return;
     const double contrib = (double)err[threadIdx.x];
@@ -538,13 +539,14 @@ __global__ void __launch_bounds__(256) k_solve_b(DfsphArgs a) {
 }
 
 // solve_b with a team per row: lanes 0..2 carry a velocity component each.
-__global__ void __launch_bounds__(kTeamBlock) k_team_solve_b(DfsphArgs a, uint32_t pieces) {
-    __shared__ TeamTerms<4> S;   // -s, x_i - x_j
+template <int L>
+__global__ void __launch_bounds__(kTeamRows * L) k_team_solve_b(DfsphArgs a, uint32_t pieces) {
+    __shared__ TeamTerms<4, L> S;   // -s, x_i - x_j
     const StepDt T = step_dt(a);
-    const uint32_t t = blockIdx.x / pieces, part = blockIdx.x - t * pieces, l = team_lane();
+    const uint32_t t = blockIdx.x / pieces, part = blockIdx.x - t * pieces, l = team_lane<L>();
     const uint4 tile = a.tiles[t];
     if (a.tile_ran ? a.tile_ran[t] == 0u : (a.state && a.state[tile.z].stopped)) return;
-    const uint32_t row = part * kTeamRows + team_row(), r = tile.x + row;
+    const uint32_t row = part * kTeamRows + team_row<L>(), r = tile.x + row;
     const bool live = row < tile.y && !halo_ghost(a, r);
     float4 p = make_float4(0.f, 0.f, 0.f, 1.f);
     float ki = 0.f, ci = 0.f, v = 0.f;
@@ -553,13 +555,13 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_solve_b(DfsphArgs a, uint32
         p = a.pos[r];
         ki = a.kappa[r];
         n = a.ncnt[r];
-        v = reinterpret_cast<const float *>(a.vadv + r)[l];
+        v = reinterpret_cast<const float *>(a.vadv + r)[l & 3];
         const float mi = a.rest_density ? a.rest_density[r] * p.w : a.mass_f;
         ci = T.dt * p.w / mi;   // dt V_i / m_i
     }
     const float w = v;   // lane 3: the fourth word, kept
     const uint32_t c = l < 3 ? 1 + l : 1;
-    team_walk<4>(
+    team_walk<L, 4>(
         S, a.nbr + ell_index(r, 0, a.shape), n > 0 ? n - 1 : 0, [&](uint32_t j) { return ldg4(a.pk + j); },
         [&](uint32_t j, const float4 &e, float *o) {
             o[1] = p.x - e.x;
@@ -569,12 +571,12 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_solve_b(DfsphArgs a, uint32
         },
         [&](const float *e) { v = __fmaf_rn(e[0], e[c], v); });
     if (l == 3) v = w;
-    if (live) {
+    if (live && l < 4) {
         reinterpret_cast<float *>(a.vadv + r)[l] = v;
         reinterpret_cast<float *>(a.pva + 2 * (size_t)r + 1)[l] = v;
     }
     if (a.halo) {
-        const float4 o = make_float4(team_get(v, 0), team_get(v, 1), team_get(v, 2), team_get(v, 3));
+        const float4 o = make_float4(team_get<L>(v, 0), team_get<L>(v, 1), team_get<L>(v, 2), team_get<L>(v, 3));
         if (live && l == 0)
             halo_each(a, r, [&](const PeerRows &P, uint32_t q) {
                 P.vadv[a.halo_vadv][q] = o;
@@ -851,12 +853,12 @@ __global__ void __launch_bounds__(256) k_tension(DfsphArgs a) {
 }
 
 // The viscosity and tension passes with a team per row.
-template <bool TENSION_SPLIT>
-__global__ void __launch_bounds__(kTeamBlock) k_team_viscosity(DfsphArgs a) {
+template <bool TENSION_SPLIT, int L>
+__global__ void __launch_bounds__(kTeamRows * L) k_team_viscosity(DfsphArgs a) {
     constexpr int W = TENSION_SPLIT ? 8 : 4;
-    __shared__ TeamTerms<W> S;   // viscosity factor, x_i - x_j, normal factor
+    __shared__ TeamTerms<W, L> S;   // viscosity factor, x_i - x_j, normal factor
     const StepDt T = step_dt(a);
-    const uint32_t r = blockIdx.x * kTeamRows + team_row(), l = team_lane();
+    const uint32_t r = blockIdx.x * kTeamRows + team_row<L>(), l = team_lane<L>();
     const bool live = r < a.nf && !halo_ghost(a, r);
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f), vi = p;
     uint32_t n = 0;
@@ -868,7 +870,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_viscosity(DfsphArgs a) {
     const float ncoef = a.k.h * a.mass_f / a.rho0;   // h m_j / rho_rest_j (fluid)
     float acc = 0.f, nrm = 0.f;
     const uint32_t c = l < 3 ? 1 + l : 1;
-    team_walk<W>(
+    team_walk<L, W>(
         S, a.nbr + ell_index(r, 0, a.shape), n > 0 ? n - 1 : 0,
         [&](uint32_t j) {
             if (j >= a.nf) return F4x2{};   // same-material neighbours only
@@ -895,16 +897,17 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_viscosity(DfsphArgs a) {
             acc = __fmaf_rn(e[0], e[c], acc);
             if constexpr (TENSION_SPLIT) nrm = __fmaf_rn(e[4], e[c], nrm);
         });
-    const float ax = team_get(acc, 0), ay = team_get(acc, 1), az = team_get(acc, 2);
-    const float nx = team_get(nrm, 0), ny = team_get(nrm, 1), nz = team_get(nrm, 2);
+    const float ax = team_get<L>(acc, 0), ay = team_get<L>(acc, 1), az = team_get<L>(acc, 2);
+    const float nx = team_get<L>(nrm, 0), ny = team_get<L>(nrm, 1), nz = team_get<L>(nrm, 2);
     if (!live || l != 0) return;
     finish_viscosity<TENSION_SPLIT>(a, T, r, vi, ax, ay, az, nx, ny, nz);
 }
 
-__global__ void __launch_bounds__(kTeamBlock) k_team_tension(DfsphArgs a) {
-    __shared__ TeamTerms<4> S;
+template <int L>
+__global__ void __launch_bounds__(kTeamRows * L) k_team_tension(DfsphArgs a) {
+    __shared__ TeamTerms<4, L> S;
     const StepDt T = step_dt(a);
-    const uint32_t r = blockIdx.x * kTeamRows + team_row(), l = team_lane();
+    const uint32_t r = blockIdx.x * kTeamRows + team_row<L>(), l = team_lane<L>();
     const bool live = r < a.nf && !halo_ghost(a, r);
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f), ni = p;
     uint32_t n = 0;
@@ -915,7 +918,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_tension(DfsphArgs a) {
     }
     const float kk = 2.f * a.rho0 / (a.rho0 + a.rho0);
     float acc = 0.f;
-    team_walk<4>(
+    team_walk<L, 4>(
         S, a.nbr + ell_index(r, 0, a.shape), n > 0 ? n - 1 : 0,
         [&](uint32_t j) {
             if (j >= a.nf) return PN{};
@@ -925,8 +928,8 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_tension(DfsphArgs a) {
             o[0] = o[1] = o[2] = o[3] = 0.f;
             if (j < a.nf) tension_term(a, p, ni, e, o[0], o[1], o[2]);
         },
-        [&](const float *e) { acc += kk * e[l]; });
-    const float tx = team_get(acc, 0), ty = team_get(acc, 1), tz = team_get(acc, 2);
+        [&](const float *e) { acc += kk * e[l & 3]; });
+    const float tx = team_get<L>(acc, 0), ty = team_get<L>(acc, 1), tz = team_get<L>(acc, 2);
     if (live && l == 0) finish_tension(a, T, r, tx, ty, tz);
 }
 
@@ -1006,6 +1009,11 @@ void dfsph_rigid_volume(cudaStream_t st, const DfsphArgs &a, const uint32_t *bnc
                         float *rest_density_b) {
     if (a.nb) k_rigid_volume<<<nblk(a.nb, 256), 256, 0, st>>>(a, bncnt, bnbr, rest_density_b);
 }
+#define VTP_TEAM_DISPATCH(L, ...)                \
+    {                                            \
+        if ((L) == 8) { constexpr int LL = 8; __VA_ARGS__ } \
+        else { constexpr int LL = 4; __VA_ARGS__ }          \
+    }
 #define VTP_UNROLL_DISPATCH(U, ...)          \
     switch (U) {                                 \
         case 1: { constexpr int UU = 1; __VA_ARGS__; } break; \
@@ -1016,7 +1024,7 @@ void dfsph_rigid_volume(cudaStream_t st, const DfsphArgs &a, const uint32_t *bnc
 
 void dfsph_ratio_alpha(cudaStream_t st, const DfsphArgs &a, int block) {
     if (!a.nf) return;
-    if (a.teams) k_team_ratio_alpha<<<nblk(a.nf, kTeamRows), kTeamBlock, 0, st>>>(a);
+    if (a.teams) VTP_TEAM_DISPATCH(a.teams, k_team_ratio_alpha<LL><<<nblk(a.nf, kTeamRows), kTeamRows * LL, 0, st>>>(a);)
     else VTP_UNROLL_DISPATCH(a.unroll, k_ratio_alpha<UU><<<nblk(a.nf, block), block, 0, st>>>(a))
 }
 void dfsph_solve_begin(cudaStream_t st, SolveState *s, LoopState *loop, int nscenes) {
@@ -1045,8 +1053,8 @@ void dfsph_solve_a(cudaStream_t st, const DfsphArgs &a, int block) {
     if (a.teams) {
         const uint32_t pieces = solve_pieces(block), n = a.ntiles * pieces;
         if (!n) return;
-        if (a.nobj_max > 1) k_team_solve_a<true><<<n, kTeamBlock, 0, st>>>(a, pieces);
-        else k_team_solve_a<false><<<n, kTeamBlock, 0, st>>>(a, pieces);
+        if (a.nobj_max > 1) VTP_TEAM_DISPATCH(a.teams, k_team_solve_a<true, LL><<<n, kTeamRows * LL, 0, st>>>(a, pieces);)
+        else VTP_TEAM_DISPATCH(a.teams, k_team_solve_a<false, LL><<<n, kTeamRows * LL, 0, st>>>(a, pieces);)
         return;
     }
     const unsigned nb = dfsph_tile_grid(a.ntiles, block, a.persistent);
@@ -1060,7 +1068,7 @@ void dfsph_solve_b(cudaStream_t st, const DfsphArgs &a, int block) {
     }
     if (a.teams) {
         const uint32_t pieces = solve_pieces(block), n = a.ntiles * pieces;
-        if (n) k_team_solve_b<<<n, kTeamBlock, 0, st>>>(a, pieces);
+        if (n) VTP_TEAM_DISPATCH(a.teams, k_team_solve_b<LL><<<n, kTeamRows * LL, 0, st>>>(a, pieces);)
         return;
     }
     const unsigned nb = dfsph_tile_grid(a.ntiles, block, a.persistent);
@@ -1085,17 +1093,17 @@ void dfsph_pressure_pack(cudaStream_t st, const DfsphArgs &a) {
 }
 void dfsph_viscosity(cudaStream_t st, const DfsphArgs &a, int block) {
     if (!a.nf) return;
-    if (a.teams) k_team_viscosity<false><<<nblk(a.nf, kTeamRows), kTeamBlock, 0, st>>>(a);
+    if (a.teams) VTP_TEAM_DISPATCH(a.teams, k_team_viscosity<false, LL><<<nblk(a.nf, kTeamRows), kTeamRows * LL, 0, st>>>(a);)
     else VTP_UNROLL_DISPATCH(a.unroll, k_viscosity<false, UU><<<nblk(a.nf, block), block, 0, st>>>(a))
 }
 void dfsph_vis_normal(cudaStream_t st, const DfsphArgs &a, int block) {
     if (!a.nf) return;
-    if (a.teams) k_team_viscosity<true><<<nblk(a.nf, kTeamRows), kTeamBlock, 0, st>>>(a);
+    if (a.teams) VTP_TEAM_DISPATCH(a.teams, k_team_viscosity<true, LL><<<nblk(a.nf, kTeamRows), kTeamRows * LL, 0, st>>>(a);)
     else VTP_UNROLL_DISPATCH(a.unroll, k_viscosity<true, UU><<<nblk(a.nf, block), block, 0, st>>>(a))
 }
 void dfsph_tension(cudaStream_t st, const DfsphArgs &a, int block) {
     if (!a.nf) return;
-    if (a.teams) k_team_tension<<<nblk(a.nf, kTeamRows), kTeamBlock, 0, st>>>(a);
+    if (a.teams) VTP_TEAM_DISPATCH(a.teams, k_team_tension<LL><<<nblk(a.nf, kTeamRows), kTeamRows * LL, 0, st>>>(a);)
     else VTP_UNROLL_DISPATCH(a.unroll, k_tension<UU><<<nblk(a.nf, block), block, 0, st>>>(a))
 }
 void dfsph_finalize(cudaStream_t st, const DfsphArgs &a) {

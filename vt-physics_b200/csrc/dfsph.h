@@ -81,7 +81,7 @@ struct DfsphArgs {
     // its neighbours from a shared-memory copy of the group's neighbourhood through the slot
     // lists; the residual partials are then per group (ngroups + 1 entries, the last for the
     // rows outside the grid).
-    bool teams;                 // neighbour passes walk a row with a team of lanes (team.cuh)
+    int teams;                  // lanes of the team that walks a row (team.cuh); 0: a thread per row
     int staged;
     Staging stg;
     const float *dtp;           // adaptive time step (CFL) on the device; null: the fixed dt above

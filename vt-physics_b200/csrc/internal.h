@@ -23,9 +23,9 @@ struct NvtxRange {
     NvtxRange &operator=(const NvtxRange &) = delete;
 };
 
-// Solvers of up to this many fluid rows walk a row with a team of four lanes (team.cuh), larger
+// Solvers of up to this many fluid rows walk a row with a team of lanes (team.cuh), larger
 // ones with a thread per row; the bits are the same.  Event-timed launches (B200, about 5 us of
-// which is the events), thread per row -> team, us: DFSPH solve_a / solve_b / ratio + alpha /
+// which is the events), thread per row -> team of four, us: DFSPH solve_a / solve_b / ratio + alpha /
 // viscosity at 2,000 rows 13.3 / 11.6 / 16.4 / 13.4 -> 9.9 / 8.5 / 9.4 / 10.4, at 32,000 rows
 // 14.5 / 12.6 / 18.7 / 14.8 -> 13.2 / 10.6 / 13.1 / 12.4, at 64,000 rows 16.4 / 14.4 / 18.8 / 16.6
 // -> 18.3 / 15.1 / 20.8 / 19.0; PBF lambda / dx / XSPH at 2,000 rows 16.9 / 12.4 / 14.6 -> 10.5 /
@@ -33,6 +33,12 @@ struct NvtxRange {
 // / 18.8 -> 20.7 / 16.7 / 18.8.  A team executes 1.6 times the instructions of the thread, so past
 // the row count that fills the GPU the thread wins (1,000,000 rows: solve_a 113 -> 168).
 constexpr uint32_t kTeamMaxRows = 49152;
+// Of them, up to this many rows take eight lanes, so that a row of 32 neighbours is one batch.  Four ->
+// eight lanes, us: PBF lambda / dx / XSPH at 2,000 rows 10.6 / 10.3 / 8.5 -> 8.4 / 8.4 / 8.4, at
+// 16,000 rows 12.3 / 10.5 / 10.6 -> 10.6 / 10.5 / 10.5, at 32,000 rows 14.6 / 12.6 / 12.6 -> 14.6 /
+// 14.2 / 14.6; DFSPH solve_a / ratio + alpha at 2,000 rows 9.9 / 10.5 -> 9.4 / 8.5, at 16,000 rows
+// 11.4 / 12.5 -> 11.8 / 10.6, at 32,000 rows 13.4 / 14.7 -> 15.0 / 14.6.
+constexpr uint32_t kTeam8MaxRows = 16384;
 
 constexpr int kConsPhases = 8;   // phases the conservation sums report (vtp_conservation.phase_mass)
 

@@ -239,10 +239,11 @@ __global__ void __launch_bounds__(256) k_pbf_xsph(PbfArgs a) {
 }
 
 // The passes with a team per row (team.cuh).
-__global__ void __launch_bounds__(kTeamBlock) k_team_pbf_lambda(PbfArgs a) {
+template <int L>
+__global__ void __launch_bounds__(kTeamRows * L) k_team_pbf_lambda(PbfArgs a) {
     pdl_enter();
-    __shared__ TeamTerms<8> S;   // m_j, W, gradW, |gradW / rho0|^2
-    const uint32_t r = blockIdx.x * kTeamRows + team_row(), l = team_lane();
+    __shared__ TeamTerms<8, L> S;   // m_j, W, gradW, |gradW / rho0|^2
+    const uint32_t r = blockIdx.x * kTeamRows + team_row<L>(), l = team_lane<L>();
     const bool live = r < a.nf && !halo_ghost(a, r);
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
     uint32_t n = 0;
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_pbf_lambda(PbfArgs a) {
     }
     // lane 0: density (self first: m_i W(0)), lanes 1..3: sum of gradients; every lane: s2
     float acc = n > 0 && l == 0 ? p.w * pbf_w0(a) : 0.f, s2 = 0.f;
-    team_walk<8>(
+    team_walk<L, 8>(
         S, a.nbr + ell_index(r, 0, a.shape), n > 0 ? n - 1 : 0, [&](uint32_t j) { return ldg4(a.pos + j); },
         [&](uint32_t, const float4 &q, float *o) {
             const LambdaPair t = lambda_pair(a, p, q);
@@ -268,17 +269,18 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_pbf_lambda(PbfArgs a) {
             o[7] = 0.f;
         },
         [&](const float *e) {
-            acc = __fmaf_rn(e[l == 0 ? 0 : 6], e[1 + l], acc);
+            acc = __fmaf_rn(e[(l & 3) == 0 ? 0 : 6], e[1 + (l & 3)], acc);
             s2 = __fadd_rn(s2, e[5]);
         });
-    const float gx = team_get(acc, 1), gy = team_get(acc, 2), gz = team_get(acc, 3);
+    const float gx = team_get<L>(acc, 1), gy = team_get<L>(acc, 2), gz = team_get<L>(acc, 3);
     if (live && l == 0) finish_lambda(a, r, acc, gx, gy, gz, s2);
 }
 
-__global__ void __launch_bounds__(kTeamBlock) k_team_pbf_dx(PbfArgs a) {
+template <int L>
+__global__ void __launch_bounds__(kTeamRows * L) k_team_pbf_dx(PbfArgs a) {
     pdl_enter();
-    __shared__ TeamTerms<4> S;   // factor, x_i - x_j
-    const uint32_t r = blockIdx.x * kTeamRows + team_row(), l = team_lane();
+    __shared__ TeamTerms<4, L> S;   // factor, x_i - x_j
+    const uint32_t r = blockIdx.x * kTeamRows + team_row<L>(), l = team_lane<L>();
     const bool live = r < a.nf && !halo_ghost(a, r);
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
     float li = 0.f;
@@ -291,7 +293,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_pbf_dx(PbfArgs a) {
     float acc = 0.f;
     const uint32_t c = l < 3 ? 1 + l : 1;
     // Boundary lambda is never written by the reference; it is taken as 0.
-    team_walk<4>(
+    team_walk<L, 4>(
         S, a.nbr + ell_index(r, 0, a.shape), n > 0 ? n - 1 : 0,
         [&](uint32_t j) { return PL{ldg4(a.pos + j), j < a.nf ? __ldg(a.lambda + j) : 0.f}; },
         [&](uint32_t, const PL &e, float *o) {
@@ -301,14 +303,15 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_pbf_dx(PbfArgs a) {
             o[0] = dx_factor(a, dist2(o[1], o[2], o[3]), p.w, e.q.w, li, e.l);
         },
         [&](const float *e) { acc = __fmaf_rn(e[0], e[c], acc); });
-    const float dx = team_get(acc, 0), dy = team_get(acc, 1), dz = team_get(acc, 2);
+    const float dx = team_get<L>(acc, 0), dy = team_get<L>(acc, 1), dz = team_get<L>(acc, 2);
     if (live && l == 0) finish_dx(a, r, p, dx, dy, dz);
 }
 
-__global__ void __launch_bounds__(kTeamBlock) k_team_pbf_xsph(PbfArgs a) {
+template <int L>
+__global__ void __launch_bounds__(kTeamRows * L) k_team_pbf_xsph(PbfArgs a) {
     pdl_enter();
-    __shared__ TeamTerms<4> S;   // W, k V_j (v_j - v_i)
-    const uint32_t r = blockIdx.x * kTeamRows + team_row(), l = team_lane();
+    __shared__ TeamTerms<4, L> S;   // W, k V_j (v_j - v_i)
+    const uint32_t r = blockIdx.x * kTeamRows + team_row<L>(), l = team_lane<L>();
     const bool live = r < a.nf && !halo_ghost(a, r);
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f), vi = p;
     uint32_t n = 0;
@@ -319,7 +322,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_pbf_xsph(PbfArgs a) {
     }
     float acc = 0.f;
     const uint32_t c = l < 3 ? 1 + l : 1;
-    team_walk<4>(
+    team_walk<L, 4>(
         S, a.nbr + ell_index(r, 0, a.shape), n > 0 ? n - 1 : 0,
         [&](uint32_t j) { return PV2{ldg4(a.pos + j), ldg4(a.vel + j), __ldg(a.vol + j)}; },
         [&](uint32_t, const PV2 &e, float *o) {
@@ -330,7 +333,7 @@ __global__ void __launch_bounds__(kTeamBlock) k_team_pbf_xsph(PbfArgs a) {
             o[3] = k * (e.v.z - vi.z);
         },
         [&](const float *e) { acc = __fmaf_rn(e[c], e[0], acc); });
-    const float ax = team_get(acc, 0), ay = team_get(acc, 1), az = team_get(acc, 2);
+    const float ax = team_get<L>(acc, 0), ay = team_get<L>(acc, 1), az = team_get<L>(acc, 2);
     if (live && l == 0) finish_xsph(a, r, p, vi, ax, ay, az);
 }
 
@@ -358,22 +361,28 @@ void pbf_init_boundary(cudaStream_t st, const PbfArgs &a, const uint32_t *bncnt,
 
 void pbf_lambda(cudaStream_t st, const PbfArgs &a, int block) {
     if (!a.nf) return;
-    if (a.teams && a.lanes == 1)
-        launch(k_team_pbf_lambda, nblk(a.nf, kTeamRows), kTeamBlock, 0, st, a);
+    if (a.teams == 8 && a.lanes == 1)
+        launch(k_team_pbf_lambda<8>, nblk(a.nf, kTeamRows), kTeamRows * 8, 0, st, a);
+    else if (a.teams && a.lanes == 1)
+        launch(k_team_pbf_lambda<4>, nblk(a.nf, kTeamRows), kTeamRows * 4, 0, st, a);
     else
         VTP_LANES_DISPATCH(a.lanes, VTP_UNROLL_DISPATCH(a.unroll, launch(k_pbf_lambda<UU, LL>, nblk(a.nf * LL, block), block, 0, st, a)))
 }
 void pbf_dx(cudaStream_t st, const PbfArgs &a, int block) {
     if (!a.nf) return;
-    if (a.teams && a.lanes == 1)
-        launch(k_team_pbf_dx, nblk(a.nf, kTeamRows), kTeamBlock, 0, st, a);
+    if (a.teams == 8 && a.lanes == 1)
+        launch(k_team_pbf_dx<8>, nblk(a.nf, kTeamRows), kTeamRows * 8, 0, st, a);
+    else if (a.teams && a.lanes == 1)
+        launch(k_team_pbf_dx<4>, nblk(a.nf, kTeamRows), kTeamRows * 4, 0, st, a);
     else
         VTP_LANES_DISPATCH(a.lanes, VTP_UNROLL_DISPATCH(a.unroll, launch(k_pbf_dx<UU, LL>, nblk(a.nf * LL, block), block, 0, st, a)))
 }
 void pbf_xsph(cudaStream_t st, const PbfArgs &a, int block) {
     if (!a.nf) return;
-    if (a.teams && a.lanes == 1)
-        launch(k_team_pbf_xsph, nblk(a.nf, kTeamRows), kTeamBlock, 0, st, a);
+    if (a.teams == 8 && a.lanes == 1)
+        launch(k_team_pbf_xsph<8>, nblk(a.nf, kTeamRows), kTeamRows * 8, 0, st, a);
+    else if (a.teams && a.lanes == 1)
+        launch(k_team_pbf_xsph<4>, nblk(a.nf, kTeamRows), kTeamRows * 4, 0, st, a);
     else
         VTP_LANES_DISPATCH(a.lanes, VTP_UNROLL_DISPATCH(a.unroll, launch(k_pbf_xsph<UU, LL>, nblk(a.nf * LL, block), block, 0, st, a)))
 }

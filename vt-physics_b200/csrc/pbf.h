@@ -9,7 +9,7 @@ namespace vtp {
 struct PbfArgs {
     uint32_t nf, nb;
     ListShape shape;
-    bool teams;                 // one lane per row configured: walk it with a team of lanes (team.cuh)
+    int teams;                  // lanes of the team that walks a row (team.cuh) where "rowLanes" is 1; 0: a thread
     Cubic k;
     float rho0, inv_rho0, rho_b, eps, dt, xsph_k;
     int form;              // 0: the reference's formulation; 1: standard PBF (poly6 / spiky, mass-weighted)

@@ -107,7 +107,7 @@ struct vtp_solver {
     bool cell_order_brick = true;   // bucket order: bricked (4^3 cells, Morton inside) or linear
     bool pdl = true;                // programmatic dependent launch between the substep's kernels
     int row_lanes = 1;        // threads per row of the PBF neighbour passes (1, 4, 8)
-    bool teams = false;       // neighbour passes walk a row with a team of lanes (team.cuh), by row count
+    int teams = 0;            // lanes of the team that walks a row (team.cuh), by row count; 0: a thread per row
     bool cell_cull = false;   // list builder skips neighbour cells beyond h (same lists)
     bool staged_solve = false;      // DFSPH pressure solve gathers from shared-memory cell-group copies
     uint32_t tape_budget_mb = 8192;  // differentiable PBF / DFSPH: device memory for resident segment tapes

@@ -659,6 +659,65 @@ __global__ void __launch_bounds__(kCellWarps * 32, 7) k_build_lists(
     }
 }
 
+// List builder for few rows: a warp takes four consecutive rows, whatever cells they lie in, eight
+// lanes each.  The candidates of a cell are laid out by every warp that has rows of it, but no warp
+// works through more than its own rows, and there are twice as many warps: the kernel's time is
+// then one short chain.  Event-timed (B200, us), a warp per cell -> this: DFSPH 2,000 rows 17.0 ->
+// 14.7, 8,000 rows 20.5 -> 16.7, 16,000 rows 20.6 -> 17.2, 32,000 rows 22.9 -> 28.8; PBF 8,000 rows
+// 12.3 -> 11.2, 16,000 rows 13.4 -> 13.5.
+constexpr uint32_t kFewRows = 16384;
+constexpr uint32_t kFewScan = 4;
+template <int MODE>
+__global__ void __launch_bounds__(kCellWarps * 32, 7) k_build_lists_few(
+    Scenes sc, uint32_t row0, uint32_t cnt, ListShape shape, const float4 *__restrict__ pos,
+    const uint32_t *__restrict__ orig, const uint32_t *__restrict__ fstart, const uint32_t *__restrict__ bstart,
+    uint32_t *__restrict__ nbr, uint32_t *__restrict__ ncnt, uint32_t *__restrict__ status,
+    uint32_t *__restrict__ overflow_count) {
+    pdl_enter();
+    __shared__ __align__(16) CellScratch scratch[kCellWarps];
+    constexpr unsigned kAll = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t first = (blockIdx.x * kCellWarps + (threadIdx.x >> 5)) * kFewScan;
+    if (first >= cnt) return;
+    CellScratch &S = scratch[threadIdx.x >> 5];
+    const int3 o = nbr_offset((int)min(lane, 26u));
+    const uint32_t n = min(kFewScan, cnt - first), k = lane % kFewScan;
+    const uint32_t row = row0 + first + min(k, n - 1u);
+    const SceneGrid mine_g = load_scene(sc, row);
+    const float4 p = pos[row];
+    const int3 c = cell_of(p.x, p.y, p.z, mine_g, sc.cell);
+    const bool inside = cell_available(c, mine_g);
+    if (lane < n && !inside) ncnt[first + lane] = 0;   // outside the grid: no neighbours, not even self
+    // one round per cell among the rows
+    for (unsigned left = __ballot_sync(kAll, lane < n && inside); left;) {
+        const int f = __ffs((int)left) - 1;
+        const int3 c0 = make_int3(__shfl_sync(kAll, c.x, f), __shfl_sync(kAll, c.y, f), __shfl_sync(kAll, c.z, f));
+        const uint32_t scene = __shfl_sync(kAll, mine_g.key_base, f);
+        const bool mine = ((left >> k) & 1u) && c.x == c0.x && c.y == c0.y && c.z == c0.z && mine_g.key_base == scene;
+        left &= ~__ballot_sync(kAll, mine);
+        const SceneGrid g = load_scene(sc, row0 + first + (uint32_t)f);
+        CellRuns runs{};
+        const int3 cc = make_int3(c0.x + o.x, c0.y + o.y, c0.z + o.z);
+        if (lane < 27u && cell_available(cc, g)) {
+            const uint32_t b = g.key_base + cell_key(cc, g);
+            runs.f0 = __ldg(fstart + b); runs.f1 = __ldg(fstart + b + 1);
+            runs.b0 = __ldg(bstart + b); runs.b1 = __ldg(bstart + b + 1);
+        }
+        const uint32_t len = (runs.f1 - runs.f0) + (runs.b1 - runs.b0);
+        uint32_t incl = len;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(kAll, incl, d);
+            if ((int)lane >= d) incl += y;
+        }
+        runs.excl = incl - len;
+        const uint32_t total = __shfl_sync(kAll, incl, 31);
+        cell_lists<MODE, kFewScan>(S, runs, total, mine, row, row0, p, sc.d2max, sc.maxnbr - 1u, shape, pos, orig, nbr,
+                                   ncnt, status, overflow_count);
+        __syncwarp();
+    }
+}
+
 #ifdef VTP_CHECKED
 // Checked build (-DVTP_CHECKED): every list entry of rows [row0, row0 + cnt)
 // after each build - count <= maxNbr, entries inside the solver's rows, no
@@ -1114,6 +1173,16 @@ void ugns_build_lists(cudaStream_t st, const Scenes &sc, const Layout &L, uint32
             case 0: L.cell_cull ? walk(M0{}, T) : walk(M0{}, F); break;
             case 1: L.cell_cull ? walk(M1{}, T) : walk(M1{}, F); break;
             default: L.cell_cull ? walk(M2{}, T) : walk(M2{}, F); break;
+        }
+    } else if (cnt <= kFewRows) {
+        auto few = [&](auto mode) {
+            launch(k_build_lists_few<decltype(mode)::value>, nblk(cnt, kCellWarps * kFewScan), kCellWarps * 32, 0, st,
+                   sc, row0, cnt, L.shape, pos, orig, u.fstart, u.bstart, nbr, ncnt, status, overflow);
+        };
+        switch (L.merge_mode) {
+            case 0: few(M0{}); break;
+            case 1: few(M1{}); break;
+            default: few(M2{}); break;
         }
     } else {
         auto cells = [&](auto mode) {
