@@ -219,35 +219,46 @@ __device__ __forceinline__ float cube_rn(float t) {
 // from it.  Density-ratio sums feed `ratio - 1`, where FP32 rounding is
 // amplified ~1e3 times in the pressure solve, so W follows the reference's
 // arithmetic; gradients use the faster form below.
+// Both sides of q = 1/2 are evaluated and one is selected: a warp's pairs fall on both, and the
+// divergent branch cost more than either side (1M rows, ratio pass 109 -> 105 us; 250k rows, PBF
+// lambda 36.3 -> 35.3).
 __device__ __forceinline__ float cubic_w(float d2, const Cubic &k) {
     const float r = sqrtf(d2);
     const float q = r * k.invh;
-    if (q > 1.f) return 0.f;
-    if (q <= 0.5f) {
-        const float q2 = q * q;
-        const float q3 = q2 * q;
-        return static_cast<float>((double)k.sigma * (6.0 * (double)q3 - 6.0 * (double)q2 + 1.0));
-    }
+    const float q2 = q * q;
+    const float q3 = q2 * q;
+    const float inner = static_cast<float>((double)k.sigma * (6.0 * (double)q3 - 6.0 * (double)q2 + 1.0));
     const float t = 1.f - q;
-    return k.sigma * 2.f * (k.cube_powf ? powf(t, 3.f) : cube_rn(t));
+    const float outer = k.sigma * 2.f * (k.cube_powf ? powf(t, 3.f) : cube_rn(t));
+    return q > 1.f ? 0.f : q <= 0.5f ? inner : outer;
+}
+
+// The hardware's approximate 1 / sqrt, without the scaling that a denormal x would need: 0 and
+// denormals give infinity.
+__device__ __forceinline__ float rsqrt_normal(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
 
 // Scalar g with gradW(r_vec) = g * r_vec; zero for q < 1e-6 or q > 1.
 // Every rounding is explicit, so g is the same bits in every kernel that
-// evaluates it, whatever the compiler contracts around the call.
+// evaluates it, whatever the compiler contracts around the call.  Without a
+// branch: the two sides of q = 1/2 share their last product, and a d2 below the
+// normal range ends in a q of infinity, outside the range.  The passes that evaluate it
+// for every pair are bound by issue: 1M rows, DFSPH ratio pass 119 -> 109 us and
+// viscosity 117 -> 107; 250k rows, PBF lambda 38.9 -> 36.3; 500k rows of a
+// mixture, viscosity and normals 126 -> 117 and precompute 82 -> 76.
 __device__ __forceinline__ float cubic_g(float d2, const Cubic &k) {
-    if (!(d2 > 0.f)) return 0.f;   // coincident particles: q < 1e-6 -> 0
-    const float rinv = rsqrtf(d2);
+    const float rinv = rsqrt_normal(d2);
     const float r = __fmul_rn(d2, rinv);
     const float q = __fmul_rn(r, k.invh);
-    if (q < 1e-6f || q > 1.f) return 0.f;
-    float f;
-    if (q <= 0.5f) f = __fmul_rn(__fmul_rn(6.f, q), __fmaf_rn(3.f, q, -2.f));
-    else {
-        const float t = __fsub_rn(1.f, q);
-        f = __fmul_rn(__fmul_rn(-6.f, t), t);
-    }
-    return __fmul_rn(__fmul_rn(f, k.sigma), __fmul_rn(rinv, k.invh));
+    const float t = __fsub_rn(1.f, q);
+    const bool inner = q <= 0.5f;
+    const float a = inner ? __fmul_rn(6.f, q) : __fmul_rn(-6.f, t);
+    const float b = inner ? __fmaf_rn(3.f, q, -2.f) : t;
+    const float g = __fmul_rn(__fmul_rn(__fmul_rn(a, b), k.sigma), __fmul_rn(rinv, k.invh));
+    return !(d2 > 0.f) || q < 1e-6f || q > 1.f ? 0.f : g;
 }
 
 // W and g together.
