@@ -271,17 +271,13 @@ __device__ __forceinline__ void cubic_wg(float d2, const Cubic &k, float &w, flo
 // kernel evaluates it (KernelFunctions.cuh:16-17).
 __global__ void k_cubic_sigma(float h, float *out);
 
-// Akinci cohesion spline sph::surface_tension_C (KernelFunctions.cuh:59-70).
+// Akinci cohesion spline sph::surface_tension_C (KernelFunctions.cuh:59-70), both sides of h / 2
+// evaluated and one selected as in cubic_w.
 __device__ __forceinline__ float tension_c(float r, float h, float csigma, float h6_64) {
-    if (r * 2.f > h && r <= h) {
-        float a = h - r;
-        return csigma * (a * a * a) * (r * r * r);
-    }
-    if (r > 0.f && r * 2.f <= h) {
-        float a = h - r;
-        return csigma * (2.f * (a * a * a) * (r * r * r) - h6_64);
-    }
-    return 0.f;
+    const float a = h - r;
+    const float far = csigma * (a * a * a) * (r * r * r);
+    const float near = csigma * (2.f * (a * a * a) * (r * r * r) - h6_64);
+    return r * 2.f > h ? (r <= h ? far : 0.f) : r > 0.f && r * 2.f <= h ? near : 0.f;
 }
 
 __device__ __forceinline__ float4 ldg4(const float4 *p) { return __ldg(p); }

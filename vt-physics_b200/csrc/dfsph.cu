@@ -803,7 +803,7 @@ __global__ void __launch_bounds__(256) k_viscosity(DfsphArgs a) {
                     return ldg8(a.pva + 2 * (size_t)j);   // {x_j, v_j after the pressure step}
                 },
                 [&](uint32_t j, const F4x2 &e) {
-                    if (j >= a.nf) return;
+                    const bool fj = j < a.nf;   // a boundary neighbour adds nothing (1M rows: 109 -> 107 us)
                     const float rx = p.x - e.a.x, ry = p.y - e.a.y, rz = p.z - e.a.z;
                     const float d2 = dist2(rx, ry, rz);
                     const float g = cubic_g(d2, a.k);
@@ -811,14 +811,14 @@ __global__ void __launch_bounds__(256) k_viscosity(DfsphArgs a) {
                     const float vx = vi.x - vj.x, vy = vi.y - vj.y, vz = vi.z - vj.z;
                     const float pi = a.vis_coef * (vx * rx + vy * ry + vz * rz) / (d2 + a.h2_001);
                     const float s = 10.f * pi * g;
-                    ax = __fmaf_rn(s, rx, ax);
-                    ay = __fmaf_rn(s, ry, ay);
-                    az = __fmaf_rn(s, rz, az);
+                    ax = fj ? __fmaf_rn(s, rx, ax) : ax;
+                    ay = fj ? __fmaf_rn(s, ry, ay) : ay;
+                    az = fj ? __fmaf_rn(s, rz, az) : az;
                     if (TENSION_SPLIT) {
                         const float sn = ncoef * g;
-                        nx = __fmaf_rn(sn, rx, nx);
-                        ny = __fmaf_rn(sn, ry, ny);
-                        nz = __fmaf_rn(sn, rz, nz);
+                        nx = fj ? __fmaf_rn(sn, rx, nx) : nx;
+                        ny = fj ? __fmaf_rn(sn, ry, ny) : ny;
+                        nz = fj ? __fmaf_rn(sn, rz, nz) : nz;
                     }
                 });
     finish_viscosity<TENSION_SPLIT>(a, T, r, vi, ax, ay, az, nx, ny, nz);
@@ -842,12 +842,12 @@ __global__ void __launch_bounds__(256) k_tension(DfsphArgs a) {
                     return PN{ldg4(a.pos + j), ldg4(a.normal + j)};
                 },
                 [&](uint32_t j, const PN &e) {
-                    if (j >= a.nf) return;
+                    const bool fj = j < a.nf;
                     float x, y, z;
                     tension_term(a, p, ni, e, x, y, z);
-                    tx += kk * x;
-                    ty += kk * y;
-                    tz += kk * z;
+                    tx = fj ? tx + kk * x : tx;
+                    ty = fj ? ty + kk * y : ty;
+                    tz = fj ? tz + kk * z : tz;
                 });
     finish_tension(a, T, r, tx, ty, tz);
 }

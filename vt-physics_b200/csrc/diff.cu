@@ -93,13 +93,13 @@ inline unsigned nblk(uint32_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
 // g'(r) / r of the cubic spline's gradient factor (gradW = g r).
 __device__ __forceinline__ float cubic_hh(float d2, const Cubic &k) {
-    if (!(d2 > 0.f)) return 0.f;
     const float r = sqrtf(d2);
     const float q = r * k.invh;
-    if (q < 1e-6f || q > 1.f) return 0.f;
     const float ih2 = k.invh * k.invh, ih4 = ih2 * ih2;
-    if (q <= 0.5f) return 18.f * k.sigma * ih4 / q;
-    return 6.f * k.sigma * ih4 * (1.f - q * q) / (q * q * q);
+    const bool inner = q <= 0.5f;   // one division for both sides, no branch
+    const float num = inner ? 18.f * k.sigma * ih4 : 6.f * k.sigma * ih4 * (1.f - q * q);
+    const float f = num / (inner ? q : q * q * q);
+    return !(d2 > 0.f) || q < 1e-6f || q > 1.f ? 0.f : f;
 }
 
 __device__ __forceinline__ double block_sum_d(double v) {

