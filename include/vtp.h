@@ -147,12 +147,13 @@ VTP_API int vtp_solver_create(int solver_type, vtp_solver **out);
  *       Morton order inside (compact neighbourhoods for the gathers) or
  *       "linear" in the reference's linear cell order; lists, exported keys
  *       and sorted order are the reference's either way;
- *   "rowLanes": threads per row of the PBF neighbour passes (1 = the list
- *       walked in order by one thread, default; 4 or 8 = the row's entries
- *       split over lanes and their sums added by a shuffle butterfly, for
- *       small scenes);
- *   "listLanes": neighbour-list builder lanes per row (0 = by row count,
- *       default; 1 or 8); every setting writes the same lists;
+ *   "rowLanes": threads per row of the PBF neighbour passes (1, default =
+ *       the terms added in list order, by one thread or, in scenes of up to
+ *       49,152 fluid rows, by a team of lanes with the same bits; 4 or 8 =
+ *       the row's entries split over lanes and their sums added by a shuffle
+ *       butterfly);
+ *   "listLanes": 0 (default), 1 or 8; accepted, the list builder is chosen by
+ *       row count and every one writes the same lists;
  *   "cubicCube": "rounded" (default) takes the (1 - q)^3 of the cubic
  *       kernel's outer branch correctly rounded, at most one ulp from the
  *       reference's powf(1 - q, 3) (KernelFunctions.cuh:29); "powf" calls powf

@@ -11,7 +11,8 @@ Tuned dimensions (keys of the solver config's "B200" block):
                  whose neighbourhoods the pressure solve copies into shared
                  memory; "cellOrder" / "stagedSolve" / "stageRows");
   * rowLanes   - threads per row of the PBF neighbour passes (1, 4, 8);
-  * listLanes  - threads per row of the list builder (0: by row count, 1, 8);
+  * listLanes  - accepted by the solver, which chooses its list builder by row
+                 count; every value measures the same;
   * adjointLanes - threads per row of the PBF adjoint's neighbour passes (1, 2,
                  4, 8), tuned for the differentiable workload only, after the
                  forward's keys, on the backward's wall-clock time.
