@@ -13,7 +13,6 @@
 // The arena is shared by every call on a device: two calls whose work
 // overlaps on the GPU (different streams, or different host threads without
 // ordering) corrupt each other's scratch.  Calls are ordered on one stream.
-#include <climits>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -202,171 +201,140 @@ __global__ void k_na_rank(vtp::Grid g, uint32_t n, const float *__restrict__ pos
                              __uint_as_float(me));
 }
 
-// Lists of up to R rows of one cell (as cell_lists of ugns.cu, for one run per cell and lists that
-// are rows of a plain array).  Lane l works for row l % R, lane h * R + k taking the h-th share of
-// row k's candidates.
-template <uint32_t R>
-__device__ __forceinline__ void na_cell_lists(vtp::CellScratch &S, uint32_t f0, uint32_t len, uint32_t excl,
-                                              uint32_t total, bool live, float4 p, const vtp::Grid &g, const Arena &a,
-                                              uint32_t *__restrict__ counts, uint32_t *__restrict__ nbrs) {
-    constexpr unsigned kAll = 0xffffffffu;
-    constexpr uint32_t H = 32u / R;
-    const uint32_t lane = threadIdx.x & 31u, k = lane % R, h = lane / R, cap = g.maxnbr - 1u;
-    const uint64_t px = vtp::f2_pack(-p.x, -p.x), py = vtp::f2_pack(-p.y, -p.y), pz = vtp::f2_pack(-p.z, -p.z);
-    const uint32_t to0 = (uint32_t)__cvta_generic_to_shared(&S.kept[lane][0]);
-    uint32_t found = 0;
-    for (uint32_t wb = 0; wb < total; wb += vtp::kCellWindow) {
-        const uint32_t wl = min(vtp::kCellWindow, total - wb);
-        const uint32_t share = ((wl + H - 1u) / H + 7u) & ~7u;
-        // The window's candidates: sorted slots first, then positions and ids in their place.
-        __syncwarp();
-        const uint32_t o0 = wb > excl ? min(wb - excl, len) : 0u, o1 = wb + wl > excl ? min(wb + wl - excl, len) : 0u;
-        for (uint32_t o = o0; o < o1; ++o) S.cand[excl + o - wb] = f0 + o;
-        __syncwarp();
-        for (uint32_t q = lane; q < H * share; q += 32u) {
-            const float far = __int_as_float(0x7f800000);
-            float4 v = make_float4(far, far, far, 0.f);
-            if (q < wl) {
-                v = __ldg(a.pos + S.cand[q]);
-                S.cand[q] = __float_as_uint(v.w);
-            }
-            S.x[0][q] = v.x;
-            S.x[1][q] = v.y;
-            S.x[2][q] = v.z;
-        }
-        __syncwarp();
-        uint32_t to = to0;
-        for (uint32_t off = 0; off < share; off += 8u) {
-            vtp::test4(S, h * share + off, off, to, px, py, pz, g.d2max);
-            vtp::test4(S, h * share + off + 4u, off + 4u, to, px, py, pz, g.d2max);
-        }
-        const uint32_t mine = live ? to - to0 : 0u;
-        uint32_t x = mine;
-#pragma unroll
-        for (uint32_t o = R; o < 32u; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(kAll, x, o);
-            if (lane >= o) x += y;
-        }
-        __syncwarp();
-#pragma unroll
-        for (uint32_t r = 0; r < R; r += 4) {   // 8 consecutive entries of 4 rows at a time
-            const uint32_t kk = r + (lane >> 3);
-            uint32_t lo[H];
-#pragma unroll
-            for (uint32_t t = 0; t < H; ++t) lo[t] = __shfl_sync(kAll, x - mine, (int)(kk + R * t));
-            const uint32_t n = __shfl_sync(kAll, x, (int)(kk + 32u - R));
-            const uint32_t before = __shfl_sync(kAll, found, (int)kk);
-            const uint32_t id = __float_as_uint(__shfl_sync(kAll, p.w, (int)kk));
-            uint32_t *out = nbrs + (size_t)id * g.maxnbr + 1u;
-            for (uint32_t e = lane & 7u; e < n && before + e < cap; e += 8u) {
-                uint32_t at = kk * vtp::kCellKept + e, share_of = 0;
-#pragma unroll
-                for (uint32_t t = 1; t < H; ++t)
-                    if (e >= lo[t]) at = (kk + R * t) * vtp::kCellKept + (e - lo[t]), share_of = t * share;
-                out[before + e] = S.cand[share_of + (&S.kept[0][0])[at]];
-            }
-        }
-        found += __shfl_sync(kAll, x, (int)(k + 32u - R));
+// Where the entries of a particle's list go: its row of the caller's array, after the particle itself.
+struct ArrayOut {
+    static constexpr bool kIds = true;   // entries are particle ids
+    uint32_t *nbrs;
+    uint32_t id, stride;                 // of this lane's particle; entries of a row of the array
+    __device__ __forceinline__ bool eights() const { return true; }
+    __device__ __forceinline__ uint32_t *mine() const { return nbrs + (size_t)id * stride + 1u; }
+    __device__ __forceinline__ uint32_t *of(uint32_t lane) const {
+        return nbrs + (size_t)__shfl_sync(0xffffffffu, id, (int)lane) * stride + 1u;
     }
-    // Self, the count and the unused slots.
+    __device__ __forceinline__ void put(uint32_t *dst, uint32_t slot, uint32_t j) const {
+        if (slot + 1u < stride) dst[slot] = j;
+    }
+};
+
+// What a list has beside its entries: the particle itself, the count and the unused slots.  One lane
+// per list has `lead` set, with the list's `found` and `out`.
+__device__ __forceinline__ void finish_lists(uint32_t found, bool lead, const ArrayOut &out,
+                                             uint32_t *__restrict__ counts) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u, n = min(found + 1u, out.stride);
+    if (lead) {
+        out.nbrs[(size_t)out.id * out.stride] = out.id;
+        counts[out.id] = n;
+    }
+    unsigned todo = __ballot_sync(kAll, lead);
+    while (todo) {   // eight lanes a list, four lists at a time
+        uint32_t src = 32u;
 #pragma unroll
-    for (uint32_t r = 0; r < R; r += 4) {
-        const uint32_t kk = r + (lane >> 3), e0 = lane & 7u;
-        const uint32_t n = min(__shfl_sync(kAll, found, (int)kk), cap) + 1u;
-        const uint32_t id = __float_as_uint(__shfl_sync(kAll, p.w, (int)kk));
-        if (!__shfl_sync(kAll, (int)live, (int)kk)) continue;
-        uint32_t *out = nbrs + (size_t)id * g.maxnbr;
-        if (e0 == 0) {
-            out[0] = id;
-            counts[id] = n;
+        for (uint32_t q = 0; q < 4u; ++q) {
+            if (todo && (lane >> 3) == q) src = (uint32_t)__ffs((int)todo) - 1u;
+            todo &= todo - 1u;
         }
-        for (uint32_t e = n + e0; e < g.maxnbr; e += 8u) out[e] = 0xffffffffu;
+        const uint32_t nk = __shfl_sync(kAll, n, (int)(src & 31u)), id = __shfl_sync(kAll, out.id, (int)(src & 31u));
+        if (src < 32u)
+            for (uint32_t e = nk + (lane & 7u); e < out.stride; e += 8u) out.nbrs[(size_t)id * out.stride + e] = 0xffffffffu;
     }
 }
 
+// The run of the neighbour cell at offset t of cell c.
+__device__ __forceinline__ vtp::CellRuns runs_at(int3 c, int t, const vtp::Grid &g, const uint32_t *start) {
+    vtp::CellRuns r{};
+    const int3 o = vtp::nbr_offset(t);
+    const int3 cc = make_int3(c.x + o.x, c.y + o.y, c.z + o.z);
+    if (vtp::cell_available(cc, g)) {
+        const uint32_t b = vtp::cell_key(cc, g);
+        r.f0 = start[b];
+        r.f1 = start[b + 1];
+    }
+    return r;
+}
+
+// A particle for walk_rows.
+struct WalkedParticle {
+    float4 p;
+    int3 c;
+    const vtp::Grid *g;
+    const uint32_t *start;
+    ArrayOut out;
+    __device__ __forceinline__ vtp::CellRuns runs(int t) const { return runs_at(c, t, *g, start); }
+};
+
 // Lists in the reference layout: self first, then the 27 cells in the reference's offset order,
-// particles of a cell by ascending id.  One warp per occupied cell (its candidates are laid out and
-// tested as in the solvers' builder), found among the kNaScan sorted slots each warp looks at.
-// Bound by issue; a thread per particle wrote every entry to a line of its own and walked its 27
-// cells alone.  404,891 particles, 60 slots: whole call 292 -> 205 us (B200).
-constexpr uint32_t kNaScan = 8;
+// particles of a cell by ascending id.  As k_build_lists (ugns.cu): a warp takes SCAN sorted particles,
+// builds the groups of one cell that start among them together, and walks the cells of the others.
+// Whole call (B200, us), a thread per particle -> a warp per cell -> this: 400,000 particles half a
+// cell apart 279 -> 216 -> 206, one cell apart 209 -> 326 -> 139, 0.35 cells apart 414 -> 499 -> 359;
+// 20,000 half a cell apart 107 -> 64 -> 64, with 10,000 of them in one cell 2,156 -> 27,800 -> 610.
+template <uint32_t SCAN>
 __global__ void __launch_bounds__(vtp::kCellWarps * 32, 7) k_na_walk(vtp::Grid g, uint32_t n, Arena a,
                                                                      uint32_t *__restrict__ counts,
                                                                      uint32_t *__restrict__ nbrs) {
     __shared__ __align__(16) vtp::CellScratch scratch[vtp::kCellWarps];
     constexpr unsigned kAll = 0xffffffffu;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t first = (blockIdx.x * vtp::kCellWarps + (threadIdx.x >> 5)) * kNaScan;
+    constexpr uint32_t R = 8;
+    const uint32_t lane = threadIdx.x & 31u, k = lane % SCAN;
+    const uint32_t first = (blockIdx.x * vtp::kCellWarps + (threadIdx.x >> 5)) * SCAN;
     if (first >= n) return;
     vtp::CellScratch &S = scratch[threadIdx.x >> 5];
-    const int3 o = vtp::nbr_offset((int)min(lane, 26u));
-    uint32_t cell_end = 0;
-    bool leads = false, outside = false;
-    uint32_t id = 0;
-    if (lane < kNaScan && first + lane < n) {
-        const float4 p = a.pos[first + lane];
-        id = __float_as_uint(p.w);
-        const int3 c = vtp::cell_of(p.x, p.y, p.z, g);
-        if (vtp::cell_available(c, g)) {
-            const uint32_t k = vtp::cell_key(c, g);
-            leads = a.start[k] == first + lane;
-            cell_end = a.start[k + 1];
-        } else {
-            outside = true;
-            counts[id] = 0;
-        }
+    const uint32_t m0 = min(SCAN, n - first), i = first + min(k, m0 - 1u);
+    const float4 p = a.pos[i];
+    const int3 own = vtp::cell_of(p.x, p.y, p.z, g);
+    const bool inside = vtp::cell_available(own, g);
+    uint32_t rows = 0;   // of the group that starts at particle i
+    bool alone = false;   // its list is not built with a group
+    if (inside) {
+        const uint32_t b = vtp::cell_key(own, g), s = a.start[b], e = a.start[b + 1];
+        const uint32_t in_group = (i - s) % R, m = min(R, e - (i - in_group));
+        bool together = m >= vtp::kGroupMin || e - s > vtp::kCrowded;
+        if (SCAN == 32u) together = together && e - s <= vtp::kSharedRows;
+        if (together && in_group == 0u && lane < m0) rows = m;
+        alone = !together;
     }
-    for (unsigned m = __ballot_sync(kAll, outside); m; m &= m - 1u) {   // outside the grid: an empty list
-        uint32_t *out = nbrs + (size_t)__shfl_sync(kAll, id, __ffs((int)m) - 1) * g.maxnbr;
-        for (uint32_t e = lane; e < g.maxnbr; e += 32u) out[e] = 0xffffffffu;
-    }
-    for (unsigned todo = __ballot_sync(kAll, leads); todo; todo &= todo - 1u) {
+    for (unsigned todo = __ballot_sync(kAll, rows != 0u); todo; todo &= todo - 1u) {
         const int leader = __ffs((int)todo) - 1;
-        const uint32_t beg = first + (uint32_t)leader, end = __shfl_sync(kAll, cell_end, leader);
-        int3 at = make_int3(INT_MIN, 0, 0);   // the cell whose run is held
-        uint32_t f0 = 0, len = 0, excl = 0, total = 0;
-        for (uint32_t rg = beg; rg < end; rg += 8u) {
-            const uint32_t m = min(8u, end - rg);
-            const float4 p = a.pos[rg + min(lane & 7u, m - 1u)];
-            const int3 c = vtp::cell_of(p.x, p.y, p.z, g);
-            // A cell on the grid's inclusive upper face shares its bucket with another cell: one
-            // round per cell among these rows.
-            for (unsigned left = (1u << m) - 1u; left;) {
-                const int f = __ffs((int)left) - 1;
-                const int3 c0 = make_int3(__shfl_sync(kAll, c.x, f), __shfl_sync(kAll, c.y, f), __shfl_sync(kAll, c.z, f));
-                const bool mine = ((left >> (lane & 7u)) & 1u) && c.x == c0.x && c.y == c0.y && c.z == c0.z;
-                left &= ~__ballot_sync(kAll, mine);
-                if (c0.x != at.x || c0.y != at.y || c0.z != at.z) {
-                    at = c0;
-                    f0 = len = 0;
-                    const int3 cc = make_int3(c0.x + o.x, c0.y + o.y, c0.z + o.z);
-                    if (lane < 27u && vtp::cell_available(cc, g)) {
-                        const uint32_t k = vtp::cell_key(cc, g);
-                        f0 = a.start[k];
-                        len = a.start[k + 1] - f0;
-                    }
-                    uint32_t incl = len;
-#pragma unroll
-                    for (int d = 1; d < 32; d <<= 1) {
-                        const uint32_t y = __shfl_up_sync(kAll, incl, d);
-                        if ((int)lane >= d) incl += y;
-                    }
-                    excl = incl - len;
-                    total = __shfl_sync(kAll, incl, 31);
-                }
-                if (m <= 4u) {
-                    const int s = (int)(lane & 3u);
-                    const float4 p4 = make_float4(__shfl_sync(kAll, p.x, s), __shfl_sync(kAll, p.y, s),
-                                                  __shfl_sync(kAll, p.z, s), __shfl_sync(kAll, p.w, s));
-                    const bool live = __shfl_sync(kAll, (int)mine, s) != 0;
-                    na_cell_lists<4>(S, f0, len, excl, total, live, p4, g, a, counts, nbrs);
-                } else {
-                    na_cell_lists<8>(S, f0, len, excl, total, mine, p, g, a, counts, nbrs);
-                }
-                __syncwarp();
-            }
+        const uint32_t m = __shfl_sync(kAll, rows, leader), beg = __shfl_sync(kAll, i, leader), kr = lane % R;
+        const float4 q = a.pos[beg + min(kr, m - 1u)];
+        const int3 c = vtp::cell_of(q.x, q.y, q.z, g);
+        // A cell on the grid's inclusive upper face shares its bucket with another cell: one round
+        // per cell among these particles.
+        for (unsigned left = (1u << m) - 1u; left;) {
+            const int f = __ffs((int)left) - 1;
+            const int3 c0 = make_int3(__shfl_sync(kAll, c.x, f), __shfl_sync(kAll, c.y, f), __shfl_sync(kAll, c.z, f));
+            const bool mine = ((left >> kr) & 1u) && c.x == c0.x && c.y == c0.y && c.z == c0.z;
+            left &= ~__ballot_sync(kAll, mine);
+            vtp::CellRuns runs{};
+            if (lane < 27u) runs = runs_at(c0, (int)lane, g, a.start);
+            const uint32_t total = vtp::place_runs(runs);
+            const ArrayOut out{nbrs, __float_as_uint(q.w), g.maxnbr};
+            const uint32_t found = vtp::cell_rows<0, R>(S, runs, total, mine, q, g.d2max, a.pos, nullptr, out);
+            finish_lists(found, mine && lane < R, out, counts);
+            __syncwarp();
         }
     }
+    // Outside the grid: an empty list.
+    for (unsigned todo = __ballot_sync(kAll, lane < m0 && !inside); todo; todo &= todo - 1u) {
+        const uint32_t id = __float_as_uint(__shfl_sync(kAll, p.w, __ffs((int)todo) - 1));
+        if (lane == 0) counts[id] = 0;
+        for (uint32_t e = lane; e < g.maxnbr; e += 32u) nbrs[(size_t)id * g.maxnbr + e] = 0xffffffffu;
+    }
+    vtp::walk_rows<0>(
+        S, __ballot_sync(kAll, alone && lane < m0), g.d2max, a.pos, nullptr,
+        [&](uint32_t l) {
+            WalkedParticle r;
+            r.p = make_float4(__shfl_sync(kAll, p.x, (int)l), __shfl_sync(kAll, p.y, (int)l),
+                              __shfl_sync(kAll, p.z, (int)l), __shfl_sync(kAll, p.w, (int)l));
+            r.c = make_int3(__shfl_sync(kAll, own.x, (int)l), __shfl_sync(kAll, own.y, (int)l),
+                            __shfl_sync(kAll, own.z, (int)l));
+            r.g = &g;
+            r.start = a.start;
+            r.out = ArrayOut{nbrs, __float_as_uint(r.p.w), g.maxnbr};
+            return r;
+        },
+        [&](const WalkedParticle &r, uint32_t found, bool lead) { finish_lists(found, lead, r.out, counts); });
 }
 
 inline unsigned nblk(uint32_t n, int b) { return (unsigned)((n + b - 1) / b); }
@@ -440,7 +408,9 @@ extern "C" VTP_API int vtp_ugns_neighbors_noalloc(const float *d_pos, uint32_t n
     k_na_scan<<<tiles, kScanThreads, 0, st>>>(nb, a);
     k_na_scatter<<<nblk(n, 256), 256, 0, st>>>(n, a);
     k_na_rank<<<nblk(n, 256), 256, 0, st>>>(g, n, d_pos, a);
-    k_na_walk<<<nblk(n, vtp::kCellWarps * kNaScan), vtp::kCellWarps * 32, 0, st>>>(g, n, a, d_counts, d_nbrs);
+    constexpr int kBlock = vtp::kCellWarps * 32;
+    if (n <= vtp::kScan8Rows) k_na_walk<8><<<nblk(n, vtp::kCellWarps * 8), kBlock, 0, st>>>(g, n, a, d_counts, d_nbrs);
+    else k_na_walk<32><<<nblk(n, kBlock), kBlock, 0, st>>>(g, n, a, d_counts, d_nbrs);
     e = cudaGetLastError();
     if (e != cudaSuccess) return vtp::fail(VTP_ERR_CUDA, cudaGetErrorString(e));
     return VTP_OK;

@@ -17,7 +17,6 @@
 #include "cells.cuh"
 #include "staged.h"
 
-#include <climits>
 #include <type_traits>
 
 
@@ -25,8 +24,9 @@ namespace vtp {
 
 namespace {
 
-// More rows than this take the builder with a thread per row.
-constexpr uint32_t kWalkRows = 300000;
+// Up to this many rows a warp of k_build_lists takes 4, with eight lanes a row: twice the warps, each
+// with half the work in sequence.
+constexpr uint32_t kScan4Rows = 16384;
 constexpr int kWalkBlock = 128;
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
@@ -383,11 +383,11 @@ struct Walker {
     }
 };
 
-// One thread per row walks its 27 cells and appends to its list: the faster builder from some
-// hundred thousand rows on (kWalkRows; 500,000 rows 138 us against 154 for k_build_lists,
-// 1,000,000 rows 240 against 258), where every SM has rows enough and the cells' shared memory
-// phases of k_build_lists cost more than the lookups they share.  Issue-bound at 80 % of the issue
-// slots (29 warp instructions per warp-level candidate test).
+// One thread per row walks its 27 cells and appends to its list: the builder of more than
+// kScan8Rows rows in lists of shape lg 0, where every SM has rows enough.  250,000 rows (B200, us),
+// against a warp per cell and against k_build_lists with 32 rows a warp: a dam break at rest 74 (70,
+// 64), after 150 substeps 101 (119, 124), clouds 0.35, 0.5, 0.7 and 1 cells apart 229 (348, 235), 98
+// (117, 104), 76 (125, 111), 44 (191, 51), with 4,000 rows in one cell 390 (8,230, 740).
 template <int MODE, bool CULL>
 __global__ void k_walk_lists(Scenes sc, uint32_t row0, uint32_t cnt, ListShape shape,
                               const float4 *__restrict__ pos, const uint32_t *__restrict__ orig,
@@ -436,129 +436,61 @@ __global__ void k_walk_lists(Scenes sc, uint32_t row0, uint32_t cnt, ListShape s
     }
 }
 
-// List builder: one warp per occupied cell.  The rows of a cell share their 27 neighbour cells,
-// so the warp lays the candidates of those cells out once in shared memory, in list order (27
-// offsets in the reference's order, each cell's two runs in MODE's order), and every row of the
-// cell walks that layout: R rows at a time, 32 / R lanes per row, each lane a contiguous share of
-// the candidates.  A lane tests two candidates per packed FP32 instruction (the roundings of
-// dist2) and keeps the accepted ones as bits; the lanes' bit counts, scanned over the row, give
-// each lane its first slot, and the lists are composed in shared memory and written segment by
-// segment.  Against a walk per row, the cell lookups, the candidate loads and the loop control
-// are paid once per cell instead of once per row.
-// It is bound by issue.  Event-timed launches (B200, us), the former builders (eight lanes per row
-// up to 131,072 rows, above that one thread per row) -> this: 16,000 rows 19 -> 12.5, 31,000 rows
-// 39 -> 23 (DFSPH blocks), 64,000 rows 68 -> 24, 128,000 rows 119 -> 41, 250,000 rows 93 -> 72.
-constexpr uint32_t kCellScan = 8;        // rows a warp scans for cells that start there: about one cell
-// The runs of one neighbour cell, held by lane t < 27 for the t-th offset, and where its
-// candidates start in list order.
-struct CellRuns {
-    uint32_t f0, f1, b0, b1, excl;
+// Where the entries of a solver's lists go.  `row`: list row of this lane's row.
+struct ListOut {
+    static constexpr bool kIds = false;   // entries are sorted rows
+    ListShape shape;
+    uint32_t *nbr;
+    uint32_t row, cap;
+    __device__ __forceinline__ bool eights() const { return shape.lg != 0u; }
+    __device__ __forceinline__ uint32_t *mine() const { return nbr + ell_index(row, 0, shape); }
+    __device__ __forceinline__ uint32_t *of(uint32_t lane) const {
+        return nbr + ell_index(__shfl_sync(0xffffffffu, row, (int)lane), 0, shape);
+    }
+    __device__ __forceinline__ void put(uint32_t *dst, uint32_t slot, uint32_t j) const {
+        if (slot < cap) dst[ell_slot(slot, shape)] = j;
+    }
 };
 
-// Lays candidates [wb, wb + wl) out: rows and positions, infinity from wl up to `padded`.
-template <int MODE>
-__device__ __forceinline__ void stage_candidates(CellScratch &S, const CellRuns &R, uint32_t wb, uint32_t wl,
-                                                 uint32_t padded, const float4 *__restrict__ pos,
-                                                 const uint32_t *__restrict__ orig) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t nf = R.f1 - R.f0, nb = R.b1 - R.b0, len = nf + nb;
-    __syncwarp();
-    if (MODE == 2) {
-        uint32_t fi = R.f0, bi = R.b0;
-        for (uint32_t o = 0; o < len; ++o) {
-            const uint32_t j = merge_next(fi, R.f1, bi, R.b1, orig);
-            if (R.excl + o - wb < wl) S.cand[R.excl + o - wb] = j;
-        }
-    } else {
-        // the part of this lane's runs that lies in the window
-        const uint32_t na = MODE == 0 ? nf : nb, a0 = MODE == 0 ? R.f0 : R.b0, c0 = (MODE == 0 ? R.b0 : R.f0) - na;
-        const uint32_t o0 = wb > R.excl ? min(wb - R.excl, len) : 0u;
-        const uint32_t o1 = wb + wl > R.excl ? min(wb + wl - R.excl, len) : 0u;
-        for (uint32_t o = o0; o < o1; ++o) S.cand[R.excl + o - wb] = (o < na ? a0 : c0) + o;
+// The runs of the neighbour cell at offset t of cell c.
+__device__ __forceinline__ CellRuns runs_at(int3 c, int t, const SceneGrid &g, const uint32_t *__restrict__ fstart,
+                                            const uint32_t *__restrict__ bstart) {
+    CellRuns r{};
+    const int3 o = nbr_offset(t);
+    const int3 cc = make_int3(c.x + o.x, c.y + o.y, c.z + o.z);
+    if (cell_available(cc, g)) {
+        const uint32_t b = g.key_base + cell_key(cc, g);
+        r.f0 = __ldg(fstart + b); r.f1 = __ldg(fstart + b + 1);
+        r.b0 = __ldg(bstart + b); r.b1 = __ldg(bstart + b + 1);
     }
-    __syncwarp();
-    for (uint32_t q = lane; q < padded; q += 32u) {
-        const float far = __int_as_float(0x7f800000);
-        float4 v = make_float4(far, far, far, 0.f);
-        if (q < wl) v = __ldg(pos + S.cand[q]);
-        S.x[0][q] = v.x;
-        S.x[1][q] = v.y;
-        S.x[2][q] = v.z;
-    }
-    __syncwarp();
+    return r;
 }
 
-// Lists of up to R rows of one cell.  Lane l works for row l % R: `row` (absolute, the same for
-// the row's lanes), `live` for rows that exist.
-template <int MODE, uint32_t R>
-__device__ __forceinline__ void cell_lists(CellScratch &S, const CellRuns &runs, uint32_t total, bool live,
-                                           uint32_t row, uint32_t row0, float4 p, float d2max, uint32_t cap,
-                                           ListShape shape, const float4 *__restrict__ pos,
-                                           const uint32_t *__restrict__ orig, uint32_t *__restrict__ nbr,
-                                           uint32_t *__restrict__ ncnt, uint32_t *__restrict__ status,
-                                           uint32_t *__restrict__ overflow_count) {
-    constexpr unsigned kAll = 0xffffffffu;
-    constexpr uint32_t H = 32u / R;   // lanes per row
-    const uint32_t lane = threadIdx.x & 31u, k = lane % R, h = lane / R;
-    const uint64_t px = f2_pack(-p.x, -p.x), py = f2_pack(-p.y, -p.y), pz = f2_pack(-p.z, -p.z);
-    const uint32_t to0 = (uint32_t)__cvta_generic_to_shared(&S.kept[lane][0]);
-    uint32_t found = 0;   // entries of the row in earlier windows
-    for (uint32_t wb = 0; wb < total; wb += kCellWindow) {
-        const uint32_t wl = min(kCellWindow, total - wb);
-        const uint32_t share = ((wl + H - 1u) / H + 7u) & ~7u;   // candidates per lane, in eights
-        stage_candidates<MODE>(S, runs, wb, wl, H * share, pos, orig);
-        uint32_t to = to0;
-        for (uint32_t off = 0; off < share; off += 8u) {
-            test4(S, h * share + off, off, to, px, py, pz, d2max);
-            test4(S, h * share + off + 4u, off + 4u, to, px, py, pz, d2max);
-        }
-        const uint32_t mine = live ? to - to0 : 0u;
-        uint32_t x = mine;
-#pragma unroll
-        for (uint32_t o = R; o < 32u; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(kAll, x, o);
-            if (lane >= o) x += y;
-        }
-        __syncwarp();
-        // The lists leave as they are stored: 8 entries of 4 rows, or H entries of R rows, at a
-        // time.  Entry e of a row is in the share of the last lane whose entries start at or
-        // before e.
-        auto flush = [&](uint32_t kk, uint32_t e0, uint32_t step) {
-            uint32_t lo[H];
-#pragma unroll
-            for (uint32_t t = 0; t < H; ++t) lo[t] = __shfl_sync(kAll, x - mine, (int)(kk + R * t));
-            const uint32_t n = __shfl_sync(kAll, x, (int)(kk + 32u - R));
-            const uint32_t before = __shfl_sync(kAll, found, (int)kk);
-            const uint32_t i = __shfl_sync(kAll, row, (int)kk) - row0;
-            uint32_t *dst = nbr + ell_index(i, 0, shape);
-            for (uint32_t e = e0; e < n; e += step) {
-                uint32_t at = kk * kCellKept + e, share_of = 0;
-#pragma unroll
-                for (uint32_t t = 1; t < H; ++t)
-                    if (e >= lo[t]) at = (kk + R * t) * kCellKept + (e - lo[t]), share_of = t * share;
-                const uint32_t slot = before + e;
-                if (slot < cap) dst[ell_slot(slot, shape)] = S.cand[share_of + (&S.kept[0][0])[at]];
-            }
-        };
-        if (shape.lg) {
-#pragma unroll
-            for (uint32_t r = 0; r < R; r += 4) flush(r + (lane >> 3), lane & 7u, 8u);
-        } else {
-            flush(k, h, H);
-        }
-        found += __shfl_sync(kAll, x, (int)(k + 32u - R));
-    }
-    if (live && h == 0) {
-        ncnt[row - row0] = min(found, cap) + 1u;
-        if (found > cap) {
-            atomicAdd(overflow_count, 1u);
-            atomicOr(status, ST_BOUNDS);
-        }
-    }
-}
+// A row for walk_rows.
+struct WalkedRow {
+    float4 p;
+    int3 c;
+    uint32_t i;
+    SceneGrid g;
+    const uint32_t *fstart, *bstart;
+    ListOut out;
+    __device__ __forceinline__ CellRuns runs(int t) const { return runs_at(c, t, g, fstart, bstart); }
+};
 
-// Each warp builds the cells that start among its kCellScan rows.
-template <int MODE>
+// The list builder up to kScan8Rows rows: a warp takes SCAN consecutive sorted rows.  The rows of a
+// cell share their 27 neighbour cells, so groups of rows of one cell are built together: the warp lays
+// the candidates of those cells out in shared memory, in list order (27 offsets in the reference's
+// order, each cell's two runs in MODE's order), the row's lanes each test a contiguous share of them,
+// two to a packed FP32 instruction (the roundings of dist2), and keep the accepted ones as byte
+// offsets into the share; the lanes' counts, scanned over the row, give each lane its first slot
+// (cell_rows, cells.cuh).  Rows of groups too small to share that work are walked side by side
+// (walk_rows).  Event-timed launches (B200, us), eight lanes per row -> a warp per cell -> this.  Dam
+// breaks at rest: PBF 16,000 rows 23 -> 13 -> 15, 64,000 rows 68 -> 25 -> 23, 120,000 rows 109 -> 44 ->
+// 41, DFSPH 16,000 rows 23 -> 17 -> 17, 128,000 rows 113 -> 50 -> 48.  After 100-200 substeps: 21 -> 21 ->
+// 23, 50 -> 48 -> 47, 80 -> 72 -> 64, 21 -> 21 -> 23, 80 -> 76 -> 62.  Clouds of 100,000 rows 0.35, 0.7 and
+// 1 cells apart: 188 -> 162 -> 91, 44 -> 58 -> 56, 27 -> 88 -> 33.  30,000 rows with 10,000 in one cell:
+// 750 -> 46,900 -> 580.
+template <int MODE, uint32_t SCAN>
 __global__ void __launch_bounds__(kCellWarps * 32, 7) k_build_lists(
     Scenes sc, uint32_t row0, uint32_t cnt, ListShape shape, const float4 *__restrict__ pos,
     const uint32_t *__restrict__ orig, const uint32_t *__restrict__ start, const uint32_t *__restrict__ fstart,
@@ -567,155 +499,89 @@ __global__ void __launch_bounds__(kCellWarps * 32, 7) k_build_lists(
     pdl_enter();
     __shared__ __align__(16) CellScratch scratch[kCellWarps];
     constexpr unsigned kAll = 0xffffffffu;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t first = (blockIdx.x * kCellWarps + (threadIdx.x >> 5)) * kCellScan;
+    constexpr uint32_t R = SCAN == 4u ? 4u : 8u;   // rows of a group
+    const uint32_t lane = threadIdx.x & 31u, k = lane % SCAN;
+    const uint32_t first = (blockIdx.x * kCellWarps + (threadIdx.x >> 5)) * SCAN;
     if (first >= cnt) return;
     CellScratch &S = scratch[threadIdx.x >> 5];
     const float d2max = sc.d2max;
     const uint32_t cap = sc.maxnbr - 1u;
-    const int3 o = nbr_offset((int)min(lane, 26u));
 
-    // Rows of this warp's window that start a cell; the warp builds the lists of those whole cells.
-    uint32_t cell_end = 0;
-    int3 own = make_int3(0, 0, 0);
-    bool leads = false;
-    if (lane < kCellScan && first + lane < cnt) {
-        const uint32_t i = row0 + first + lane;
-        const SceneGrid g = load_scene(sc, i);
-        const float4 p = pos[i];
-        own = cell_of(p.x, p.y, p.z, g, sc.cell);
-        if (cell_available(own, g)) {
-            const uint32_t k = g.key_base + cell_key(own, g);
-            leads = __ldg(start + k) == i;
-            cell_end = __ldg(start + k + 1);
-        } else {
-            ncnt[first + lane] = 0;   // outside the grid: no neighbours, not even self
-        }
+    // This lane's row of the warp's SCAN rows, and the group it is in.
+    const uint32_t n = min(SCAN, cnt - first), i = row0 + first + min(k, n - 1u);
+    const SceneGrid g = load_scene(sc, i);
+    const float4 p = pos[i];
+    const int3 own = cell_of(p.x, p.y, p.z, g, sc.cell);
+    uint32_t rows = 0;   // of the group that starts at row i
+    bool walked = false;
+    if (cell_available(own, g)) {
+        const uint32_t b = g.key_base + cell_key(own, g), s = __ldg(start + b), e = __ldg(start + b + 1);
+        const uint32_t in_group = (i - s) % R, m = min(R, e - (i - in_group));
+        const bool together = m >= (SCAN == 4u ? kGroupMin4 : kGroupMin) || e - s > kCrowded;
+        if (together && in_group == 0u && lane < n) rows = m;
+        walked = !together && k < n;
+    } else if (lane < n) {
+        ncnt[first + lane] = 0;   // outside the grid: no neighbours, not even self
     }
-    for (unsigned todo = __ballot_sync(kAll, leads); todo; todo &= todo - 1u) {
+    for (unsigned todo = __ballot_sync(kAll, rows != 0u); todo; todo &= todo - 1u) {
         const int leader = __ffs((int)todo) - 1;
-        const uint32_t beg = row0 + first + (uint32_t)leader;
-        const uint32_t end = __shfl_sync(kAll, cell_end, leader);
+        const uint32_t m = __shfl_sync(kAll, rows, leader), beg = __shfl_sync(kAll, i, leader);
+        const uint32_t kr = lane % R, row = beg + min(kr, m - 1u);
+        const SceneGrid gg = load_scene(sc, beg);
+        const float4 q = pos[row];
         int3 c0 = make_int3(__shfl_sync(kAll, own.x, leader), __shfl_sync(kAll, own.y, leader),
                             __shfl_sync(kAll, own.z, leader));
-        const SceneGrid g = load_scene(sc, beg);
-        int3 at = make_int3(INT_MIN, 0, 0);   // the cell whose runs are held
-        CellRuns runs{};
-        uint32_t total = 0;
-        for (uint32_t rg = beg; rg < end; rg += 8u) {
-            const uint32_t n = min(8u, end - rg);
-            const uint32_t row = rg + min(lane & 7u, n - 1u);
-            const float4 p = pos[row];
-            // A bucket of the bricked order is one cell.  In the linear order a cell on the grid's
-            // inclusive upper face shares its bucket with another cell: one round per cell then.
-            for (unsigned left = (1u << n) - 1u; left;) {
-                bool mine = (lane & 7u) < n;
-                if (g.brick) {
-                    left = 0;
-                } else {
-                    const int3 c = cell_of(p.x, p.y, p.z, g, sc.cell);
-                    const int f = __ffs((int)left) - 1;
-                    c0 = make_int3(__shfl_sync(kAll, c.x, f), __shfl_sync(kAll, c.y, f), __shfl_sync(kAll, c.z, f));
-                    mine = ((left >> (lane & 7u)) & 1u) && c.x == c0.x && c.y == c0.y && c.z == c0.z;
-                    left &= ~__ballot_sync(kAll, mine);
-                }
-                if (c0.x != at.x || c0.y != at.y || c0.z != at.z) {
-                    at = c0;
-                    runs = CellRuns{};
-                    if (lane < 27u) {
-                        const int3 cc = make_int3(c0.x + o.x, c0.y + o.y, c0.z + o.z);
-                        if (cell_available(cc, g)) {
-                            const uint32_t k = g.key_base + cell_key(cc, g);
-                            runs.f0 = __ldg(fstart + k); runs.f1 = __ldg(fstart + k + 1);
-                            runs.b0 = __ldg(bstart + k); runs.b1 = __ldg(bstart + k + 1);
-                        }
-                    }
-                    const uint32_t len = (runs.f1 - runs.f0) + (runs.b1 - runs.b0);
-                    uint32_t incl = len;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const uint32_t y = __shfl_up_sync(kAll, incl, o);
-                        if ((int)lane >= o) incl += y;
-                    }
-                    runs.excl = incl - len;
-                    total = __shfl_sync(kAll, incl, 31);
-                }
-                // Up to four rows of a last, short group take 8 lanes each, else 4 lanes each.
-                if (n <= 4u) {
-                    const uint32_t row4 = __shfl_sync(kAll, row, (int)(lane & 3u));
-                    const float4 p4 = make_float4(__shfl_sync(kAll, p.x, (int)(lane & 3u)),
-                                                  __shfl_sync(kAll, p.y, (int)(lane & 3u)),
-                                                  __shfl_sync(kAll, p.z, (int)(lane & 3u)), 0.f);
-                    const bool live = __shfl_sync(kAll, (int)mine, (int)(lane & 3u)) != 0;
-                    cell_lists<MODE, 4>(S, runs, total, live, row4, row0, p4, d2max, cap, shape, pos, orig,
-                                        nbr, ncnt, status, overflow_count);
-                } else {
-                    cell_lists<MODE, 8>(S, runs, total, mine, row, row0, p, d2max, cap, shape, pos, orig,
-                                        nbr, ncnt, status, overflow_count);
-                }
-                __syncwarp();
+        // A bucket of the bricked order is one cell.  In the linear order a cell on the grid's
+        // inclusive upper face shares its bucket with another cell: one round per cell then.
+        for (unsigned left = (1u << m) - 1u; left;) {
+            bool mine = kr < m;
+            if (gg.brick) {
+                left = 0;
+            } else {
+                const int3 c = cell_of(q.x, q.y, q.z, gg, sc.cell);
+                const int f = __ffs((int)left) - 1;
+                c0 = make_int3(__shfl_sync(kAll, c.x, f), __shfl_sync(kAll, c.y, f), __shfl_sync(kAll, c.z, f));
+                mine = ((left >> kr) & 1u) && c.x == c0.x && c.y == c0.y && c.z == c0.z;
+                left &= ~__ballot_sync(kAll, mine);
             }
+            CellRuns runs{};
+            if (lane < 27u) runs = runs_at(c0, (int)lane, gg, fstart, bstart);
+            const uint32_t total = place_runs(runs);
+            const ListOut out{shape, nbr, row - row0, cap};
+            const uint32_t found = cell_rows<MODE, R>(S, runs, total, mine, q, d2max, pos, orig, out);
+            if (mine && lane < R) {
+                ncnt[row - row0] = min(found, cap) + 1u;
+                if (found > cap) {
+                    atomicAdd(overflow_count, 1u);
+                    atomicOr(status, ST_BOUNDS);
+                }
+            }
+            __syncwarp();
         }
     }
-}
-
-// List builder for few rows: a warp takes four consecutive rows, whatever cells they lie in, eight
-// lanes each.  The candidates of a cell are laid out by every warp that has rows of it, but no warp
-// works through more than its own rows, and there are twice as many warps: the kernel's time is
-// then one short chain.  Event-timed (B200, us), a warp per cell -> this: DFSPH 2,000 rows 17.0 ->
-// 14.7, 8,000 rows 20.5 -> 16.7, 16,000 rows 20.6 -> 17.2, 32,000 rows 22.9 -> 28.8; PBF 8,000 rows
-// 12.3 -> 11.2, 16,000 rows 13.4 -> 13.5.
-constexpr uint32_t kFewRows = 16384;
-constexpr uint32_t kFewScan = 4;
-template <int MODE>
-__global__ void __launch_bounds__(kCellWarps * 32, 7) k_build_lists_few(
-    Scenes sc, uint32_t row0, uint32_t cnt, ListShape shape, const float4 *__restrict__ pos,
-    const uint32_t *__restrict__ orig, const uint32_t *__restrict__ fstart, const uint32_t *__restrict__ bstart,
-    uint32_t *__restrict__ nbr, uint32_t *__restrict__ ncnt, uint32_t *__restrict__ status,
-    uint32_t *__restrict__ overflow_count) {
-    pdl_enter();
-    __shared__ __align__(16) CellScratch scratch[kCellWarps];
-    constexpr unsigned kAll = 0xffffffffu;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t first = (blockIdx.x * kCellWarps + (threadIdx.x >> 5)) * kFewScan;
-    if (first >= cnt) return;
-    CellScratch &S = scratch[threadIdx.x >> 5];
-    const int3 o = nbr_offset((int)min(lane, 26u));
-    const uint32_t n = min(kFewScan, cnt - first), k = lane % kFewScan;
-    const uint32_t row = row0 + first + min(k, n - 1u);
-    const SceneGrid mine_g = load_scene(sc, row);
-    const float4 p = pos[row];
-    const int3 c = cell_of(p.x, p.y, p.z, mine_g, sc.cell);
-    const bool inside = cell_available(c, mine_g);
-    if (lane < n && !inside) ncnt[first + lane] = 0;   // outside the grid: no neighbours, not even self
-    // one round per cell among the rows
-    for (unsigned left = __ballot_sync(kAll, lane < n && inside); left;) {
-        const int f = __ffs((int)left) - 1;
-        const int3 c0 = make_int3(__shfl_sync(kAll, c.x, f), __shfl_sync(kAll, c.y, f), __shfl_sync(kAll, c.z, f));
-        const uint32_t scene = __shfl_sync(kAll, mine_g.key_base, f);
-        const bool mine = ((left >> k) & 1u) && c.x == c0.x && c.y == c0.y && c.z == c0.z && mine_g.key_base == scene;
-        left &= ~__ballot_sync(kAll, mine);
-        const SceneGrid g = load_scene(sc, row0 + first + (uint32_t)f);
-        CellRuns runs{};
-        const int3 cc = make_int3(c0.x + o.x, c0.y + o.y, c0.z + o.z);
-        if (lane < 27u && cell_available(cc, g)) {
-            const uint32_t b = g.key_base + cell_key(cc, g);
-            runs.f0 = __ldg(fstart + b); runs.f1 = __ldg(fstart + b + 1);
-            runs.b0 = __ldg(bstart + b); runs.b1 = __ldg(bstart + b + 1);
-        }
-        const uint32_t len = (runs.f1 - runs.f0) + (runs.b1 - runs.b0);
-        uint32_t incl = len;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(kAll, incl, d);
-            if ((int)lane >= d) incl += y;
-        }
-        runs.excl = incl - len;
-        const uint32_t total = __shfl_sync(kAll, incl, 31);
-        cell_lists<MODE, kFewScan>(S, runs, total, mine, row, row0, p, sc.d2max, sc.maxnbr - 1u, shape, pos, orig, nbr,
-                                   ncnt, status, overflow_count);
-        __syncwarp();
-    }
+    walk_rows<MODE>(
+        S, __ballot_sync(kAll, walked && lane < SCAN), d2max, pos, orig,
+        [&](uint32_t l) {
+            WalkedRow r;
+            r.i = __shfl_sync(kAll, i, (int)l);
+            r.p = make_float4(__shfl_sync(kAll, p.x, (int)l), __shfl_sync(kAll, p.y, (int)l),
+                              __shfl_sync(kAll, p.z, (int)l), 0.f);
+            r.c = make_int3(__shfl_sync(kAll, own.x, (int)l), __shfl_sync(kAll, own.y, (int)l),
+                            __shfl_sync(kAll, own.z, (int)l));
+            r.g = load_scene(sc, r.i);
+            r.fstart = fstart;
+            r.bstart = bstart;
+            r.out = ListOut{shape, nbr, r.i - row0, cap};
+            return r;
+        },
+        [&](const WalkedRow &r, uint32_t found, bool lead) {
+            if (!lead) return;
+            ncnt[r.i - row0] = min(found, cap) + 1u;
+            if (found > cap) {
+                atomicAdd(overflow_count, 1u);
+                atomicOr(status, ST_BOUNDS);
+            }
+        });
 }
 
 #ifdef VTP_CHECKED
@@ -1160,7 +1026,7 @@ void ugns_build_lists(cudaStream_t st, const Scenes &sc, const Layout &L, uint32
     using M2 = std::integral_constant<int, 2>;
     // Lists of either builder are the same; a thread per row writes shape lg 0 well (its stores of
     // one entry index share a line), so it takes the large solvers, whose lists have that shape.
-    if (cnt > kWalkRows && L.shape.lg == 0) {
+    if (cnt > kScan8Rows && L.shape.lg == 0) {
         auto walk = [&](auto mode, auto cull) {
             constexpr int M = decltype(mode)::value;
             constexpr bool C = decltype(cull)::value;
@@ -1174,25 +1040,20 @@ void ugns_build_lists(cudaStream_t st, const Scenes &sc, const Layout &L, uint32
             case 1: L.cell_cull ? walk(M1{}, T) : walk(M1{}, F); break;
             default: L.cell_cull ? walk(M2{}, T) : walk(M2{}, F); break;
         }
-    } else if (cnt <= kFewRows) {
-        auto few = [&](auto mode) {
-            launch(k_build_lists_few<decltype(mode)::value>, nblk(cnt, kCellWarps * kFewScan), kCellWarps * 32, 0, st,
-                   sc, row0, cnt, L.shape, pos, orig, u.fstart, u.bstart, nbr, ncnt, status, overflow);
-        };
-        switch (L.merge_mode) {
-            case 0: few(M0{}); break;
-            case 1: few(M1{}); break;
-            default: few(M2{}); break;
-        }
     } else {
-        auto cells = [&](auto mode) {
-            launch(k_build_lists<decltype(mode)::value>, nblk(cnt, kCellWarps * kCellScan), kCellWarps * 32, 0, st, sc,
+        auto cells = [&](auto mode, auto scan) {
+            constexpr uint32_t SCAN = decltype(scan)::value;
+            launch(k_build_lists<decltype(mode)::value, SCAN>, nblk(cnt, kCellWarps * SCAN), kCellWarps * 32, 0, st, sc,
                    row0, cnt, L.shape, pos, orig, start, u.fstart, u.bstart, nbr, ncnt, status, overflow);
         };
+        auto build = [&](auto mode) {
+            if (cnt <= kScan4Rows) cells(mode, std::integral_constant<uint32_t, 4>{});
+            else cells(mode, std::integral_constant<uint32_t, 8>{});
+        };
         switch (L.merge_mode) {
-            case 0: cells(M0{}); break;
-            case 1: cells(M1{}); break;
-            default: cells(M2{}); break;
+            case 0: build(M0{}); break;
+            case 1: build(M1{}); break;
+            default: build(M2{}); break;
         }
     }
 #ifdef VTP_CHECKED
