@@ -110,3 +110,14 @@ def test_a_sparse_cloud_costs_no_more_than_a_fluid(vtp_gpu, n):
     spray, spray_size = _cloud(n, 1.0)
     assert _noalloc(vtp_gpu, spray, spray_size, 60, 6)[2] <= _noalloc(vtp_gpu, fluid, fluid_size, 60, 6)[2]
     assert _build_ms(vtp_gpu, _scene(spray, spray_size)) <= _build_ms(vtp_gpu, _scene(fluid, fluid_size))
+
+
+def test_a_crowded_cell_of_interleaved_objects_merges_its_runs_once(vtp_gpu):
+    """Fluid and wall particles of one cell whose attach ids interleave are merged by id.  A binary
+    search per candidate looks 13 times at 4,000 + 4,000 particles, against 8 instructions for each
+    row that tests the candidate; a merge that starts again for each 320 candidates looks 4,000 times."""
+    p, size = _cloud(30000, 0.5, 4000)
+    walls = _cloud(30000, 0.5, 4000, seed=1)[0]
+    after = _scene(p, size)
+    after.objects.append(scenes.SceneObject("wall", walls, 1))
+    assert _build_ms(vtp_gpu, _scene(p, size, walls)) <= 2 * _build_ms(vtp_gpu, after)

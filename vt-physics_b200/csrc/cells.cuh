@@ -86,27 +86,66 @@ __device__ __forceinline__ uint32_t place_runs(CellRuns &r) {
     return __shfl_sync(kAll, incl, 31);
 }
 
+// How many of the first o candidates of a cell merged by id are fluid rows: the merge path's crossing
+// of diagonal o.
+__device__ __forceinline__ uint32_t merge_split(const CellRuns &R, uint32_t o, const uint32_t *__restrict__ orig) {
+    const uint32_t nf = R.f1 - R.f0, nb = R.b1 - R.b0;
+    uint32_t lo = o > nb ? o - nb : 0u, hi = min(o, nf);
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (__ldg(orig + R.f0 + mid) < __ldg(orig + R.b0 + (o - mid - 1u))) lo = mid + 1u;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// Candidates [o, end) of a cell in list order into cand[0 .. end - o).
+template <int MODE>
+__device__ __forceinline__ void lay_out(uint32_t *cand, const CellRuns &R, uint32_t o, uint32_t end, uint32_t split,
+                                        const uint32_t *__restrict__ orig) {
+    if (MODE == 2) {
+        uint32_t f = R.f0 + split, b = R.b0 + (o - split);
+        for (; o < end; ++o) *cand++ = merge_next(f, R.f1, b, R.b1, orig);
+    } else {
+        const uint32_t a0 = MODE == 0 ? R.f0 : R.b0, na = (MODE == 0 ? R.f1 : R.b1) - a0;
+        const uint32_t c0 = (MODE == 0 ? R.b0 : R.f0) - na;
+        for (; o < end; ++o) *cand++ = (o < na ? a0 : c0) + o;
+    }
+}
+
+// Runs longer than this are laid out by the whole warp, others by the lane that holds them (B200, us:
+// 30,000 rows with 10,000 in one cell 578 -> 450, with 3,000 and 3,000 interleaved wall particles 887 ->
+// 203; a fluid at rest has runs of eight, the same time).
+constexpr uint32_t kLongRun = 32;
+
 // Lays candidates [wb, wb + wl) out: rows (their ids from pos.w with IDS) and positions, infinity
 // from wl up to `padded`.
 template <int MODE, bool IDS>
 __device__ __forceinline__ void stage_candidates(CellScratch &S, const CellRuns &R, uint32_t wb, uint32_t wl,
                                                  uint32_t padded, const float4 *__restrict__ pos,
                                                  const uint32_t *__restrict__ orig) {
+    constexpr unsigned kAll = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t nf = R.f1 - R.f0, nb = R.b1 - R.b0, len = nf + nb;
+    const uint32_t len = (R.f1 - R.f0) + (R.b1 - R.b0);
+    // the part of this lane's runs that lies in the window
+    const uint32_t o0 = wb > R.excl ? min(wb - R.excl, len) : 0u;
+    const uint32_t o1 = wb + wl > R.excl ? min(wb + wl - R.excl, len) : 0u;
     __syncwarp();
-    if (MODE == 2) {
-        uint32_t fi = R.f0, bi = R.b0;
-        for (uint32_t o = 0; o < len; ++o) {
-            const uint32_t j = merge_next(fi, R.f1, bi, R.b1, orig);
-            if (R.excl + o - wb < wl) S.cand[R.excl + o - wb] = j;
-        }
-    } else {
-        // the part of this lane's runs that lies in the window
-        const uint32_t na = MODE == 0 ? nf : nb, a0 = MODE == 0 ? R.f0 : R.b0, c0 = (MODE == 0 ? R.b0 : R.f0) - na;
-        const uint32_t o0 = wb > R.excl ? min(wb - R.excl, len) : 0u;
-        const uint32_t o1 = wb + wl > R.excl ? min(wb + wl - R.excl, len) : 0u;
-        for (uint32_t o = o0; o < o1; ++o) S.cand[R.excl + o - wb] = (o < na ? a0 : c0) + o;
+    if (len <= kLongRun && o0 < o1)
+        lay_out<MODE>(S.cand + (R.excl + o0 - wb), R, o0, o1, MODE == 2 ? merge_split(R, o0, orig) : 0u, orig);
+    for (unsigned todo = __ballot_sync(kAll, len > kLongRun && o0 < o1); todo; todo &= todo - 1u) {
+        const int src = __ffs((int)todo) - 1;
+        CellRuns r;
+        r.f0 = __shfl_sync(kAll, R.f0, src);
+        r.f1 = __shfl_sync(kAll, R.f1, src);
+        r.b0 = __shfl_sync(kAll, R.b0, src);
+        r.b1 = __shfl_sync(kAll, R.b1, src);
+        r.excl = __shfl_sync(kAll, R.excl, src);
+        const uint32_t beg = __shfl_sync(kAll, o0, src), end = __shfl_sync(kAll, o1, src);
+        const uint32_t each = (end - beg + 31u) / 32u, o = min(beg + lane * each, end);   // a lane's share of it
+        if (o < end)
+            lay_out<MODE>(S.cand + (r.excl + o - wb), r, o, min(o + each, end),
+                          MODE == 2 ? merge_split(r, o, orig) : 0u, orig);
     }
     __syncwarp();
     for (uint32_t q = lane; q < padded; q += 32u) {
