@@ -164,8 +164,8 @@ __device__ __forceinline__ void stage_candidates(CellScratch &S, const CellRuns 
 
 // Appends `off` to the lane's accepted candidates at shared address `to` if 0 < d2 <= d2max
 // (`0 < |x_i - x_j|` also drops the row itself): predicated, no branch.  The asm names no memory
-// clobber, so that the next candidates' loads are not held up by it: what it stores is read only
-// after a warp barrier.
+// clobber, so that the next candidates' loads are not held up by it; kept_done() after the last of
+// them tells the compiler of the stores.
 __device__ __forceinline__ void keep_candidate(uint32_t &to, uint32_t off, float d2, float d2max) {
     asm(
         "{\n\t.reg .pred p;\n\t"
@@ -176,6 +176,9 @@ __device__ __forceinline__ void keep_candidate(uint32_t &to, uint32_t off, float
         : "+r"(to)
         : "r"(off), "f"(d2), "f"(d2max));
 }
+
+// What keep_candidate stored may be read from here on.
+__device__ __forceinline__ void kept_done() { asm volatile("" ::: "memory"); }
 
 // Tests the 4 candidates at index `at` (offset `off` of the lane's share) against -p = (px, py, pz).
 __device__ __forceinline__ void test4(const CellScratch &S, uint32_t at, uint32_t off, uint32_t &to, uint64_t px,
@@ -216,6 +219,7 @@ __device__ __forceinline__ uint32_t cell_rows(CellScratch &S, const CellRuns &ru
             test4(S, h * share + off, off, to, px, py, pz, d2max);
             test4(S, h * share + off + 4u, off + 4u, to, px, py, pz, d2max);
         }
+        kept_done();
         const uint32_t mine = live ? to - to0 : 0u;
         uint32_t x = mine;
 #pragma unroll
