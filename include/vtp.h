@@ -152,8 +152,9 @@ VTP_API int vtp_solver_create(int solver_type, vtp_solver **out);
  *       49,152 fluid rows, by a team of lanes with the same bits; 4 or 8 =
  *       the row's entries split over lanes and their sums added by a shuffle
  *       butterfly);
- *   "listLanes": 0 (default), 1 or 8; accepted, the list builder is chosen by
- *       row count and every one writes the same lists;
+ *   "listLanes": the list builder (0 = by row count, default; 1 = a thread
+ *       per row; 8 = rows of a cell together, four or eight lanes a row); every
+ *       setting writes the same lists;
  *   "cubicCube": "rounded" (default) takes the (1 - q)^3 of the cubic
  *       kernel's outer branch correctly rounded, at most one ulp from the
  *       reference's powf(1 - q, 3) (KernelFunctions.cuh:29); "powf" calls powf

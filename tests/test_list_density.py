@@ -121,3 +121,38 @@ def test_a_crowded_cell_of_interleaved_objects_merges_its_runs_once(vtp_gpu):
     after = _scene(p, size)
     after.objects.append(scenes.SceneObject("wall", walls, 1))
     assert _build_ms(vtp_gpu, _scene(p, size, walls)) <= 2 * _build_ms(vtp_gpu, after)
+
+
+@pytest.mark.parametrize("kind", ["PBF", "IMM"])   # lists of both shapes at this size
+def test_list_lanes_choose_the_builder(vtp_gpu, kind):
+    """"listLanes": a thread per row (1), rows of a cell together (8), by row count (0)."""
+    import torch
+    sc = _scene(*_cloud(3000, 0.5)) if kind == "PBF" else scenes.layered_mixture("IMM", 14, seed=3)
+    used = []
+    for lanes in (0, 1, 8):
+        s = vtp_gpu.solver_from_scene(sc, extra={"listLanes": lanes})
+        assert s.initialize(), s.last_error
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            s.get_neighbors(60)
+            torch.cuda.synchronize()
+        names = [e.key for e in prof.key_averages()]
+        used.append({b for b in ("k_walk_lists", "k_build_lists") if any(b in n for n in names)})
+        s.destroy()
+    assert used == [{"k_build_lists"}, {"k_walk_lists"}, {"k_build_lists"}]
+
+
+@pytest.mark.parametrize("cull", [False, True])
+@pytest.mark.parametrize("attach", ["after", "before", "between"])
+@pytest.mark.parametrize("n", [3000, 131073])
+def test_a_thread_per_row_matches_the_oracle(vtp_gpu, oracle_lib, n, attach, cull):
+    """Every order of a cell's two runs, with and without cell culling, in lists of both shapes."""
+    p, size = _cloud(n, 0.5, 100, seed=2)
+    wall = scenes.SceneObject("wall", _cloud(n // 8, 0.6, 50, seed=3)[0], 1)
+    sc = _scene(p, size)
+    sc.objects.insert({"after": 2, "before": 0, "between": 1}[attach], wall)
+    s = vtp_gpu.solver_from_scene(sc, extra={"listLanes": 1, "cellCull": cull})
+    assert s.initialize(), s.last_error
+    want = oracle_lib.neighbors(s.get_field("pos"), oracle_lib.make_grid(sc.config["PBF"]["Required"]))
+    cnt, nbr = s.get_neighbors(60)
+    s.destroy()
+    assert np.array_equal(cnt, want[0]) and np.array_equal(nbr, want[1])

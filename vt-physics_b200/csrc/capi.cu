@@ -173,7 +173,7 @@ int vtp_solver::parse_config(const json &c) {
         force_div = force_inc = 0;
         force_seq.clear();
         device_loop = true; use_graphs = true; stage_timers = false; stop_on_crash = true;
-        block = 128; unroll = 4; persistent_tiles = false; cube_powf = false; row_lanes = 1;
+        block = 128; unroll = 4; persistent_tiles = false; cube_powf = false; list_lanes = 0; row_lanes = 1;
         cell_cull = false; staged_solve = false; stage_rows = 2048; tape_budget_mb = 8192; adj_lanes = 0;
         cfl = 0.f;
         cell_order_brick = true;
@@ -219,10 +219,9 @@ int vtp_solver::parse_config(const json &c) {
             stage_rows = b.value("stageRows", 2048);
             if (stage_rows < 256 || stage_rows > (int)vtp::kStageMaxRows)
                 return fail(VTP_ERR_CONFIG, "stageRows must be in [256, 32767]");
-            // One builder serves every row count; the key keeps its values and the lists never depended on it.
-            const int list_lanes = b.value("listLanes", 0);
+            list_lanes = b.value("listLanes", 0);
             if (list_lanes != 0 && list_lanes != 1 && list_lanes != 8)
-                return fail(VTP_ERR_CONFIG, "listLanes must be 0, 1 or 8");
+                return fail(VTP_ERR_CONFIG, "listLanes must be 0 (by row count), 1 or 8");
             const std::string cube = b.value("cubicCube", std::string("rounded"));
             if (cube != "rounded" && cube != "powf")
                 return fail(VTP_ERR_CONFIG, "cubicCube must be \"rounded\" or \"powf\"");
@@ -477,6 +476,7 @@ int vtp_solver::initialize() {
         mode = mode < 0 ? m : (mode == m ? m : 2);
     }
     L.merge_mode = mode < 0 ? 0 : mode;
+    L.list_lanes = list_lanes;
     L.cell_cull = cell_cull;
     teams = persistent_tiles || (type != VTP_SOLVER_DFSPH && type != VTP_SOLVER_PBF) ? 0
             : L.nf <= vtp::kTeam8MaxRows                                             ? 8

@@ -48,7 +48,8 @@ struct Layout {
     uint32_t n = 0, nf = 0, nb = 0;
     ListShape shape;           // neighbour-list storage (maxnbr - 1 entries per row)
     int merge_mode = 0;        // 0: fluid ids < boundary ids, 1: boundary ids < fluid ids, 2: general
-    bool cell_cull = false;    // the walking list builders skip neighbour cells beyond h of the row (same lists)
+    int list_lanes = 0;        // list builder: 0 by row count, 1 a thread per row, 8 groups of rows (same lists)
+    bool cell_cull = false;    // the builders with a thread per row skip neighbour cells beyond h of the row (same lists)
 };
 
 // Neighbour-search working set (one per solver).

@@ -108,7 +108,8 @@ struct vtp_solver {
     bool pdl = true;                // programmatic dependent launch between the substep's kernels
     int row_lanes = 1;        // threads per row of the PBF neighbour passes (1, 4, 8)
     int teams = 0;            // lanes of the team that walks a row (team.cuh), by row count; 0: a thread per row
-    bool cell_cull = false;   // list builder skips neighbour cells beyond h (same lists)
+    int list_lanes = 0;       // list builder: 0 by row count, 1 a thread per row, 8 groups of rows (same lists)
+    bool cell_cull = false;   // the builder with a thread per row skips neighbour cells beyond h (same lists)
     bool staged_solve = false;      // DFSPH pressure solve gathers from shared-memory cell-group copies
     uint32_t tape_budget_mb = 8192;  // differentiable PBF / DFSPH: device memory for resident segment tapes
     int adj_lanes = 0;              // differentiable PBF: lanes per row of the adjoint's neighbour passes (0: by rows)

@@ -388,7 +388,7 @@ struct Walker {
 // against a warp per cell and against k_build_lists with 32 rows a warp: a dam break at rest 74 (70,
 // 64), after 150 substeps 101 (119, 124), clouds 0.35, 0.5, 0.7 and 1 cells apart 229 (348, 235), 98
 // (117, 104), 76 (125, 111), 44 (191, 51), with 4,000 rows in one cell 390 (8,230, 740).
-template <int MODE, bool CULL>
+template <int MODE, bool CULL, class Slots>
 __global__ void k_walk_lists(Scenes sc, uint32_t row0, uint32_t cnt, ListShape shape,
                               const float4 *__restrict__ pos, const uint32_t *__restrict__ orig,
                               const uint32_t *__restrict__ fstart, const uint32_t *__restrict__ bstart,
@@ -405,12 +405,13 @@ __global__ void k_walk_lists(Scenes sc, uint32_t row0, uint32_t cnt, ListShape s
         ncnt[r] = 0;
         return;
     }
-    Walker<RowSlots> w;
+    Walker<Slots> w;
     w.px = p.x; w.py = p.y; w.pz = p.z;
     w.self = i;
     w.cnt = 1;
     w.maxnbr = sc.maxnbr;
-    w.out = nbr + row_index(r, shape);
+    if constexpr (std::is_same_v<Slots, AnySlots>) w.at = AnySlots{shape};
+    w.out = nbr + ell_index(r, 0, shape);
     w.overflow = false;
     const float d2max = sc.d2max;
     FaceGaps fg;
@@ -1026,12 +1027,16 @@ void ugns_build_lists(cudaStream_t st, const Scenes &sc, const Layout &L, uint32
     using M2 = std::integral_constant<int, 2>;
     // Lists of either builder are the same; a thread per row writes shape lg 0 well (its stores of
     // one entry index share a line), so it takes the large solvers, whose lists have that shape.
-    if (cnt > kScan8Rows && L.shape.lg == 0) {
-        auto walk = [&](auto mode, auto cull) {
+    if (L.list_lanes == 1 || (L.list_lanes == 0 && cnt > kScan8Rows && L.shape.lg == 0)) {
+        auto walk_as = [&](auto mode, auto cull, auto slots) {
             constexpr int M = decltype(mode)::value;
             constexpr bool C = decltype(cull)::value;
-            launch(k_walk_lists<M, C>, nblk(cnt, kWalkBlock), kWalkBlock, 0, st, sc, row0, cnt, L.shape, pos, orig,
-                   u.fstart, u.bstart, nbr, ncnt, status, overflow);
+            launch(k_walk_lists<M, C, decltype(slots)>, nblk(cnt, kWalkBlock), kWalkBlock, 0, st, sc, row0, cnt,
+                   L.shape, pos, orig, u.fstart, u.bstart, nbr, ncnt, status, overflow);
+        };
+        auto walk = [&](auto mode, auto cull) {
+            if (L.shape.lg == 0) walk_as(mode, cull, RowSlots{});
+            else walk_as(mode, cull, AnySlots{});
         };
         const std::true_type T;
         const std::false_type F;
