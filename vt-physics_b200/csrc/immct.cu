@@ -111,8 +111,8 @@ struct ImmState {
     uint32_t bodies_seen = 0;        // counter[5] at the last launch count
     float4 *tpk = nullptr;
     float4 *pk2 = nullptr;           // [2 nf] packed gather rows (viscosity -> tension / conformation)
-    float *bfrac_dev = nullptr;      // the same on the device (allocated by the first read of the fractions)
-    std::vector<float> bfrac;        // boundary rows' phase fractions in attach order (host)
+    std::vector<float> bfrac;        // every particle's phase fractions as attached (host)
+    float *bfrac_dev = nullptr;      // the same on the device; null: no room for them
     cudaGraphConditionalHandle cond{};
 };
 
@@ -958,6 +958,9 @@ int immct_init(vtp_solver &s) {
             CUI(cudaMemcpyAsync(m.Q[c].b[b], vtp::sym_diag(c) ? one.data() : zero.data(), nf * sizeof(float),
                                 cudaMemcpyHostToDevice, s.st));
     m.bfrac.assign(s.hphase.begin(), s.hphase.end());
+    m.bfrac_dev = s.alloc_spare<float>(m.bfrac.size());
+    if (m.bfrac_dev)
+        CUI(cudaMemcpyAsync(m.bfrac_dev, m.bfrac.data(), m.bfrac.size() * sizeof(float), cudaMemcpyHostToDevice, s.st));
     m.have_tension = s.gamma != 0.f;
     // Both buffers hold the initial state; from here on the phase arrays swap in
     // lockstep with the row order (one swap per substep sort).
@@ -1145,21 +1148,14 @@ int immct_enqueue_tick(vtp_solver &s, cudaStream_t st, bool capture) {
     return VTP_OK;
 }
 
-// Phase fractions of every particle in attach order: the boundary's are the attached ones, kept on
-// the device from the first read on (copied from the host each time where there is no room for
-// them), and the fluid rows are scattered over them.  500k fluid rows, two substeps and a read of
-// positions, velocities and fractions: 7.0 ms with the fractions put in order on the host, 3.9 here.
+// Phase fractions of every particle in attach order: the attached ones, kept on the device (copied
+// from the host where there is no room for them), stay the boundary's, and the fluid rows are
+// scattered over them.  500k fluid rows, two substeps and a read of positions, velocities and
+// fractions: 7.0 ms with the fractions put in order on the host, 3.9 here.
 static int imm_fractions(vtp_solver &s, float *dev_out) {
     ImmState &m = *s.imm;
-    const size_t bytes = m.bfrac.size() * sizeof(float);
-    if (!m.bfrac_dev) {
-        if (s.alloc(&m.bfrac_dev, m.bfrac.size()) == VTP_OK)
-            CUI(cudaMemcpyAsync(m.bfrac_dev, m.bfrac.data(), bytes, cudaMemcpyHostToDevice, s.st));
-        else
-            cudaGetLastError();   // no room: m.bfrac_dev stays null
-    }
     const float *all = m.bfrac_dev ? m.bfrac_dev : m.bfrac.data();
-    CUI(cudaMemcpyAsync(dev_out, all, bytes, cudaMemcpyDefault, s.st));
+    CUI(cudaMemcpyAsync(dev_out, all, m.bfrac.size() * sizeof(float), cudaMemcpyDefault, s.st));
     if (s.L.nf) vtp::k_fractions<<<vtp::nblk(s.L.nf, 256), 256, 0, s.st>>>(imm_args(s), s.orig.c(), dev_out);
     CUI(cudaGetLastError());
     CUI(cudaStreamSynchronize(s.st));

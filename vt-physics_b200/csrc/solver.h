@@ -1,6 +1,7 @@
 // The solver object behind the C ABI handle (shared by capi.cu and immct.cu).
 #pragma once
 
+#include <algorithm>
 #include <functional>
 #include <memory>
 #include <string>
@@ -234,6 +235,22 @@ struct vtp_solver {
         if (e != cudaSuccess) return vtp::fail(VTP_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
         allocs.push_back(*p);
         return VTP_OK;
+    }
+
+    // Memory that only saves time: null where it would leave little for what is allocated later
+    // (graphs, staging buffers).
+    template <class T>
+    T *alloc_spare(size_t count) {
+        constexpr size_t kLeft = 256u << 20;
+        size_t free_bytes = 0, total = 0;
+        void *p = nullptr;
+        if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || free_bytes < count * sizeof(T) + kLeft ||
+            cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        allocs.push_back(p);
+        return static_cast<T *>(p);
     }
 
     int parse_config(const nlohmann::json &c);
