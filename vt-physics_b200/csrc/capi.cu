@@ -482,8 +482,8 @@ int vtp_solver::initialize() {
             : L.nf <= vtp::kTeam8MaxRows                                             ? 8
             : L.nf <= vtp::kTeamMaxRows                                              ? 4
                                                                                      : 0;
-    L.shape.stride = vtp::list_stride(maxnbr > 1 ? maxnbr - 1 : 1);
     L.shape.lg = teams ? vtp::kTeamListLg : 0u;
+    L.shape.stride = vtp::list_stride(maxnbr > 1 ? maxnbr - 1 : 1, L.shape.lg);
 
     // Grids as UniformGirdNeighborSearcher::setConfig (UniformGridNeighborSearch.cpp:214-218),
     // one per scene, each followed by its own outside bucket.
@@ -621,8 +621,6 @@ int vtp_solver::initialize() {
     } else {
         for (int k = 0; k < 2; ++k) AL(&vadv.b[k], n);
         AL(&pva, 2 * (size_t)n);
-        pva2 = pva;
-        if (type == VTP_SOLVER_DFSPH) { AL(&pva2, 2 * (size_t)n); }
         AL(&pk, n);
         AL(&ratio, L.nf);
         AL(&alpha, L.nf);
@@ -714,6 +712,11 @@ int vtp_solver::initialize() {
         AL(&partials, npart * nobj_max + 1);
         if (type != VTP_SOLVER_DFSPH) {
             if ((rc = immct_alloc(*this))) return rc;
+        }
+        pva2 = pva;
+        if (type == VTP_SOLVER_DFSPH && !one_pva) {
+            float4 *p = alloc_spare<float4>(2 * (size_t)n);
+            if (p) pva2 = p;
         }
     }
     // Neighbour search of the initial state (initialize(): m_neighborSearcher.update(pos)),
@@ -903,9 +906,9 @@ int vtp_solver::enqueue_tick(cudaStream_t s, bool capture) {
         PROF(this, "ugns_lists", vtp::ugns_build_lists(s, scn(), L, 0, L.nf, pos.c(), orig.c(), u, u.nbr, u.ncnt,
                                                        d_status, d_overflow));
     }
-    // The ratio / alpha pass packs the divergence solve's rows and starts both solves, the forces
-    // pass packs the density solve's.
-    const bool packed = L.nf > 0;
+    // The ratio / alpha pass packs the divergence solve's rows and starts both solves; the forces
+    // pass, which reads those rows, packs the density solve's where they have an array of their own.
+    const bool packed = L.nf > 0, two = pva2 != pva;
     vtp::DfsphArgs ra = dfsph_args();
     ra.pack = pva;
     ra.reset = solve;
@@ -915,7 +918,7 @@ int vtp_solver::enqueue_tick(cudaStream_t s, bool capture) {
     launches_per_tick += vtp::ugns_sort_launches(nbuckets) + 2;  // sort, lists, ratio / alpha
     if ((rc = enqueue_solve(s, 0, capture, packed))) return rc;
     vtp::DfsphArgs a = dfsph_args();
-    a.pack = pva2;
+    a.pack = two ? pva2 : nullptr;
     PROF(this, "dfsph_pressure_pack", vtp::dfsph_pressure_pack(s, a));
     launches_per_tick += 1;
     if (gamma == 0.f) {
@@ -928,7 +931,7 @@ int vtp_solver::enqueue_tick(cudaStream_t s, bool capture) {
         launches_per_tick += 2;
     }
     vel.swap(); vadv.swap();
-    if ((rc = enqueue_solve(s, 1, capture, packed))) return rc;
+    if ((rc = enqueue_solve(s, 1, capture, packed && two))) return rc;
     PROF(this, "dfsph_finalize", vtp::dfsph_finalize(s, dfsph_args()));
     launches_per_tick += 1;
     return VTP_OK;

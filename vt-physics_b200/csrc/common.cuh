@@ -169,12 +169,12 @@ __device__ __forceinline__ int3 nbr_offset(int t) {
 // 32 / 2^lg consecutive rows.  lg 0 for passes with a thread per row (a warp reads entry t of its
 // 32 rows from one line); lg 3 for passes with a team of lanes per row (a team reads consecutive
 // entries of its row, a warp's 8 rows read two lines).  The stride (entries a row has room for) is
-// a multiple of 8.
+// a multiple of 2^lg.
 struct ListShape {
     uint32_t stride = 0, lg = 0;
 };
 constexpr uint32_t kTeamListLg = 3;
-inline uint32_t list_stride(uint32_t entries) { return (entries + 7u) / 8u * 8u; }
+inline uint32_t list_stride(uint32_t entries, uint32_t lg) { return (entries + (1u << lg) - 1u) >> lg << lg; }
 // Offset of entry t from the row's first entry.
 __device__ __forceinline__ uint32_t ell_slot(uint32_t t, ListShape s) {
     return ((t >> s.lg) << 5) | (t & ((1u << s.lg) - 1u));

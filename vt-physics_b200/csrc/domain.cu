@@ -479,10 +479,10 @@ int vtp_domain_create(const char *config_json, const float *fluid_pos, uint32_t 
         if (mode == 1 && nb && (rc = vtp_solver_attach_object(d->s, boundary_pos, nb, nullptr, bj.c_str()))) return rc;
         if ((rc = vtp_solver_attach_object(d->s, fl.data(), capacity, nullptr, fj.c_str()))) return rc;
         if (mode == 0 && nb && (rc = vtp_solver_attach_object(d->s, boundary_pos, nb, nullptr, bj.c_str()))) return rc;
+        d->s->one_pva = true;   // the peers store into the packed rows, and each solve packs them anew
         if ((rc = vtp_solver_initialize(d->s))) return rc;
         vtp_solver *s = d->s;
         if (s->L.nf != capacity || s->L.nb != nb) return fail(VTP_ERR_STATE, "domain worker layout");
-        s->pva2 = s->pva;   // one set of packed rows: the peers store into it, and each solve packs it anew
         d->st = s->st;
         CU(cudaMallocHost((void **)&d->h_status, 2 * sizeof(uint32_t)));
         if ((rc = d->alloc(&d->status, 1))) return rc;

@@ -146,7 +146,9 @@ struct vtp_solver {
     float *ratio = nullptr, *alpha = nullptr, *kappa = nullptr, *delta = nullptr, *rest_b = nullptr;
     float4 *acc_tmp = nullptr, *normal = nullptr;
     float4 *pva = nullptr, *pk = nullptr;   // packed gather rows of the pressure solves
-    float4 *pva2 = nullptr;                 // DFSPH: the density solve's own pva (the forces pass fills it); else pva
+    float4 *pva2 = nullptr;                 // DFSPH: the density solve's own pva (the forces pass fills it), where
+                                            // there is room for one; else pva
+    bool one_pva = false;                   // a slab's worker: no second one
     double *partials = nullptr, *inv_count = nullptr;
     uint16_t *obj_of = nullptr;
     vtp::SolveState *solve = nullptr;   // [2][S]: divergence, density per scene
