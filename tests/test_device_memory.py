@@ -101,3 +101,20 @@ def test_a_slab_worker_holds_one_array_of_packed_rows(vtp_gpu):
     d.close()
     own = (4 * 4 + 4 + 1 + 4 + 8 * 4) * n
     assert taken <= solver - 32 * n + own + 8 * PAGE
+
+
+def test_a_solver_that_does_not_fit_leaves_the_next_one_alone(vtp_gpu):
+    import torch
+    sc = _fluid("PBF", 1_000_000)
+    taken = _taken(vtp_gpu, sc)
+    torch.cuda.empty_cache()
+    filler = torch.empty(_free() - taken // 2, dtype=torch.uint8, device="cuda")
+    s = vtp_gpu.solver_from_scene(sc)
+    with pytest.raises(vtp_gpu.VtpError, match="out of device memory"):
+        s.initialize()
+    s.destroy()
+    del filler
+    torch.cuda.empty_cache()
+    small = vtp_gpu.solver_from_scene(_fluid("PBF", 1000))
+    assert small.initialize() and small.tickNsteps(1), small.last_error
+    small.destroy()

@@ -27,6 +27,8 @@ bool &pdl_flag() {
 }
 int fail(int code, const std::string &msg) {
     g_last_error = msg;
+    // The CUDA error is reported here: left standing, the next call would report it as its own.
+    if (code == VTP_ERR_CUDA || code == VTP_ERR_NOMEM) cudaGetLastError();
     return code;
 }
 }  // namespace vtp
