@@ -109,3 +109,54 @@ def test_fractions_are_read_in_attach_order(vtp_gpu):
     assert np.array_equal(s.get_field("vol_frac"), after)
     assert np.abs(after[fluid].astype(np.float64).sum(1) - 1.0).max() < 1e-5
     s.destroy()
+
+
+def _bits(s, lo, hi):
+    return _state(s, lo, hi) + [np.array([s.stats()[k] for k in ("total_div_iters", "total_incomp_iters")])]
+
+
+@pytest.mark.parametrize("n_side, tension", [(7, 0.001), (13, 0.001), (13, 0.0)])
+def test_tension_and_objects_give_the_same_bits_on_every_path(vtp_gpu, n_side, tension):
+    """Two fluid objects (a residual mean each) with and without surface tension: alone (eight lanes a
+    row), in a batch whose rows are the last of one path or the first of the next, and with a thread
+    per row asked for by "persistentTiles"."""
+    probe = scenes.colliding_blocks(3, tension, n_side=n_side)
+    nf = probe.n_fluid
+    s = vtp_gpu.solver_from_scene(probe)
+    assert s.tickNsteps(6), s.last_error
+    want = _bits(s, 0, probe.n_total)
+    s.destroy()
+    assert np.isfinite(want[0]).all() and want[3].min() > 0
+    t = vtp_gpu.solver_from_scene(probe, extra={"persistentTiles": True})
+    assert t.tickNsteps(6), t.last_error
+    for x, y in zip(_bits(t, 0, probe.n_total), want):
+        assert np.array_equal(x, y)
+    t.destroy()
+    for rows in (16384, 16385, 49152, 49153):
+        filler = _filler("DFSPH", rows - nf)
+        filler.config["DFSPH"]["Required"]["surfaceTensionCoefficient"] = tension
+        b, ranges = vtp_gpu.solver_from_scenes([filler, probe])
+        assert b.initialize(), b.last_error
+        assert b.tickNsteps(6), b.last_error
+        for name, x, y in zip(("pos", "vel", "density"), _state(b, *ranges[1]), want):
+            assert np.array_equal(x, y), (rows, name)
+        stats = b.scene_stats(1)
+        assert [stats["total_div_iters"], stats["total_incomp_iters"]] == list(want[3]), rows
+        b.destroy()
+
+
+@pytest.mark.parametrize("kind, extra", [("PBF", {"pbfFormulation": "standard"}), ("DFSPH", {"cfl": 0.4}),
+                                         ("DFSPH", {"blockSize": 96}), ("DFSPH", {"blockSize": 256, "unroll": 1})])
+@pytest.mark.parametrize("n", [3000, 30000])
+def test_options_give_the_same_bits_with_and_without_teams(vtp_gpu, kind, extra, n):
+    """Eight and four lanes a row against a thread: the standard PBF kernels, the adaptive step, and
+    residual tiles of three and eight warps."""
+    sc = scenes.dam_break(kind, n, seed=n)
+    got = []
+    for more in ({}, {"persistentTiles": True}):
+        s = vtp_gpu.solver_from_scene(sc, extra={**extra, **more})
+        assert s.tickNsteps(4), s.last_error
+        got.append(_bits(s, 0, sc.n_total))
+        s.destroy()
+    for x, y in zip(*got):
+        assert np.array_equal(x, y)

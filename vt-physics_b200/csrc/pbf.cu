@@ -97,10 +97,11 @@ __device__ __forceinline__ void finish_lambda(const PbfArgs &a, uint32_t r, floa
     halo_each(a, r, [&](const PeerRows &P, uint32_t q) { P.lambda[q] = lam; });
 }
 
-// (lambda_i + lambda_j) g, or (lambda_i m_j + lambda_j m_i) g in the standard form, of a pair.
+// (lambda_i + lambda_j) g, or (lambda_i m_j + lambda_j m_i) g in the standard form, of a pair.  Which
+// of the two products is fused is fixed here: the compiler chose differently in the passes that inline it.
 __device__ __forceinline__ float dx_factor(const PbfArgs &a, float d2, float mi, float mj, float li, float lj) {
     if (a.form == 0) return (li + lj) * cubic_g(d2, a.k);
-    return (li * mj + lj * mi) * spiky_g(d2, a);
+    return __fmaf_rn(li, mj, __fmul_rn(lj, mi)) * spiky_g(d2, a);
 }
 // The correction sum applied to row r: position (second buffer) and velocity.
 __device__ __forceinline__ void finish_dx(const PbfArgs &a, uint32_t r, const float4 &p, float dx, float dy, float dz) {
