@@ -132,7 +132,9 @@ VTP_API int vtp_solver_create(int solver_type, vtp_solver **out);
  *   "deviceLoop": false drives the pressure-solve loops from the host;
  *   "useGraphs": false launches kernels one by one instead of a CUDA graph;
  *   "blockSize": threads per block of the neighbour passes (32..256);
- *   "unroll": neighbour-list entries in flight per thread (1, 2, 4, 8);
+ *   "unroll": neighbour-list entries in flight per thread (1, 2, 4, 8) where
+ *       a thread walks a row: mixtures, and PBF and DFSPH of more than 49,152
+ *       fluid rows;
  *   "persistentTiles": true runs the pressure-solve passes as a persistent
  *       grid looping over the scene-offset tiles (default: one block per tile);
  *   "pbfFormulation": "reference" (default: the reference's PBF arithmetic,
