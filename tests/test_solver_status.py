@@ -53,3 +53,25 @@ def test_one_call_frame_reports_the_stop(vtp_gpu):
     p.free()
     v.free()
     s.destroy()
+
+
+@pytest.mark.parametrize("kind", ["DFSPH", "IMM", "IMMCT"])
+def test_host_driven_solves_start_from_the_solver_s_state(vtp_gpu, kind):
+    """"deviceLoop": false runs the solves from the host, without graphs, from the state the caller has
+    set: the same bits as the captured substeps."""
+    import numpy as np
+    sc = (scenes.dam_break("DFSPH", 5000, seed=3) if kind == "DFSPH" else scenes.layered_mixture(kind, 14, seed=3))
+    rng = np.random.default_rng(1)
+    fluid = np.concatenate([np.full(o.n, o.material == 0) for o in sc.objects])
+    vel = np.where(fluid[:, None], 0.05 * rng.standard_normal((fluid.size, 3)), 0.0).astype(np.float32)
+    got = []
+    for extra in ({}, {"useGraphs": False}, {"deviceLoop": False}):
+        s = vtp.solver_from_scene(sc, extra=extra)
+        assert s.initialize(), s.last_error
+        s.set_field("vel", vel)
+        assert s.tickNsteps(3), s.last_error
+        got.append([s.get_field("pos"), s.get_field("vel")] + ([s.get_field("vol_frac")] if kind != "DFSPH" else []))
+        s.destroy()
+    for other in got[1:]:
+        for x, y in zip(got[0], other):
+            assert np.array_equal(x, y)

@@ -942,27 +942,36 @@ int vtp_solver::enqueue_tick(cudaStream_t s, bool capture) {
 int vtp_solver::build_graphs() {
     // Capture two substep graphs: the double buffers swap an odd number of
     // times per substep, so the second graph starts where the first ended.
-    int start_state[4] = {pos.cur, vel.cur, orig.cur, vadv.cur};
+    const int start_state[4] = {pos.cur, vel.cur, orig.cur, vadv.cur};
+    // A capture that fails has swapped buffers that no kernel has filled: back to where it began.
+    auto failed = [&](int rc) {
+        pos.cur = start_state[0]; vel.cur = start_state[1]; orig.cur = start_state[2]; vadv.cur = start_state[3];
+        if (imm) immct_set_parity(*this, orig.cur);
+        for (auto &ge : gexec)
+            if (ge) cudaGraphExecDestroy(ge), ge = nullptr;
+        return rc;
+    };
     for (int p = 0; p < 2; ++p) {
         gstate[p][0] = pos.cur; gstate[p][1] = vel.cur; gstate[p][2] = orig.cur; gstate[p][3] = vadv.cur;
         launches_per_tick = 0;
-        CU(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
+        cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed);
+        if (e != cudaSuccess) return failed(fail(VTP_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e)));
         int rc = enqueue_tick(st, true);
         cudaGraph_t g = nullptr;
-        cudaError_t e = cudaStreamEndCapture(st, &g);
+        e = cudaStreamEndCapture(st, &g);
         if (rc) {
             if (g) cudaGraphDestroy(g);
-            return rc;
+            return failed(rc);
         }
-        if (e != cudaSuccess) return fail(VTP_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
+        if (e != cudaSuccess) return failed(fail(VTP_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e)));
         e = cudaGraphInstantiate(&gexec[p], g, 0);
         cudaGraphDestroy(g);
-        if (e != cudaSuccess) return fail(VTP_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(e));
+        if (e != cudaSuccess) return failed(fail(VTP_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(e)));
     }
     if (imm) immct_set_parity(*this, orig.cur);
     if (pos.cur != start_state[0] || vel.cur != start_state[1] || orig.cur != start_state[2] ||
         vadv.cur != start_state[3])
-        return fail(VTP_ERR_STATE, "substep buffer parity does not repeat after two substeps");
+        return failed(fail(VTP_ERR_STATE, "substep buffer parity does not repeat after two substeps"));
     graphs_ready = true;
     parity = 0;
     return VTP_OK;
@@ -1012,6 +1021,7 @@ int vtp_solver::tick_n(uint32_t n, const std::function<int()> &tail) {
         CU(cudaMemsetAsync(solve, 0, 2 * scenes.size() * sizeof(vtp::SolveState), st));
         CU(cudaMemsetAsync(loop, 0, 2 * sizeof(vtp::LoopState), st));
     }
+    if (solves && !device_loop) use_graphs = false;   // the host drives the solves: nothing to capture
     if (use_graphs && !graphs_ready) {
         if ((rc = build_graphs())) {
             // A failed capture leaves the stream usable; fall back to direct launches.
