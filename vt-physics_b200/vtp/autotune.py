@@ -4,18 +4,20 @@ Tuned dimensions (keys of the solver config's "B200" block):
   * blockSize  - threads per block = fluid rows per scene-offset tile of the
                  pressure solve (32..256);
   * unroll     - neighbour-list entries whose gathers a thread keeps in
-                 flight (1, 2, 4, 8);
+                 flight (1, 2, 4, 8; no effect where a team walks each row);
   * cell tile  - how rows are grouped into cells and cell tiles: "linear"
                  (the reference's cell order), "brick" (4 x 4 x 4-cell
                  bricks, Morton order inside) or, for DFSPH, "staged" (bricks
                  whose neighbourhoods the pressure solve copies into shared
                  memory; "cellOrder" / "stagedSolve" / "stageRows");
-  * rowLanes   - threads per row of the PBF neighbour passes (1, 4, 8);
-  * listLanes  - accepted by the solver, which chooses its list builder by row
-                 count; every value measures the same;
+  * rowLanes   - threads per row of the PBF neighbour passes (1: the terms in
+                 list order, small scenes with a team of lanes; 4, 8);
+  * listLanes  - the list builder (0: by row count, 1: a thread per row, 8: rows
+                 of a cell together);
   * adjointLanes - threads per row of the PBF adjoint's neighbour passes (1, 2,
-                 4, 8), tuned for the differentiable workload only, after the
-                 forward's keys, on the backward's wall-clock time.
+                 4, 8; the solver's own choice, by row count, is one of them),
+                 tuned for the differentiable workload only, after the forward's
+                 keys, on the backward's wall-clock time.
 Every candidate is timed with the library's per-kernel CUDA-event profiler
 (the substep's kernel time; the adjoint's keys: a recorded rollout's backward),
 by coordinate descent from the current best:
