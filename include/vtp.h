@@ -443,7 +443,7 @@ VTP_API int vtp_solver_dfsph_solve_backward(vtp_solver *s, const float *vbar_out
  * race: order them on one stream. */
 #define VTP_NOALLOC_MAX_PARTICLES 1048576u
 #define VTP_NOALLOC_MAX_CELLS 2097152u
-#define VTP_NOALLOC_SCRATCH_BYTES 50336512ull
+#define VTP_NOALLOC_SCRATCH_BYTES 46142208ull
 VTP_API int vtp_ugns_neighbors_noalloc(const float *d_pos, uint32_t n, const float lb[3], const float size[3],
                                        float cell, uint32_t max_nbr, uint32_t *d_counts, uint32_t *d_nbrs,
                                        void *stream);

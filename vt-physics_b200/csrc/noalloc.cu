@@ -40,8 +40,7 @@ constexpr size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 constexpr size_t kOffKey = 0;
 constexpr size_t kOffRank = kOffKey + align256(4ull * kMaxParticles);
 constexpr size_t kOffTmp = kOffRank + align256(4ull * kMaxParticles);
-constexpr size_t kOffSorted = kOffTmp + align256(4ull * kMaxParticles);
-constexpr size_t kOffPos = kOffSorted + align256(4ull * kMaxParticles);
+constexpr size_t kOffPos = kOffTmp + align256(4ull * kMaxParticles);
 constexpr size_t kOffCount = kOffPos + align256(16ull * kMaxParticles);
 constexpr size_t kOffStart = kOffCount + align256(4ull * (kMaxKeys + 1));
 constexpr size_t kOffTiles = kOffStart + align256(4ull * (kMaxKeys + 2));
@@ -52,7 +51,7 @@ static_assert(kArenaBytes == VTP_NOALLOC_SCRATCH_BYTES, "scratch size in vtp.h o
 __device__ __align__(256) unsigned char g_noalloc_scratch[kArenaBytes];
 
 struct Arena {
-    uint32_t *key, *rank, *tmp, *sorted, *count, *start, *tiles;
+    uint32_t *key, *rank, *tmp, *count, *start, *tiles;
     float4 *pos;
 };
 
@@ -61,7 +60,6 @@ Arena arena_at(unsigned char *base) {
     a.key = (uint32_t *)(base + kOffKey);
     a.rank = (uint32_t *)(base + kOffRank);
     a.tmp = (uint32_t *)(base + kOffTmp);
-    a.sorted = (uint32_t *)(base + kOffSorted);
     a.pos = (float4 *)(base + kOffPos);
     a.count = (uint32_t *)(base + kOffCount);
     a.start = (uint32_t *)(base + kOffStart);
@@ -196,7 +194,6 @@ __global__ void k_na_rank(vtp::Grid g, uint32_t n, const float *__restrict__ pos
         for (uint32_t x = s0; x < s1; ++x) r += a.tmp[x] < me ? 1u : 0u;
         dst = s0 + r;
     }
-    a.sorted[dst] = me;
     a.pos[dst] = make_float4(pos[3 * (size_t)me], pos[3 * (size_t)me + 1], pos[3 * (size_t)me + 2],
                              __uint_as_float(me));
 }
