@@ -246,8 +246,8 @@ __device__ __forceinline__ float rsqrt_normal(float x) {
 // evaluates it, whatever the compiler contracts around the call.  Without a
 // branch: the two sides of q = 1/2 share their last product, and a d2 below the
 // normal range ends in a q of infinity, outside the range.  The passes that evaluate it
-// for every pair are bound by issue: 1M rows, DFSPH ratio pass 119 -> 109 us and
-// viscosity 117 -> 107; 250k rows, PBF lambda 38.9 -> 36.3; 500k rows of a
+// for every pair share their time between issue and gathers: 1M rows, DFSPH ratio pass 119 -> 109 us
+// and viscosity 117 -> 109; 250k rows, PBF lambda 38.9 -> 36.3; 500k rows of a
 // mixture, viscosity and normals 126 -> 117 and precompute 82 -> 76.
 __device__ __forceinline__ float cubic_g(float d2, const Cubic &k) {
     const float rinv = rsqrt_normal(d2);

@@ -490,7 +490,8 @@ struct WalkedRow {
 // 41, DFSPH 16,000 rows 23 -> 17 -> 17, 128,000 rows 113 -> 50 -> 48.  After 100-200 substeps: 21 -> 21 ->
 // 23, 50 -> 48 -> 47, 80 -> 72 -> 64, 21 -> 21 -> 23, 80 -> 76 -> 62.  Clouds of 100,000 rows 0.35, 0.7 and
 // 1 cells apart: 188 -> 162 -> 91, 44 -> 58 -> 56, 27 -> 88 -> 33.  30,000 rows with 10,000 in one cell:
-// 750 -> 46,900 -> 450.
+// 750 -> 46,900 -> 450.  Bound by latencies: at 120,000 rows 44 % of the issue slots, 64 % of the L1
+// rate, and the 36 % of the warp slots that its shared memory allows.
 template <int MODE, uint32_t SCAN>
 __global__ void __launch_bounds__(kCellWarps * 32, 7) k_build_lists(
     Scenes sc, uint32_t row0, uint32_t cnt, ListShape shape, const float4 *__restrict__ pos,
