@@ -156,3 +156,15 @@ def test_a_thread_per_row_matches_the_oracle(vtp_gpu, oracle_lib, n, attach, cul
     cnt, nbr = s.get_neighbors(60)
     s.destroy()
     assert np.array_equal(cnt, want[0]) and np.array_equal(nbr, want[1])
+
+
+def test_scan_of_a_large_grid_runs_at_memory_rate(vtp_gpu):
+    """27 million buckets are read twice, zeroed and written: 16 bytes each, 66 us at 6.5 TB/s, three
+    launches.  Three times that leaves room for the launches and for reads that miss the L2."""
+    sc = _scene(*_cloud(8000, 0.5))
+    sc.config["PBF"]["Required"]["simSpaceSize"] = [300 * H] * 3
+    s = vtp_gpu.solver_from_scene(sc)
+    assert s.initialize(), s.last_error
+    best = min(s.profile_kernels(1)["ugns_cell_scan"][0] for _ in range(5))
+    s.destroy()
+    assert best <= 3 * 300 ** 3 * 16 / 6.5e9

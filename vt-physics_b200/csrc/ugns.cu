@@ -177,8 +177,6 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(uint32_t *__restric
         uint32_t v = 0;
         for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kScanThreads) v += sums[t];
         block_excl_scan(v, before);
-    } else {
-        before = sums[blockIdx.x];
     }
     // Each thread scans kScanItems consecutive counters.
     __shared__ uint32_t tile[kScanTile];
@@ -197,7 +195,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(uint32_t *__restric
         s += vals[k];
     }
     uint32_t total;
-    uint32_t off = block_excl_scan(s, total) + before + base_add;
+    uint32_t off = block_excl_scan(s, total) + (PREFIX ? before : sums[blockIdx.x]) + base_add;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         const size_t idx = t0 + (size_t)threadIdx.x * kScanItems + k;
