@@ -313,48 +313,53 @@ struct AnySlots {
 // are issued, so each thread keeps U gathers and U index loads in flight.
 // `use(j, data)` runs in list order, which keeps FP32 accumulation order
 // identical for every U.  (The last partial batch one gather at a time: with
-// its gathers issued together the solve passes are 3-9 % slower at 1M rows.)  Where `use` leaves the
-// fusing of its products to the compiler (mixtures), the form of the loop decides it too: each U
-// keeps its own.
+// its gathers issued together the solve passes are 3-9 % slower at 1M rows.)
 template <int U, class Slots, class Load, class Use>
 __device__ __forceinline__ void nbr_loop_at(const uint32_t *__restrict__ lst, Slots at, uint32_t cnt, Load load,
                                             Use use) {
-    if constexpr (U <= 1) {
-        for (uint32_t t = 0; t < cnt; ++t) {
-            const uint32_t j = __ldcs(lst + at(t));
-            use(j, load(j));
-        }
-    } else {
-        using T = decltype(load(0u));
-        uint32_t nxt[U];
+    using T = decltype(load(0u));
+    uint32_t nxt[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) nxt[u] = (uint32_t)u < cnt ? __ldcs(lst + at((uint32_t)u)) : 0u;
-        uint32_t t = 0;
-        for (; t + U <= cnt; t += U) {
-            uint32_t j[U];
+    for (int u = 0; u < U; ++u) nxt[u] = (uint32_t)u < cnt ? __ldcs(lst + at((uint32_t)u)) : 0u;
+    uint32_t t = 0;
+    for (; t + U <= cnt; t += U) {
+        uint32_t j[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) j[u] = nxt[u];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const uint32_t tt = t + U + (uint32_t)u;
-                nxt[u] = tt < cnt ? __ldcs(lst + at(tt)) : 0u;
-            }
-            T d[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) d[u] = load(j[u]);
-#pragma unroll
-            for (int u = 0; u < U; ++u) use(j[u], d[u]);
-        }
+        for (int u = 0; u < U; ++u) j[u] = nxt[u];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            if (t + (uint32_t)u < cnt) use(nxt[u], load(nxt[u]));
+            const uint32_t tt = t + U + (uint32_t)u;
+            nxt[u] = tt < cnt ? __ldcs(lst + at(tt)) : 0u;
         }
+        T d[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) d[u] = load(j[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) use(j[u], d[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        if (t + (uint32_t)u < cnt) use(nxt[u], load(nxt[u]));
     }
 }
 // In the passes with a thread per row.
 template <int U, class Load, class Use>
 __device__ __forceinline__ void nbr_loop(const uint32_t *__restrict__ lst, uint32_t cnt, Load load, Use use) {
     nbr_loop_at<U>(lst, RowSlots{}, cnt, load, use);
+}
+
+// nbr_loop whose form for U = 1 is the plain loop: for a `use` that leaves the fusing of its products
+// to the compiler, which decides by the form of the loop.
+template <int U, class Load, class Use>
+__device__ __forceinline__ void nbr_loop_plain(const uint32_t *__restrict__ lst, uint32_t cnt, Load load, Use use) {
+    if constexpr (U <= 1) {
+        for (uint32_t t = 0; t < cnt; ++t) {
+            const uint32_t j = __ldcs(lst + (size_t)t * 32u);
+            use(j, load(j));
+        }
+    } else {
+        nbr_loop<U>(lst, cnt, load, use);
+    }
 }
 
 // Lane groups for rows walked by L lanes each (L divides 32; the L lanes of a

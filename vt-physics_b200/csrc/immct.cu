@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(256) k_drift_diffuse(ImmArgs a, int retry) {
         const uint32_t *lst = a.nbr + row_index(r, a.shape);
         const float ndt = -a.dt;
         // drift
-        nbr_loop<U>(lst, n > 0 ? n - 1 : 0,
+        nbr_loop_plain<U>(lst, n > 0 ? n - 1 : 0,
                     [&](uint32_t j) {
                         if (j >= a.nf) return DG{};
                         return DG{ldg4(a.pos + j), ldg4(a.vel + j), __ldg(a.flag + j)};
@@ -646,7 +646,7 @@ __global__ void __launch_bounds__(256) k_drift_diffuse(ImmArgs a, int retry) {
                     });
         // diffusion
         const float dtcf = a.dt * a.p.Cf;
-        nbr_loop<U>(lst, n > 0 ? n - 1 : 0,
+        nbr_loop_plain<U>(lst, n > 0 ? n - 1 : 0,
                     [&](uint32_t j) {
                         if (j >= a.nf) return DG{};
                         return DG{ldg4(a.pos + j), make_float4(0.f, 0.f, 0.f, 0.f), __ldg(a.flag + j)};
