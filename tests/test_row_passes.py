@@ -176,3 +176,17 @@ def test_unroll_of_one_gives_a_small_mixture_the_same_bits(vtp_gpu, kind):
     for other in got[1:]:
         for x, y in zip(got[0], other):
             assert np.array_equal(x, y)
+
+
+def test_a_staged_solver_takes_a_thread_per_row(vtp_gpu):
+    """The staged solve's kernels read a list's entries a thread per row, in lists laid out for that;
+    the other passes then read the same lists, whatever the row count."""
+    import torch
+    s = vtp_gpu.solver_from_scene(scenes.dam_break("DFSPH", 3000, seed=2), extra={"stagedSolve": True})
+    assert s.initialize(), s.last_error
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        s.profile_kernels(1)
+        torch.cuda.synchronize()
+    names = " ".join(e.key for e in prof.key_averages())
+    s.destroy()
+    assert "k_solve_a_staged" in names and "k_viscosity" in names and "k_team" not in names

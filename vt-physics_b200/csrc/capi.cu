@@ -480,12 +480,6 @@ int vtp_solver::initialize() {
     L.merge_mode = mode < 0 ? 0 : mode;
     L.list_lanes = list_lanes;
     L.cell_cull = cell_cull;
-    teams = persistent_tiles || (type != VTP_SOLVER_DFSPH && type != VTP_SOLVER_PBF) ? 0
-            : L.nf <= vtp::kTeam8MaxRows                                             ? 8
-            : L.nf <= vtp::kTeamMaxRows                                              ? 4
-                                                                                     : 0;
-    L.shape.lg = teams ? vtp::kTeamListLg : 0u;
-    L.shape.stride = vtp::list_stride(maxnbr > 1 ? maxnbr - 1 : 1, L.shape.lg);
 
     // Grids as UniformGirdNeighborSearcher::setConfig (UniformGridNeighborSearch.cpp:214-218),
     // one per scene, each followed by its own outside bucket.
@@ -518,6 +512,17 @@ int vtp_solver::initialize() {
         sc.bbase = bb; bb += sc.nb;
     }
     nbuckets = (uint32_t)key_base;
+    // Staged pressure solve: one scene in bricked order whose cells' fluid and boundary runs do not
+    // interleave.  Its passes and builder take a thread per row, so the solver's lists have their shape
+    // (30,000 rows, B200, us: solve_a 30 against 39 and solve_b 21 against 23 on the teams' lists).
+    staged = staged_solve && type == VTP_SOLVER_DFSPH && S == 1 && scenes[0].grid.brick && L.merge_mode != 2 &&
+             L.nf > 0;
+    teams = persistent_tiles || staged || (type != VTP_SOLVER_DFSPH && type != VTP_SOLVER_PBF) ? 0
+            : L.nf <= vtp::kTeam8MaxRows                                                       ? 8
+            : L.nf <= vtp::kTeamMaxRows                                                        ? 4
+                                                                                               : 0;
+    L.shape.lg = teams ? vtp::kTeamListLg : 0u;
+    L.shape.stride = vtp::list_stride(maxnbr > 1 ? maxnbr - 1 : 1, L.shape.lg);
     d2max = sqrt_threshold(h);
     kc.h = h;
     kc.invh = 1.f / h;
@@ -691,10 +696,7 @@ int vtp_solver::initialize() {
         if (!tiles.empty())
             CU(cudaMemcpyAsync(d_tiles, tiles.data(), tiles.size() * sizeof(uint4), cudaMemcpyHostToDevice, st));
         CU(cudaMemcpyAsync(d_scene_tiles, stl.data(), S * sizeof(vtp::SceneTiles), cudaMemcpyHostToDevice, st));
-        // Staged pressure solve: one scene in bricked order whose cells' fluid and boundary runs
-        // do not interleave; residual partials per cell group (plus one for the rows outside).
-        staged = staged_solve && type == VTP_SOLVER_DFSPH && S == 1 && scenes[0].grid.brick &&
-                 L.merge_mode != 2 && L.nf > 0;
+        // Staged solve: residual partials per cell group (plus one for the rows outside).
         size_t npart = std::max<size_t>((size_t)ntiles * (teams ? vtp::solve_pieces(block) : 1u), 1);
         if (staged) {
             stg.ngroups = scenes[0].grid.nkey / vtp::kStageBuckets;

@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(kStageBlock) k_solve_a_staged(DfsphArgs a) {
         };
         const uint32_t cnt = n > 0 ? n - 1 : 0;
         if (staged) {
-            slot_loop<U>(a.stg.snbr + ell_index(r, 0, a.shape), a.shape, cnt,
+            slot_loop<U>(a.stg.snbr + row_index(r, a.shape), cnt,
                          [&](uint16_t s) {
                              uint32_t q = (uint32_t)(s & 0x7fffu);
 #ifdef VTP_CHECKED
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(kStageBlock) k_solve_a_staged(DfsphArgs a) {
                          },
                          use);
         } else {
-            nbr_loop_at<U>(a.nbr + ell_index(r, 0, a.shape), AnySlots{a.shape}, cnt,
+            nbr_loop<U>(a.nbr + row_index(r, a.shape), cnt,
                         [&](uint32_t j) { return ldg8(a.pva + 2 * (size_t)j); }, use);
         }
         if (d < 0.f) d = 0.f;
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(kStageBlock) k_solve_b_staged(DfsphArgs a) {
         };
         const uint32_t cnt = n > 0 ? n - 1 : 0;
         if (staged) {
-            slot_loop<U>(a.stg.snbr + ell_index(r, 0, a.shape), a.shape, cnt,
+            slot_loop<U>(a.stg.snbr + row_index(r, a.shape), cnt,
                          [&](uint16_t s) {
                              uint32_t q = (uint32_t)(s & 0x7fffu);
 #ifdef VTP_CHECKED
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(kStageBlock) k_solve_b_staged(DfsphArgs a) {
                          },
                          [&](uint16_t s, const float4 &e) { step(!(s & kSlotBoundary), e); });
         } else {
-            nbr_loop_at<U>(a.nbr + ell_index(r, 0, a.shape), AnySlots{a.shape}, cnt, [&](uint32_t j) { return ldg4(a.pk + j); },
+            nbr_loop<U>(a.nbr + row_index(r, a.shape), cnt, [&](uint32_t j) { return ldg4(a.pk + j); },
                         [&](uint32_t j, const float4 &e) { step(j < a.nf, e); });
         }
         a.vadv[r] = v;

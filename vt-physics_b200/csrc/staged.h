@@ -117,15 +117,15 @@ __device__ __forceinline__ uint32_t slot_row(const GroupPlan &P, int u, uint32_t
     return boundary ? P.bs[u] + l : P.fs[u] + (l - P.nbl[u]);
 }
 
-// nbr_loop over a slot list (2-byte entries, ELL layout): U entries' loads in flight.
+// nbr_loop over a slot list (2-byte entries in lists of lg 0): U entries' loads in flight.
 template <int U, class Load, class Use>
-__device__ __forceinline__ void slot_loop(const uint16_t *__restrict__ lst, ListShape shape, uint32_t cnt, Load load, Use use) {
+__device__ __forceinline__ void slot_loop(const uint16_t *__restrict__ lst, uint32_t cnt, Load load, Use use) {
     using T = decltype(load((uint16_t)0));
     uint32_t t = 0;
     for (; t + U <= cnt; t += U) {
         uint16_t j[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) j[u] = __ldcs(lst + ell_slot(t + u, shape));
+        for (int u = 0; u < U; ++u) j[u] = __ldcs(lst + (size_t)(t + u) * 32u);
         T d[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) d[u] = load(j[u]);
@@ -133,7 +133,7 @@ __device__ __forceinline__ void slot_loop(const uint16_t *__restrict__ lst, List
         for (int u = 0; u < U; ++u) use(j[u], d[u]);
     }
     for (; t < cnt; ++t) {
-        const uint16_t j = __ldcs(lst + ell_slot(t, shape));
+        const uint16_t j = __ldcs(lst + (size_t)t * 32u);
         use(j, load(j));
     }
 }

@@ -650,13 +650,12 @@ __global__ void __launch_bounds__(kStageBlock) k_build_lists_staged(
         FaceGaps fg;
         if (CULL) fg.init(p, c, g, sc.cell);
         if (!staged) {
-            Walker<AnySlots> w;
+            Walker<RowSlots> w;
             w.px = p.x; w.py = p.y; w.pz = p.z;
             w.self = r;
             w.cnt = 1;
             w.maxnbr = maxnbr;
-            w.out = nbr + ell_index(r, 0, shape);
-            w.at = AnySlots{shape};
+            w.out = nbr + row_index(r, shape);
             w.overflow = false;
             for (int t = 0; t < 27; ++t) {
                 const int3 o = nbr_offset(t);
@@ -678,8 +677,8 @@ __global__ void __launch_bounds__(kStageBlock) k_build_lists_staged(
             }
             continue;
         }
-        uint32_t *const out = nbr + ell_index(r, 0, shape);
-        uint16_t *const sout = stg.snbr + ell_index(r, 0, shape);
+        uint32_t *const out = nbr + row_index(r, shape);
+        uint16_t *const sout = stg.snbr + row_index(r, shape);
         uint32_t cnt = 1;
         bool over = false;
         for (int t = 0; t < 27; ++t) {
@@ -704,8 +703,8 @@ __global__ void __launch_bounds__(kStageBlock) k_build_lists_staged(
                 if (d2 > 0.f && d2 <= d2max) {
                     if (room || cnt < maxnbr) {
                         const bool bnd = MODE == 0 ? sl >= sb : sl < sb;
-                        out[ell_slot(cnt - 1, shape)] = __float_as_uint(q.w);
-                        sout[ell_slot(cnt - 1, shape)] = (uint16_t)(sl | (bnd ? kSlotBoundary : 0u));
+                        out[(size_t)(cnt - 1) * 32u] = __float_as_uint(q.w);
+                        sout[(size_t)(cnt - 1) * 32u] = (uint16_t)(sl | (bnd ? kSlotBoundary : 0u));
                         ++cnt;
                     } else {
                         over = true;
